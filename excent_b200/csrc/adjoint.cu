@@ -13,9 +13,7 @@
 //   dL/dw[e] = (G_e - sum_{e' in row u} wn[e'] G_e') / rowsum_u, G = dL/dwn.
 // No reference counterpart (the reference has no weights and no adjoint).
 //
-// The push passes use a touched-vertex frontier (a vertex is re-examined
-// only after its residual changed) and run as one CUDA graph with a
-// conditional while node. FP64 pull (Jacobi) solvers of the same fixed
+// A solve is one cooperative launch that runs every pass. FP64 pull (Jacobi) solvers of the same fixed
 // points give finite differences and the oracle gradient for verification.
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
@@ -27,15 +25,34 @@
 
 #include "common.h"
 #include "device.cuh"
+#include "gridsync.cuh"
 
 namespace excent {
 
 static constexpr int WB = 256;
+static constexpr int WP = 1024;             // threads per block of the persistent push, one block per SM
+static constexpr unsigned WLONG = 256;      // longer lists are scattered, summed and scaled as segments ...
+static constexpr unsigned WSEG = 512;       // ... of this many entries, one warp each
+static constexpr int WUNROLL = 4;           // entries per lane in flight
 
 struct WCtrl {
-    int pass, max_passes, done, err;
-    ull pushed_v[2];
-    ull total_v, total_e;
+    int pass, max_passes, pad0, pad1;
+    ull pushed_v[2];   // vertices pushed, by pass parity
+    ull nseg[2];       // segments queued, by pass parity
+    ull total_e;
+    GridBar bar;
+};
+
+// A stretch of one list: the queued scatter of a long list, or (static) the
+// rows that are longer than WLONG.
+struct WSegment {
+    ull base;       // first entry
+    unsigned len;
+    float f;        // scatter weight (queue)
+};
+struct WRowSeg {
+    ull base;
+    unsigned len, row;
 };
 
 struct WArgs {
@@ -47,121 +64,214 @@ struct WArgs {
     float eps;
     float* x;
     float* r;
-    uint32_t* touched[2];
-    int words;
+    WSegment* seg;
+    ull seg_cap;
     WCtrl* ctrl;
 };
 
-__device__ __forceinline__ void wmark(uint32_t* t, int u) {
-    const uint32_t bit = 1u << (u & 31);
-    if (!(t[u >> 5] & bit)) atomicOr(&t[u >> 5], bit);
-}
-
-// One pass: lanes take the touched vertices of a bitmap word, then the warp
-// scatters each pushed vertex's list with s * d * wt[e] per entry.
-__global__ void __launch_bounds__(WB) k_wpass(WArgs a) {
+// The whole delta-push in one cooperative launch. A pass is two phases with a
+// grid barrier after each: every vertex above eps is taken and its list
+// scattered (s * d * wt[e] per entry), then the lists longer than WLONG, which
+// the first phase only queued, are scattered one segment per warp.
+//
+// What bounds it: one red.global per pushed entry, and, in the many passes
+// with little to push, the two barriers and the scan of r (n floats, in L2).
+// A warp's 32 lists are scattered as one stretch of entries with every lane
+// busy, and no warp has more than 32 * WLONG entries: with whole lists on one
+// warp a pass lasted as long as the longest list (69k entries in 540 dependent
+// steps on an R-MAT of 1M vertices, 16.8M entries: 300 ms for forward and
+// gradient together).
+__global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const long long gw = (long long)wib * gridDim.x + blockIdx.x;   // neighbouring tiles on different SMs
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const int par = a.ctrl->pass & 1;
-    uint32_t* cur = par ? a.touched[1] : a.touched[0];   // no run-time index into the parameters
-    uint32_t* nxt = par ? a.touched[0] : a.touched[1];
-    ull pv = 0, pe = 0;
-    for (long long w = gw; w < a.words; w += nwarps) {
-        const uint32_t bits = cur[w];
-        if (!bits) continue;
-        __syncwarp();
-        if (lane == 0) cur[w] = 0;
-        const int v = (int)(w * 32 + lane);
-        float d = 0.f;
-        ull b0 = 0;
-        unsigned deg = 0;
-        if ((bits >> lane) & 1u) {
-            if (fabsf(a.r[v]) > a.eps) {
-                d = atomicExch(&a.r[v], 0.f);
-                a.x[v] += d;
+    const long long ntiles = ((long long)a.n + 31) / 32;
+    __shared__ ull s_base[WP / 32][32];   // per warp: the tile's nonempty lists, compacted
+    __shared__ unsigned s_ex[WP / 32][32];
+    __shared__ float s_f[WP / 32][32];
+    __shared__ ull s_v[WP / 32];
+    unsigned epoch = 0;
+    ull pe = 0;
+    const int max_passes = a.ctrl->max_passes;
+    for (int pass = 0;; pass++) {
+        const int par = pass & 1;
+        ull pv = 0;
+        for (long long t0 = gw; t0 < ntiles; t0 += 4 * nwarps) {
+            float rv[4];   // four tiles' residuals in flight before they are examined
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const long long v = (t0 + k * nwarps) * 32 + lane;
+                rv[k] = v < a.n ? a.r[v] : 0.f;
             }
-            if (d != 0.f) {
-                b0 = a.idx[v];
-                deg = (unsigned)(a.idx[v + 1] - b0);
-                pv++;
-                pe += deg;
+#pragma unroll 1
+            for (int k = 0; k < 4; k++) {
+                const float rk = k == 0 ? rv[0] : k == 1 ? rv[1] : k == 2 ? rv[2] : rv[3];
+                if (!__any_sync(FULL, fabsf(rk) > a.eps)) continue;
+                const long long v = (t0 + k * nwarps) * 32 + lane;
+                float d = 0.f;
+                ull b0 = 0;
+                unsigned deg = 0;
+                if (fabsf(rk) > a.eps) {
+                    d = atomicExch(&a.r[v], 0.f);
+                    a.x[v] += d;
+                    if (d != 0.f) {
+                        b0 = a.idx[v];
+                        deg = (unsigned)(a.idx[v + 1] - b0);
+                        pv++;
+                        pe += deg;
+                    }
+                }
+                const float f = a.s * d;
+                const unsigned nseg = deg > WLONG ? (deg + WSEG - 1) / WSEG : 0u;
+                const unsigned sincl = warp_incl_scan(nseg, lane);
+                const unsigned stot = __shfl_sync(FULL, sincl, 31);
+                if (stot) {   // long lists: one queue reservation per warp
+                    ull at = 0;
+                    if (lane == 0) at = atomicAdd(&a.ctrl->nseg[par], (ull)stot);
+                    at = __shfl_sync(FULL, at, 0) + (sincl - nseg);
+                    for (unsigned i = 0; i < nseg && at + i < a.seg_cap; i++)
+                        a.seg[at + i] = WSegment{b0 + (ull)i * WSEG, min(WSEG, deg - i * WSEG), f};
+                }
+                const unsigned ds = nseg ? 0u : deg;
+                const unsigned nz = __ballot_sync(FULL, ds != 0);
+                if (!nz) continue;
+                const unsigned incl = warp_incl_scan(ds, lane);
+                const unsigned tot = __shfl_sync(FULL, incl, 31);
+                const unsigned ex = incl - ds;
+                if (ds) {
+                    const int rank = __popc(nz & ((1u << lane) - 1u));
+                    s_base[wib][rank] = b0; s_ex[wib][rank] = ex; s_f[wib][rank] = f;
+                }
+                __syncwarp();
+                const unsigned le = lane == 31 ? FULL : (2u << lane) - 1u;
+                for (unsigned j0 = 0; j0 < tot; j0 += 32 * WUNROLL) {
+                    int u[WUNROLL];
+                    float w[WUNROLL];
+#pragma unroll
+                    for (int q = 0; q < WUNROLL; q++) {
+                        // owner of entry wb + lane: the last nonempty list starting at or before it
+                        const unsigned wb = j0 + 32 * q, j = wb + lane;
+                        const unsigned starts =
+                            __reduce_or_sync(FULL, (ds && ex >= wb && ex - wb < 32) ? 1u << (ex - wb) : 0u);
+                        const int o = __popc(__ballot_sync(FULL, ds && ex <= wb)) - 1 + __popc(starts & le & ~1u);
+                        u[q] = -1;
+                        w[q] = 0.f;
+                        if (j < tot) {
+                            const ull e = s_base[wib][o] + (j - s_ex[wib][o]);
+                            u[q] = ld_edge(a.adj + e);
+                            w[q] = s_f[wib][o] * __ldcs(a.wt + e);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < WUNROLL; q++)
+                        if (u[q] >= 0) red_add(a.r, u[q], w[q]);
+                }
+                __syncwarp();
             }
         }
-        uint32_t mm = __ballot_sync(FULL, d != 0.f && deg > 0);
-        while (mm) {
-            const int sl = __ffs(mm) - 1;
-            mm &= mm - 1;
-            const ull bb = __shfl_sync(FULL, b0, sl);
-            const unsigned dd = __shfl_sync(FULL, deg, sl);
-            const float f = a.s * __shfl_sync(FULL, d, sl);
-            for (unsigned i0 = 0; i0 < dd; i0 += 128) {
-                int u[4];
-                float wt[4];
+        pv = warp_sum(pv);
+        if (lane == 0) s_v[wib] = pv;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            ull tv = 0;
+            for (int i = 0; i < WP / 32; i++) tv += s_v[i];
+            if (tv) atomicAdd(&a.ctrl->pushed_v[par], tv);
+        }
+        if (!grid_sync(&a.ctrl->bar, epoch)) return;
+        const ull taken = a.ctrl->pushed_v[par], queued = a.ctrl->nseg[par];
+        if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next pass's counters: nobody uses them before the barrier
+            a.ctrl->pushed_v[par ^ 1] = 0;
+            a.ctrl->nseg[par ^ 1] = 0;
+            if (taken) a.ctrl->pass = pass + 1;
+        }
+        const ull nseg = min(queued, a.seg_cap);
+        for (ull i = gw; i < nseg; i += nwarps) {
+            const WSegment g = a.seg[i];
+            for (unsigned i0 = 0; i0 < g.len; i0 += 32 * WUNROLL) {
+                int u[WUNROLL];
+                float w[WUNROLL];
 #pragma unroll
-                for (int k = 0; k < 4; k++) {   // four entries per lane in flight
-                    const unsigned i = i0 + 32 * k + lane;
-                    u[k] = i < dd ? ld_edge(a.adj + bb + i) : -1;
-                    wt[k] = i < dd ? __ldcs(a.wt + bb + i) : 0.f;
+                for (int q = 0; q < WUNROLL; q++) {
+                    const unsigned j = i0 + 32 * q + lane;
+                    u[q] = j < g.len ? ld_edge(a.adj + g.base + j) : -1;
+                    w[q] = j < g.len ? __ldcs(a.wt + g.base + j) : 0.f;
                 }
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (u[k] >= 0) red_add(a.r, u[k], f * wt[k]);
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (u[k] >= 0) wmark(nxt, u[k]);
+                for (int q = 0; q < WUNROLL; q++)
+                    if (u[q] >= 0) red_add(a.r, u[q], g.f * w[q]);
             }
         }
+        if (!taken || pass + 1 >= max_passes) break;
+        if (!grid_sync(&a.ctrl->bar, epoch)) return;
     }
-    __shared__ ull s_v[WB / 32], s_e[WB / 32];
-    pv = warp_sum(pv);
     pe = warp_sum(pe);
-    if (lane == 0) { s_v[wib] = pv; s_e[wib] = pe; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ull tv = 0, te = 0;
-        for (int i = 0; i < WB / 32; i++) { tv += s_v[i]; te += s_e[i]; }
-        if (tv) atomicAdd(&a.ctrl->pushed_v[par], tv);
-        if (te) atomicAdd(&a.ctrl->total_e, te);
-    }
+    if (lane == 0 && pe) atomicAdd(&a.ctrl->total_e, pe);
 }
 
-__global__ void k_wend(WCtrl* c, cudaGraphConditionalHandle cond, int use_cond) {
-    const int par = c->pass & 1;
-    const ull pv = c->pushed_v[par];
-    c->total_v += pv;
-    c->pushed_v[par ^ 1] = 0;
-    const bool more = pv > 0 && c->pass + 1 < c->max_passes;
-    if (pv > 0) c->pass++;
-    if (!more) c->done = 1;
-    if (use_cond) cudaGraphSetConditional(cond, more ? 1u : 0u);
-}
-
-// x = 0, r = c0 * t (t NULL: all ones), touched where r != 0.
-__global__ void k_wseed(int n, const float* t, float c0, float* x, float* r, uint32_t* touched) {
+// x = 0, r = c0 * t (t NULL: all ones).
+__global__ void k_wseed(int n, const float* t, float c0, float* x, float* r) {
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const float rv = c0 * (t ? t[v] : 1.f);
         x[v] = 0.f;
-        r[v] = rv;
-        if (rv != 0.f) atomicOr(&touched[v >> 5], 1u << (v & 31));
+        r[v] = c0 * (t ? t[v] : 1.f);
     }
 }
 
-// Row sums and normalised weights (FP32 for the push, FP64 for the tools).
+// The rows longer than WLONG as segments, in any order (once per graph).
+__global__ void k_wrowsegs(int n, const ull* idx, WRowSeg* out, ull* cnt) {
+    for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < n; u += (long long)gridDim.x * blockDim.x) {
+        const ull b = idx[u], deg = idx[u + 1] - b;
+        if (deg <= WLONG) continue;
+        const ull k = (deg + WSEG - 1) / WSEG, at = atomicAdd(cnt, k);
+        for (ull i = 0; i < k; i++)
+            out[at + i] = WRowSeg{b + i * WSEG, (unsigned)min((ull)WSEG, deg - i * WSEG), (unsigned)u};
+    }
+}
+
+// Row sums and normalised weights (FP32 for the push, FP64 for the tools): one
+// warp per row of up to WLONG entries. The longer rows start at 0 here; their
+// segments are summed by k_wsegsum and scaled by k_wsegnorm, one warp per
+// segment (a whole row on one warp took 69k / 32 dependent steps, twice).
 __global__ void k_wnorm(int n, const ull* idx, const float* w, float* wn, double* wn64, double* rowsum) {
     const long long u = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (u >= n) return;
+    const ull b = idx[u], e1 = idx[u + 1];
+    if (e1 - b > WLONG) {
+        if (lane == 0) rowsum[u] = 0;
+        return;
+    }
     double s = 0;
-    for (ull e = idx[u] + lane; e < idx[u + 1]; e += 32) s += w[e];
+    for (ull e = b + lane; e < e1; e += 32) s += w[e];
     s = warp_sum(s);
     s = __shfl_sync(FULL, s, 0);
-    for (ull e = idx[u] + lane; e < idx[u + 1]; e += 32) {
+    for (ull e = b + lane; e < e1; e += 32) {
         const double q = (double)w[e] / s;
         wn[e] = (float)q;
         wn64[e] = q;
     }
     if (lane == 0) rowsum[u] = s;
+}
+__global__ void k_wsegsum(ull nseg, const WRowSeg* seg, const float* w, double* rowsum) {
+    const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= nseg) return;
+    const WRowSeg g = seg[i];
+    double s = 0;
+    for (unsigned j = lane; j < g.len; j += 32) s += w[g.base + j];
+    s = warp_sum(s);
+    if (lane == 0) atomicAdd(&rowsum[g.row], s);
+}
+__global__ void k_wsegnorm(ull nseg, const WRowSeg* seg, const float* w, const double* rowsum, float* wn, double* wn64) {
+    const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= nseg) return;
+    const WRowSeg g = seg[i];
+    const double s = rowsum[g.row];
+    for (unsigned j = lane; j < g.len; j += 32) {
+        const double q = (double)w[g.base + j] / s;
+        wn[g.base + j] = (float)q;
+        wn64[g.base + j] = q;
+    }
 }
 
 __global__ void k_wpermute(ull m, const unsigned* perm, const float* wn, const double* wn64, float* wt, double* wt64) {
@@ -169,6 +279,11 @@ __global__ void k_wpermute(ull m, const unsigned* perm, const float* wn, const d
         wt[e] = wn[perm[e]];
         wt64[e] = wn64[perm[e]];
     }
+}
+
+__global__ void k_winverse(ull m, const unsigned* perm, unsigned* inv) {
+    for (ull e = blockIdx.x * (ull)blockDim.x + threadIdx.x; e < m; e += (ull)gridDim.x * blockDim.x)
+        inv[perm[e]] = (unsigned)e;
 }
 
 // Transposed CSR from keys (dst << scale | src) sorted with the original edge ids.
@@ -192,19 +307,48 @@ __global__ void k_wkeys(int n, int shift, const ull* idx, const int* adj, uint64
     }
 }
 
-// Gradient through the row normalisation, one warp per row u.
+// Gradient through the row normalisation: dL/dw[e] = (G_e - sum wn G) / rowsum
+// with G_e = s x_u lam_v, one warp per row of up to WLONG entries; the longer
+// rows' sums are accumulated by k_wgradsum and finished by k_wgradseg.
 __global__ void k_wgrad(int n, const ull* idx, const int* adj, const float* wn, const double* rowsum, const float* x,
-                        const float* lam, float s, float* gw) {
+                        const float* lam, float s, float* gw, double* rowdot) {
     const long long u = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (u >= n) return;
+    const ull b = idx[u], e1 = idx[u + 1];
+    if (e1 - b > WLONG) {
+        if (lane == 0) rowdot[u] = 0;
+        return;
+    }
     const double xu = x[u];
     double dot = 0;
-    for (ull e = idx[u] + lane; e < idx[u + 1]; e += 32) dot += (double)wn[e] * s * xu * lam[adj[e]];
+    for (ull e = b + lane; e < e1; e += 32) dot += (double)wn[e] * s * xu * lam[adj[e]];
     dot = warp_sum(dot);
     dot = __shfl_sync(FULL, dot, 0);
     const double rs = rowsum[u];
-    for (ull e = idx[u] + lane; e < idx[u + 1]; e += 32) gw[e] = (float)(((double)s * xu * lam[adj[e]] - dot) / rs);
+    for (ull e = b + lane; e < e1; e += 32) gw[e] = (float)(((double)s * xu * lam[adj[e]] - dot) / rs);
+}
+__global__ void k_wgradsum(ull nseg, const WRowSeg* seg, const int* adj, const float* wn, const float* x,
+                           const float* lam, float s, double* rowdot) {
+    const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= nseg) return;
+    const WRowSeg g = seg[i];
+    const double xu = x[g.row];
+    double dot = 0;
+    for (unsigned j = lane; j < g.len; j += 32) dot += (double)wn[g.base + j] * s * xu * lam[adj[g.base + j]];
+    dot = warp_sum(dot);
+    if (lane == 0) atomicAdd(&rowdot[g.row], dot);
+}
+__global__ void k_wgradseg(ull nseg, const WRowSeg* seg, const int* adj, const double* rowsum, const float* x,
+                           const float* lam, float s, const double* rowdot, float* gw) {
+    const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= nseg) return;
+    const WRowSeg g = seg[i];
+    const double xu = x[g.row], dot = rowdot[g.row], rs = rowsum[g.row];
+    for (unsigned j = lane; j < g.len; j += 32)
+        gw[g.base + j] = (float)(((double)s * xu * lam[adj[g.base + j]] - dot) / rs);
 }
 
 __global__ void k_wscale(int n, const float* in, float f, float* out) {
@@ -270,17 +414,16 @@ struct excent_wgraph {
     float* d_wt = nullptr;        // transposed order
     double* d_wt64 = nullptr;
     float *d_x = nullptr, *d_r = nullptr, *d_lam = nullptr;
-    uint32_t* d_t[2] = {nullptr, nullptr};
+    WSegment* d_seg = nullptr;    // queue of long-list segments of one pass (either direction)
+    ull seg_cap = 0;
+    WRowSeg* d_rowseg = nullptr;  // rows of the forward graph longer than WLONG
+    ull n_rowseg = 0;
+    double* d_rowdot = nullptr;
     WCtrl* d_ctrl = nullptr;
     double *d_v64[2] = {nullptr, nullptr};
     ull* d_mx = nullptr;
     double* d_red = nullptr;
     cudaStream_t st = nullptr;
-    cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // forward, adjoint
-    cudaGraph_t graph[2] = {nullptr, nullptr};
-    int gmax[2] = {-1, -1};
-    float geps[2] = {-1, -1}, gs[2] = {0, 0};
-    int grid = 0;
     bool have_fwd = false;
     bool host_t = false;          // transposed lists and weights in pinned, mapped host memory
     int* h_adjT = nullptr;
@@ -291,20 +434,9 @@ struct excent_wgraph {
     ull launches = 0;
 };
 
-static void wg_drop_graphs(excent_wgraph* g) {
-    for (int k = 0; k < 2; k++) {
-        if (g->gexec[k]) cudaGraphExecDestroy(g->gexec[k]);
-        if (g->graph[k]) cudaGraphDestroy(g->graph[k]);
-        g->gexec[k] = nullptr;
-        g->graph[k] = nullptr;
-        g->gmax[k] = -1;
-    }
-}
-
 static void wg_free(excent_wgraph* g) {
     cudaSetDevice(g->dev);
     cudaDeviceSynchronize();
-    wg_drop_graphs(g);
     if (g->host_t) {
         cudaFreeHost(g->h_adjT);
         cudaFreeHost(g->h_wt);
@@ -312,7 +444,7 @@ static void wg_free(excent_wgraph* g) {
         g->d_adjT = nullptr; g->d_wt = nullptr; g->d_wt64 = nullptr;
     }
     void* ps[] = {g->d_wn, g->d_wn64, g->d_rowsum, g->d_idxT, g->d_adjT, g->d_perm, g->d_inv, g->d_wt, g->d_wt64,
-                  g->d_x, g->d_r, g->d_lam, g->d_t[0], g->d_t[1], g->d_ctrl, g->d_v64[0], g->d_v64[1], g->d_mx,
+                  g->d_x, g->d_r, g->d_lam, g->d_seg, g->d_rowseg, g->d_rowdot, g->d_ctrl, g->d_v64[0], g->d_v64[1], g->d_mx,
                   g->d_red};
     for (void* p : ps) if (p) cudaFree(p);
     if (g->st) cudaStreamDestroy(g->st);
@@ -322,9 +454,17 @@ static void wg_free(excent_wgraph* g) {
 #define WG_ALLOC(ptr, bytes) do { if (cudaMalloc((void**)&(ptr), (bytes)) != cudaSuccess) { cudaGetLastError(); \
     ::excent::set_error("wgraph: device allocation of %llu bytes failed (%s)", (ull)(bytes), #ptr); return EXCENT_ERR_NOMEM; } } while (0)
 
+static unsigned seg_blocks(const excent_wgraph* g) { return (unsigned)((g->n_rowseg * 32 + WB - 1) / WB); }
+
 static int wg_normalise(excent_wgraph* g) {
     const unsigned wb = (unsigned)(((long long)g->n * 32 + WB - 1) / WB);
     k_wnorm<<<wb, WB, 0, g->st>>>(g->n, g->d_idx, g->d_wraw, g->d_wn, g->d_wn64, g->d_rowsum);
+    if (g->n_rowseg) {
+        const unsigned sb = seg_blocks(g);
+        k_wsegsum<<<sb, WB, 0, g->st>>>(g->n_rowseg, g->d_rowseg, g->d_wraw, g->d_rowsum);
+        k_wsegnorm<<<sb, WB, 0, g->st>>>(g->n_rowseg, g->d_rowseg, g->d_wraw, g->d_rowsum, g->d_wn, g->d_wn64);
+        g->launches += 2;
+    }
     if (g->m) k_wpermute<<<2048, WB, 0, g->st>>>(g->m, g->d_perm, g->d_wn, g->d_wn64, g->d_wt, g->d_wt64);
     g->launches += 2;
     EX_CUDA(cudaGetLastError());
@@ -353,9 +493,10 @@ static int wg_setup(excent_wgraph* g, int device, int n, ull m, const ull* d_idx
     WG_ALLOC(g->d_x, (size_t)n * 4);
     WG_ALLOC(g->d_r, (size_t)n * 4);
     WG_ALLOC(g->d_lam, (size_t)n * 4);
-    const size_t words = ((size_t)n + 31) / 32;
-    WG_ALLOC(g->d_t[0], words * 4);
-    WG_ALLOC(g->d_t[1], words * 4);
+    // every list longer than WLONG in one pass: at most m / WSEG full segments and one more per such list
+    g->seg_cap = m / WSEG + m / WLONG + 1;
+    WG_ALLOC(g->d_seg, g->seg_cap * sizeof(WSegment));
+    WG_ALLOC(g->d_rowdot, (size_t)n * 8);
     WG_ALLOC(g->d_ctrl, sizeof(WCtrl));
     WG_ALLOC(g->d_mx, 2 * sizeof(ull));
     WG_ALLOC(g->d_red, sizeof(double));
@@ -398,16 +539,15 @@ static int wg_setup(excent_wgraph* g, int device, int n, ull m, const ull* d_idx
     if (v0) cudaFree(v0);
     if (tmp) cudaFree(tmp);
     if (rc != EXCENT_OK) return rc;
-    // inverse permutation (forward edge -> transposed edge), on the host once
+    // inverse permutation (forward edge -> transposed edge), and the long rows
     if (m) {
-        std::vector<unsigned> perm(m), inv(m);
-        EX_CUDA(cudaMemcpy(perm.data(), g->d_perm, m * 4, cudaMemcpyDeviceToHost));
-        for (ull i = 0; i < m; i++) inv[perm[i]] = (unsigned)i;
-        EX_CUDA(cudaMemcpy(g->d_inv, inv.data(), m * 4, cudaMemcpyHostToDevice));
+        k_winverse<<<2048, WB, 0, g->st>>>(m, g->d_perm, g->d_inv);
+        WG_ALLOC(g->d_rowseg, g->seg_cap * sizeof(WRowSeg));
+        EX_CUDA(cudaMemsetAsync(g->d_mx, 0, sizeof(ull), g->st));
+        k_wrowsegs<<<g->sms * 8, WB, 0, g->st>>>(n, d_idx, g->d_rowseg, g->d_mx);
+        EX_CUDA(cudaMemcpyAsync(&g->n_rowseg, g->d_mx, sizeof(ull), cudaMemcpyDeviceToHost, g->st));
+        EX_CUDA(cudaStreamSynchronize(g->st));
     }
-    int occ = 0;
-    EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wpass, WB, 0));
-    g->grid = g->sms * std::max(1, occ);
     return wg_normalise(g);
 }
 
@@ -446,8 +586,7 @@ static WArgs wargs(excent_wgraph* g, bool transposed, float s, float eps, float*
     a.adj = transposed ? g->d_adjT : g->d_adj;
     a.wt = transposed ? g->d_wt : g->d_wn;
     a.s = s; a.eps = eps; a.x = x; a.r = r;
-    a.touched[0] = g->d_t[0]; a.touched[1] = g->d_t[1];
-    a.words = (int)(((size_t)g->n + 31) / 32);
+    a.seg = g->d_seg; a.seg_cap = g->seg_cap;
     a.ctrl = g->d_ctrl;
     return a;
 }
@@ -456,50 +595,18 @@ static WArgs wargs(excent_wgraph* g, bool transposed, float s, float eps, float*
 // (forward lists) or W (transposed lists). Result in x.
 static int wg_push(excent_wgraph* g, bool transposed, float s, float eps, int max_passes, const float* seed, float c0,
                    float* x, int* passes, ull* pushed) {
-    const size_t words = ((size_t)g->n + 31) / 32;
-    EX_CUDA(cudaMemsetAsync(g->d_t[0], 0, words * 4, g->st));
-    EX_CUDA(cudaMemsetAsync(g->d_t[1], 0, words * 4, g->st));
-    k_wseed<<<g->sms * 8, WB, 0, g->st>>>(g->n, seed, c0, x, g->d_r, g->d_t[0]);
-    g->launches++;
+    k_wseed<<<g->sms * 8, WB, 0, g->st>>>(g->n, seed, c0, x, g->d_r);
     WCtrl c{};
     c.max_passes = max_passes;
     EX_CUDA(cudaMemcpyAsync(g->d_ctrl, &c, sizeof c, cudaMemcpyHostToDevice, g->st));
-    const int k = transposed ? 1 : 0;
     WArgs a = wargs(g, transposed, s, eps, x, g->d_r);
-    if (!g->gexec[k] || g->gmax[k] != max_passes || g->geps[k] != eps || g->gs[k] != s) {
-        if (g->gexec[k]) { cudaGraphExecDestroy(g->gexec[k]); g->gexec[k] = nullptr; }
-        if (g->graph[k]) { cudaGraphDestroy(g->graph[k]); g->graph[k] = nullptr; }
-        cudaGraph_t gr;
-        EX_CUDA(cudaGraphCreate(&gr, 0));
-        cudaGraphConditionalHandle h;
-        EX_CUDA(cudaGraphConditionalHandleCreate(&h, gr, 1, cudaGraphCondAssignDefault));
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = h;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t node;
-        EX_CUDA(cudaGraphAddNode(&node, gr, nullptr, 0, &cp));
-        cudaStream_t cs;
-        EX_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-        EX_CUDA(cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                              cudaStreamCaptureModeThreadLocal));
-        k_wpass<<<g->grid, WB, 0, cs>>>(a);
-        k_wend<<<1, 1, 0, cs>>>(g->d_ctrl, h, 1);
-        cudaGraph_t captured;
-        const cudaError_t ce = cudaStreamEndCapture(cs, &captured);
-        cudaStreamDestroy(cs);
-        EX_CUDA(ce);
-        EX_CUDA(cudaGraphInstantiate(&g->gexec[k], gr, 0));
-        g->graph[k] = gr;
-        g->gmax[k] = max_passes;
-        g->geps[k] = eps;
-        g->gs[k] = s;
-    }
-    EX_CUDA(cudaGraphLaunch(g->gexec[k], g->st));
+    // one block per SM, fewer where there is not a tile of 32 vertices for each
+    const int grid = (int)std::max(1ll, std::min<long long>(g->sms, ((long long)g->n + 31) / 32));
+    EX_CUDA(launch_grid(k_wsolve, grid, WP, 0, a, &g->d_ctrl->bar, g->st));
+    EX_CUDA(cudaMemcpyAsync(&c, g->d_ctrl, sizeof c, cudaMemcpyDeviceToHost, g->st));
     EX_CUDA(cudaStreamSynchronize(g->st));
-    EX_CUDA(cudaMemcpy(&c, g->d_ctrl, sizeof c, cudaMemcpyDeviceToHost));
-    g->launches += 2ull * (c.pass + 1);
+    g->launches += 2;
+    if (c.bar.failed) EX_FAIL(EXCENT_ERR_STATE, "wgraph: a wait between the blocks of the push timed out");
     if (passes) *passes = c.pass;
     if (pushed) *pushed = c.total_e;
     return EXCENT_OK;
@@ -532,8 +639,17 @@ extern "C" int excent_wgraph_vjp(excent_wgraph* g, const float* d_c, float eps, 
     }
     if (d_grad_w && g->m) {
         const unsigned wb = (unsigned)(((long long)g->n * 32 + WB - 1) / WB);
-        k_wgrad<<<wb, WB, 0, g->st>>>(g->n, g->d_idx, g->d_adj, g->d_wn, g->d_rowsum, g->d_x, g->d_lam, s, d_grad_w);
+        k_wgrad<<<wb, WB, 0, g->st>>>(g->n, g->d_idx, g->d_adj, g->d_wn, g->d_rowsum, g->d_x, g->d_lam, s, d_grad_w,
+                                      g->d_rowdot);
         g->launches++;
+        if (g->n_rowseg) {
+            const unsigned sb = seg_blocks(g);
+            k_wgradsum<<<sb, WB, 0, g->st>>>(g->n_rowseg, g->d_rowseg, g->d_adj, g->d_wn, g->d_x, g->d_lam, s,
+                                             g->d_rowdot);
+            k_wgradseg<<<sb, WB, 0, g->st>>>(g->n_rowseg, g->d_rowseg, g->d_adj, g->d_rowsum, g->d_x, g->d_lam, s,
+                                             g->d_rowdot, d_grad_w);
+            g->launches += 2;
+        }
     }
     EX_CUDA(cudaGetLastError());
     EX_CUDA(cudaStreamSynchronize(g->st));
@@ -676,7 +792,6 @@ extern "C" int excent_wgraph_host_transposed(excent_wgraph* g) {
     if (g->host_t || g->m == 0) return EXCENT_OK;
     EX_CUDA(cudaSetDevice(g->dev));
     EX_CUDA(cudaDeviceSynchronize());
-    wg_drop_graphs(g);
     const unsigned fl = cudaHostAllocMapped | cudaHostAllocPortable;
     int* ha = nullptr;
     float* hw = nullptr;
