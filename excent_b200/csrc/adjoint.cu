@@ -26,76 +26,88 @@
 #include "common.h"
 #include "device.cuh"
 #include "gridsync.cuh"
+#include "pull.cuh"
 
 namespace excent {
 
 static constexpr int WB = 256;
 static constexpr int WP = 1024;             // threads per block of the persistent push, one block per SM
-static constexpr unsigned WLONG = 256;      // longer lists are scattered, summed and scaled as segments ...
-static constexpr unsigned WSEG = 512;       // ... of this many entries, one warp each
 static constexpr int WUNROLL = 4;           // entries per lane in flight
 
 struct WCtrl {
     int pass, max_passes, pad0, pad1;
-    ull pushed_v[2];   // vertices pushed, by pass parity
-    ull nseg[2];       // segments queued, by pass parity
+    ull demand[2];     // entries of the lists of the vertices taken, by pass parity
+    ull taken[2];      // vertices taken
     ull total_e;
     GridBar bar;
 };
 
-// A stretch of one list: the queued scatter of a long list, or (static) the
-// rows that are longer than WLONG.
-struct WSegment {
-    ull base;       // first entry
-    unsigned len;
-    float f;        // scatter weight (queue)
-};
-struct WRowSeg {
-    ull base;
-    unsigned len, row;
+// A weighted CSR: per-entry weight (row-normalised), long lists also as segments.
+struct WLists {
+    const ull* idx;
+    const int* adj;
+    const float* wt;
+    const ListSeg* seg;
+    ull nseg;
 };
 
 struct WArgs {
     int n;
-    const ull* idx;
-    const int* adj;
-    const float* wt;    // per-edge weight (row-normalised, forward or transposed order)
+    WLists out;        // the lists a push scatters along
+    WLists in;         // the transposed lists: what a vertex gathers from
+    ull pull_min;      // passes of at least this demand gather, the others scatter
     float s;
     float eps;
     float* x;
     float* r;
-    WSegment* seg;
-    ull seg_cap;
+    float* d;          // what each vertex had taken in this pass
     WCtrl* ctrl;
 };
 
+struct WGather {
+    const int* adj;
+    const float* wt;
+    const float* d;
+    struct Key { int u = -1; float w = 0.f; };
+    __device__ __forceinline__ Key key(ull e) const {
+        Key k;
+        k.u = ld_edge(adj + e);
+        k.w = __ldcs(wt + e);
+        return k;
+    }
+    __device__ __forceinline__ float value(const Key& k) const {
+        const float q = k.u >= 0 ? d[k.u] : 0.f;
+        return q != 0.f ? k.w * q : 0.f;   // a vertex that pushed nothing delivers nothing, whatever its weights are
+    }
+};
+
 // The whole delta-push in one cooperative launch. A pass is two phases with a
-// grid barrier after each: every vertex above eps is taken and its list
-// scattered (s * d * wt[e] per entry), then the lists longer than WLONG, which
-// the first phase only queued, are scattered one segment per warp.
+// grid barrier after each: every vertex above eps is taken into d; then
+// s * d * wt[e] is delivered along every list, gathered over the transposed
+// lists while at least pull_min entries are to be delivered, scattered below.
+// Both read every short list edge-balanced and the long ones as segments.
 //
-// What bounds it: one red.global per pushed entry, and, in the many passes
-// with little to push, the two barriers and the scan of r (n floats, in L2).
-// A warp's 32 lists are scattered as one stretch of entries with every lane
-// busy, and no warp has more than 32 * WLONG entries: with whole lists on one
-// warp a pass lasted as long as the longest list (69k entries in 540 dependent
-// steps on an R-MAT of 1M vertices, 16.8M entries: 300 ms for forward and
-// gradient together).
+// What bounds it: a gather and 8 bytes per entry in the dense passes, then the
+// latency of the phases (75 us for a dense pass of 16.8M entries). On an R-MAT
+// of 1M vertices and 16.8M entries, forward and gradient together took 305 ms
+// with whole lists on one warp, 58.7 ms scattering them split (38 G entries/s:
+// reductions to the same vertices serialise) and take 14.5 ms gathering
+// (181-196 G entries/s).
 __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const long long gw = (long long)wib * gridDim.x + blockIdx.x;   // neighbouring tiles on different SMs
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     const long long ntiles = ((long long)a.n + 31) / 32;
-    __shared__ ull s_base[WP / 32][32];   // per warp: the tile's nonempty lists, compacted
-    __shared__ unsigned s_ex[WP / 32][32];
-    __shared__ float s_f[WP / 32][32];
-    __shared__ ull s_v[WP / 32];
+    __shared__ PullScratch<float> s_tile[WP / 32];   // per warp: the tile's nonempty lists (acc: push weights)
+    __shared__ ull s_v[WP / 32], s_e[WP / 32];
+    __shared__ unsigned s_next;
+    PullScratch<float>& S = s_tile[wib];
+    const WGather gather{a.in.adj, a.in.wt, a.d};
     unsigned epoch = 0;
-    ull pe = 0;
     const int max_passes = a.ctrl->max_passes;
     for (int pass = 0;; pass++) {
         const int par = pass & 1;
-        ull pv = 0;
+        ull pv = 0, pe = 0;
         for (long long t0 = gw; t0 < ntiles; t0 += 4 * nwarps) {
             float rv[4];   // four tiles' residuals in flight before they are examined
 #pragma unroll
@@ -103,36 +115,75 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
                 const long long v = (t0 + k * nwarps) * 32 + lane;
                 rv[k] = v < a.n ? a.r[v] : 0.f;
             }
-#pragma unroll 1
+#pragma unroll
             for (int k = 0; k < 4; k++) {
-                const float rk = k == 0 ? rv[0] : k == 1 ? rv[1] : k == 2 ? rv[2] : rv[3];
-                if (!__any_sync(FULL, fabsf(rk) > a.eps)) continue;
                 const long long v = (t0 + k * nwarps) * 32 + lane;
-                float d = 0.f;
-                ull b0 = 0;
-                unsigned deg = 0;
-                if (fabsf(rk) > a.eps) {
-                    d = atomicExch(&a.r[v], 0.f);
-                    a.x[v] += d;
-                    if (d != 0.f) {
-                        b0 = a.idx[v];
-                        deg = (unsigned)(a.idx[v + 1] - b0);
-                        pv++;
-                        pe += deg;
+                if (v >= a.n) continue;
+                const bool take = fabsf(rv[k]) > a.eps;
+                a.d[v] = take ? rv[k] : 0.f;
+                if (take) {
+                    a.r[v] = 0.f;
+                    a.x[v] += rv[k];
+                    pv++;
+                    pe += a.out.idx[v + 1] - a.out.idx[v];
+                }
+            }
+        }
+        pv = warp_sum(pv);
+        pe = warp_sum(pe);
+        if (lane == 0) { s_v[wib] = pv; s_e[wib] = pe; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_next = 0;
+            ull tv = 0, te = 0;
+            for (int i = 0; i < WP / 32; i++) { tv += s_v[i]; te += s_e[i]; }
+            if (tv) atomicAdd(&a.ctrl->taken[par], tv);
+            if (te) atomicAdd(&a.ctrl->demand[par], te);
+        }
+        if (!grid_sync(&a.ctrl->bar, epoch)) return;
+        const ull taken = a.ctrl->taken[par], demand = a.ctrl->demand[par];
+        if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next pass's counters: nobody uses them before the barrier
+            a.ctrl->taken[par ^ 1] = 0;
+            a.ctrl->demand[par ^ 1] = 0;
+            a.ctrl->total_e += demand;
+            if (taken) a.ctrl->pass = pass + 1;
+        }
+        if (demand >= a.pull_min && demand) {
+            gather_phase<float>(a.n, a.in.idx, a.in.seg, a.in.nseg, gather, [&](unsigned v, float sum, bool part) {
+                if (sum == 0.f) return;
+                if (part) atomicAdd(&a.r[v], a.s * sum);
+                else a.r[v] += a.s * sum;
+            }, &s_next, S, lane);
+        } else if (demand) {
+            for (ull i = gw; i < a.out.nseg; i += nwarps) {
+                const ListSeg g = a.out.seg[i];
+                const float f = a.s * a.d[g.row];
+                if (f == 0.f) continue;
+                for (unsigned i0 = 0; i0 < g.len; i0 += 32 * WUNROLL) {
+                    int u[WUNROLL];
+                    float w[WUNROLL];
+#pragma unroll
+                    for (int q = 0; q < WUNROLL; q++) {
+                        const unsigned j = i0 + 32 * q + lane;
+                        u[q] = j < g.len ? ld_edge(a.out.adj + g.base + j) : -1;
+                        w[q] = j < g.len ? __ldcs(a.out.wt + g.base + j) : 0.f;
                     }
+#pragma unroll
+                    for (int q = 0; q < WUNROLL; q++)
+                        if (u[q] >= 0) red_add(a.r, u[q], f * w[q]);
                 }
-                const float f = a.s * d;
-                const unsigned nseg = deg > WLONG ? (deg + WSEG - 1) / WSEG : 0u;
-                const unsigned sincl = warp_incl_scan(nseg, lane);
-                const unsigned stot = __shfl_sync(FULL, sincl, 31);
-                if (stot) {   // long lists: one queue reservation per warp
-                    ull at = 0;
-                    if (lane == 0) at = atomicAdd(&a.ctrl->nseg[par], (ull)stot);
-                    at = __shfl_sync(FULL, at, 0) + (sincl - nseg);
-                    for (unsigned i = 0; i < nseg && at + i < a.seg_cap; i++)
-                        a.seg[at + i] = WSegment{b0 + (ull)i * WSEG, min(WSEG, deg - i * WSEG), f};
+            }
+            for (long long tile = gw; tile < ntiles; tile += nwarps) {
+                const long long v = tile * 32 + lane;
+                const float f = v < a.n ? a.s * a.d[v] : 0.f;
+                if (!__any_sync(FULL, f != 0.f)) continue;
+                ull b0 = 0;
+                unsigned ds = 0;
+                if (f != 0.f) {
+                    b0 = a.out.idx[v];
+                    const ull dv = a.out.idx[v + 1] - b0;
+                    ds = dv > PULL_LONG ? 0u : (unsigned)dv;
                 }
-                const unsigned ds = nseg ? 0u : deg;
                 const unsigned nz = __ballot_sync(FULL, ds != 0);
                 if (!nz) continue;
                 const unsigned incl = warp_incl_scan(ds, lane);
@@ -140,7 +191,7 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
                 const unsigned ex = incl - ds;
                 if (ds) {
                     const int rank = __popc(nz & ((1u << lane) - 1u));
-                    s_base[wib][rank] = b0; s_ex[wib][rank] = ex; s_f[wib][rank] = f;
+                    S.base[rank] = b0; S.ex[rank] = ex; S.acc[rank] = f;
                 }
                 __syncwarp();
                 const unsigned le = lane == 31 ? FULL : (2u << lane) - 1u;
@@ -157,9 +208,9 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
                         u[q] = -1;
                         w[q] = 0.f;
                         if (j < tot) {
-                            const ull e = s_base[wib][o] + (j - s_ex[wib][o]);
-                            u[q] = ld_edge(a.adj + e);
-                            w[q] = s_f[wib][o] * __ldcs(a.wt + e);
+                            const ull e = S.base[o] + (j - S.ex[o]);
+                            u[q] = ld_edge(a.out.adj + e);
+                            w[q] = S.acc[o] * __ldcs(a.out.wt + e);
                         }
                     }
 #pragma unroll
@@ -169,43 +220,9 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
                 __syncwarp();
             }
         }
-        pv = warp_sum(pv);
-        if (lane == 0) s_v[wib] = pv;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            ull tv = 0;
-            for (int i = 0; i < WP / 32; i++) tv += s_v[i];
-            if (tv) atomicAdd(&a.ctrl->pushed_v[par], tv);
-        }
-        if (!grid_sync(&a.ctrl->bar, epoch)) return;
-        const ull taken = a.ctrl->pushed_v[par], queued = a.ctrl->nseg[par];
-        if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next pass's counters: nobody uses them before the barrier
-            a.ctrl->pushed_v[par ^ 1] = 0;
-            a.ctrl->nseg[par ^ 1] = 0;
-            if (taken) a.ctrl->pass = pass + 1;
-        }
-        const ull nseg = min(queued, a.seg_cap);
-        for (ull i = gw; i < nseg; i += nwarps) {
-            const WSegment g = a.seg[i];
-            for (unsigned i0 = 0; i0 < g.len; i0 += 32 * WUNROLL) {
-                int u[WUNROLL];
-                float w[WUNROLL];
-#pragma unroll
-                for (int q = 0; q < WUNROLL; q++) {
-                    const unsigned j = i0 + 32 * q + lane;
-                    u[q] = j < g.len ? ld_edge(a.adj + g.base + j) : -1;
-                    w[q] = j < g.len ? __ldcs(a.wt + g.base + j) : 0.f;
-                }
-#pragma unroll
-                for (int q = 0; q < WUNROLL; q++)
-                    if (u[q] >= 0) red_add(a.r, u[q], g.f * w[q]);
-            }
-        }
         if (!taken || pass + 1 >= max_passes) break;
         if (!grid_sync(&a.ctrl->bar, epoch)) return;
     }
-    pe = warp_sum(pe);
-    if (lane == 0 && pe) atomicAdd(&a.ctrl->total_e, pe);
 }
 
 // x = 0, r = c0 * t (t NULL: all ones).
@@ -216,19 +233,8 @@ __global__ void k_wseed(int n, const float* t, float c0, float* x, float* r) {
     }
 }
 
-// The rows longer than WLONG as segments, in any order (once per graph).
-__global__ void k_wrowsegs(int n, const ull* idx, WRowSeg* out, ull* cnt) {
-    for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < n; u += (long long)gridDim.x * blockDim.x) {
-        const ull b = idx[u], deg = idx[u + 1] - b;
-        if (deg <= WLONG) continue;
-        const ull k = (deg + WSEG - 1) / WSEG, at = atomicAdd(cnt, k);
-        for (ull i = 0; i < k; i++)
-            out[at + i] = WRowSeg{b + i * WSEG, (unsigned)min((ull)WSEG, deg - i * WSEG), (unsigned)u};
-    }
-}
-
 // Row sums and normalised weights (FP32 for the push, FP64 for the tools): one
-// warp per row of up to WLONG entries. The longer rows start at 0 here; their
+// warp per row of up to PULL_LONG entries. The longer rows start at 0 here; their
 // segments are summed by k_wsegsum and scaled by k_wsegnorm, one warp per
 // segment (a whole row on one warp took 69k / 32 dependent steps, twice).
 __global__ void k_wnorm(int n, const ull* idx, const float* w, float* wn, double* wn64, double* rowsum) {
@@ -236,7 +242,7 @@ __global__ void k_wnorm(int n, const ull* idx, const float* w, float* wn, double
     const int lane = threadIdx.x & 31;
     if (u >= n) return;
     const ull b = idx[u], e1 = idx[u + 1];
-    if (e1 - b > WLONG) {
+    if (e1 - b > PULL_LONG) {
         if (lane == 0) rowsum[u] = 0;
         return;
     }
@@ -251,21 +257,21 @@ __global__ void k_wnorm(int n, const ull* idx, const float* w, float* wn, double
     }
     if (lane == 0) rowsum[u] = s;
 }
-__global__ void k_wsegsum(ull nseg, const WRowSeg* seg, const float* w, double* rowsum) {
+__global__ void k_wsegsum(ull nseg, const ListSeg* seg, const float* w, double* rowsum) {
     const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= nseg) return;
-    const WRowSeg g = seg[i];
+    const ListSeg g = seg[i];
     double s = 0;
     for (unsigned j = lane; j < g.len; j += 32) s += w[g.base + j];
     s = warp_sum(s);
     if (lane == 0) atomicAdd(&rowsum[g.row], s);
 }
-__global__ void k_wsegnorm(ull nseg, const WRowSeg* seg, const float* w, const double* rowsum, float* wn, double* wn64) {
+__global__ void k_wsegnorm(ull nseg, const ListSeg* seg, const float* w, const double* rowsum, float* wn, double* wn64) {
     const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= nseg) return;
-    const WRowSeg g = seg[i];
+    const ListSeg g = seg[i];
     const double s = rowsum[g.row];
     for (unsigned j = lane; j < g.len; j += 32) {
         const double q = (double)w[g.base + j] / s;
@@ -308,7 +314,7 @@ __global__ void k_wkeys(int n, int shift, const ull* idx, const int* adj, uint64
 }
 
 // Gradient through the row normalisation: dL/dw[e] = (G_e - sum wn G) / rowsum
-// with G_e = s x_u lam_v, one warp per row of up to WLONG entries; the longer
+// with G_e = s x_u lam_v, one warp per row of up to PULL_LONG entries; the longer
 // rows' sums are accumulated by k_wgradsum and finished by k_wgradseg.
 __global__ void k_wgrad(int n, const ull* idx, const int* adj, const float* wn, const double* rowsum, const float* x,
                         const float* lam, float s, float* gw, double* rowdot) {
@@ -316,7 +322,7 @@ __global__ void k_wgrad(int n, const ull* idx, const int* adj, const float* wn, 
     const int lane = threadIdx.x & 31;
     if (u >= n) return;
     const ull b = idx[u], e1 = idx[u + 1];
-    if (e1 - b > WLONG) {
+    if (e1 - b > PULL_LONG) {
         if (lane == 0) rowdot[u] = 0;
         return;
     }
@@ -328,24 +334,24 @@ __global__ void k_wgrad(int n, const ull* idx, const int* adj, const float* wn, 
     const double rs = rowsum[u];
     for (ull e = b + lane; e < e1; e += 32) gw[e] = (float)(((double)s * xu * lam[adj[e]] - dot) / rs);
 }
-__global__ void k_wgradsum(ull nseg, const WRowSeg* seg, const int* adj, const float* wn, const float* x,
+__global__ void k_wgradsum(ull nseg, const ListSeg* seg, const int* adj, const float* wn, const float* x,
                            const float* lam, float s, double* rowdot) {
     const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= nseg) return;
-    const WRowSeg g = seg[i];
+    const ListSeg g = seg[i];
     const double xu = x[g.row];
     double dot = 0;
     for (unsigned j = lane; j < g.len; j += 32) dot += (double)wn[g.base + j] * s * xu * lam[adj[g.base + j]];
     dot = warp_sum(dot);
     if (lane == 0) atomicAdd(&rowdot[g.row], dot);
 }
-__global__ void k_wgradseg(ull nseg, const WRowSeg* seg, const int* adj, const double* rowsum, const float* x,
+__global__ void k_wgradseg(ull nseg, const ListSeg* seg, const int* adj, const double* rowsum, const float* x,
                            const float* lam, float s, const double* rowdot, float* gw) {
     const ull i = (blockIdx.x * (ull)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= nseg) return;
-    const WRowSeg g = seg[i];
+    const ListSeg g = seg[i];
     const double xu = x[g.row], dot = rowdot[g.row], rs = rowsum[g.row];
     for (unsigned j = lane; j < g.len; j += 32)
         gw[g.base + j] = (float)(((double)s * xu * lam[adj[g.base + j]] - dot) / rs);
@@ -414,10 +420,10 @@ struct excent_wgraph {
     float* d_wt = nullptr;        // transposed order
     double* d_wt64 = nullptr;
     float *d_x = nullptr, *d_r = nullptr, *d_lam = nullptr;
-    WSegment* d_seg = nullptr;    // queue of long-list segments of one pass (either direction)
-    ull seg_cap = 0;
-    WRowSeg* d_rowseg = nullptr;  // rows of the forward graph longer than WLONG
-    ull n_rowseg = 0;
+    ListSeg* d_rowseg = nullptr;  // the long lists of the forward graph as segments
+    ListSeg* d_colseg = nullptr;  // and of the transposed graph
+    ull n_rowseg = 0, n_colseg = 0;
+    float* d_d = nullptr;         // what a pass has taken
     double* d_rowdot = nullptr;
     WCtrl* d_ctrl = nullptr;
     double *d_v64[2] = {nullptr, nullptr};
@@ -444,7 +450,7 @@ static void wg_free(excent_wgraph* g) {
         g->d_adjT = nullptr; g->d_wt = nullptr; g->d_wt64 = nullptr;
     }
     void* ps[] = {g->d_wn, g->d_wn64, g->d_rowsum, g->d_idxT, g->d_adjT, g->d_perm, g->d_inv, g->d_wt, g->d_wt64,
-                  g->d_x, g->d_r, g->d_lam, g->d_seg, g->d_rowseg, g->d_rowdot, g->d_ctrl, g->d_v64[0], g->d_v64[1], g->d_mx,
+                  g->d_x, g->d_r, g->d_lam, g->d_rowseg, g->d_colseg, g->d_d, g->d_rowdot, g->d_ctrl, g->d_v64[0], g->d_v64[1], g->d_mx,
                   g->d_red};
     for (void* p : ps) if (p) cudaFree(p);
     if (g->st) cudaStreamDestroy(g->st);
@@ -473,6 +479,17 @@ static int wg_normalise(excent_wgraph* g) {
     return EXCENT_OK;
 }
 
+// The long lists of one direction as segments (once per graph).
+static int wg_segments(excent_wgraph* g, const ull* idx, ListSeg** seg, ull* count) {
+    WG_ALLOC(*seg, list_seg_cap(g->m) * sizeof(ListSeg));
+    EX_CUDA(cudaMemsetAsync(g->d_mx, 0, sizeof(ull), g->st));
+    k_list_segs<<<g->sms * 8, WB, 0, g->st>>>(g->n, idx, *seg, g->d_mx);
+    EX_CUDA(cudaGetLastError());
+    EX_CUDA(cudaMemcpyAsync(count, g->d_mx, sizeof(ull), cudaMemcpyDeviceToHost, g->st));
+    EX_CUDA(cudaStreamSynchronize(g->st));
+    return EXCENT_OK;
+}
+
 static int wg_setup(excent_wgraph* g, int device, int n, ull m, const ull* d_idx, const int* d_adj, const float* d_w) {
     EX_CUDA(cudaSetDevice(device));
     g->dev = device;
@@ -493,9 +510,7 @@ static int wg_setup(excent_wgraph* g, int device, int n, ull m, const ull* d_idx
     WG_ALLOC(g->d_x, (size_t)n * 4);
     WG_ALLOC(g->d_r, (size_t)n * 4);
     WG_ALLOC(g->d_lam, (size_t)n * 4);
-    // every list longer than WLONG in one pass: at most m / WSEG full segments and one more per such list
-    g->seg_cap = m / WSEG + m / WLONG + 1;
-    WG_ALLOC(g->d_seg, g->seg_cap * sizeof(WSegment));
+    WG_ALLOC(g->d_d, (size_t)n * 4);
     WG_ALLOC(g->d_rowdot, (size_t)n * 8);
     WG_ALLOC(g->d_ctrl, sizeof(WCtrl));
     WG_ALLOC(g->d_mx, 2 * sizeof(ull));
@@ -539,14 +554,11 @@ static int wg_setup(excent_wgraph* g, int device, int n, ull m, const ull* d_idx
     if (v0) cudaFree(v0);
     if (tmp) cudaFree(tmp);
     if (rc != EXCENT_OK) return rc;
-    // inverse permutation (forward edge -> transposed edge), and the long rows
+    // inverse permutation (forward edge -> transposed edge), and the long lists of both directions
     if (m) {
         k_winverse<<<2048, WB, 0, g->st>>>(m, g->d_perm, g->d_inv);
-        WG_ALLOC(g->d_rowseg, g->seg_cap * sizeof(WRowSeg));
-        EX_CUDA(cudaMemsetAsync(g->d_mx, 0, sizeof(ull), g->st));
-        k_wrowsegs<<<g->sms * 8, WB, 0, g->st>>>(n, d_idx, g->d_rowseg, g->d_mx);
-        EX_CUDA(cudaMemcpyAsync(&g->n_rowseg, g->d_mx, sizeof(ull), cudaMemcpyDeviceToHost, g->st));
-        EX_CUDA(cudaStreamSynchronize(g->st));
+        EX_TRY(wg_segments(g, d_idx, &g->d_rowseg, &g->n_rowseg));
+        EX_TRY(wg_segments(g, g->d_idxT, &g->d_colseg, &g->n_colseg));
     }
     return wg_normalise(g);
 }
@@ -582,11 +594,14 @@ extern "C" int excent_wgraph_set_weights(excent_wgraph* g, const float* d_w) {
 static WArgs wargs(excent_wgraph* g, bool transposed, float s, float eps, float* x, float* r) {
     WArgs a{};
     a.n = g->n;
-    a.idx = transposed ? g->d_idxT : g->d_idx;
-    a.adj = transposed ? g->d_adjT : g->d_adj;
-    a.wt = transposed ? g->d_wt : g->d_wn;
-    a.s = s; a.eps = eps; a.x = x; a.r = r;
-    a.seg = g->d_seg; a.seg_cap = g->seg_cap;
+    const WLists fwd{g->d_idx, g->d_adj, g->d_wn, g->d_rowseg, g->n_rowseg};
+    const WLists tr{g->d_idxT, g->d_adjT, g->d_wt, g->d_colseg, g->n_colseg};
+    a.out = transposed ? tr : fwd;
+    a.in = transposed ? fwd : tr;
+    // a gather reads every list, at about four times the scatter's rate; where one direction's
+    // lists lie in host memory, the solve stays with the other
+    a.pull_min = g->host_t ? (transposed ? 0 : ~0ull) : g->m / 4;
+    a.s = s; a.eps = eps; a.x = x; a.r = r; a.d = g->d_d;
     a.ctrl = g->d_ctrl;
     return a;
 }
