@@ -36,8 +36,8 @@ static constexpr int WUNROLL = 4;           // entries per lane in flight
 
 struct WCtrl {
     int pass, max_passes, pad0, pad1;
-    ull demand[2];     // entries of the lists of the vertices taken, by pass parity
-    ull taken[2];      // vertices taken
+    ull demand[2];     // entries of the lists of the vertices above eps, by pass parity
+    ull above[2];      // vertices above eps
     ull total_e;
     GridBar bar;
 };
@@ -55,12 +55,13 @@ struct WArgs {
     int n;
     WLists out;        // the lists a push scatters along
     WLists in;         // the transposed lists: what a vertex gathers from
-    ull pull_min;      // passes of at least this demand gather, the others scatter
+    ull m;
+    ull pull_min;      // a pass after one of at least this demand gathers, the others scatter
     float s;
     float eps;
     float* x;
     float* r;
-    float* d;          // what each vertex had taken in this pass
+    float* d;          // what each vertex had taken in this pass (0 at the start)
     WCtrl* ctrl;
 };
 
@@ -82,10 +83,16 @@ struct WGather {
 };
 
 // The whole delta-push in one cooperative launch. A pass is two phases with a
-// grid barrier after each: every vertex above eps is taken into d; then
-// s * d * wt[e] is delivered along every list, gathered over the transposed
-// lists while at least pull_min entries are to be delivered, scattered below.
-// Both read every short list edge-balanced and the long ones as segments.
+// grid barrier after each: residuals are taken into d; then s * d * wt[e] is
+// delivered along every list. It gathers over the transposed lists while the
+// pass before had at least pull_min entries to deliver, and scatters below
+// that; both read the short lists edge-balanced and the long ones as segments.
+// A gather reads every list anyway, so its passes take every residual, not
+// only those above eps. What such passes leave is nearly the same everywhere,
+// where a push leaves anything between 0 and eps, so they go on to eps / 2:
+// four more passes, and an error below the push's (to eps itself it was a
+// third above it, 1.3e-5 against 9.8e-6 in dL/dt of 1M vertices). x gets what a pass has taken in the next one, so that a pass that
+// finds nothing above eps ends the solve with nothing taken.
 //
 // What bounds it: a gather and 8 bytes per entry in the dense passes, then the
 // latency of the phases (75 us for a dense pass of 16.8M entries). On an R-MAT
@@ -105,25 +112,28 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
     const WGather gather{a.in.adj, a.in.wt, a.d};
     unsigned epoch = 0;
     const int max_passes = a.ctrl->max_passes;
+    bool pull = a.pull_min <= a.m;
     for (int pass = 0;; pass++) {
         const int par = pass & 1;
         ull pv = 0, pe = 0;
         for (long long t0 = gw; t0 < ntiles; t0 += 4 * nwarps) {
-            float rv[4];   // four tiles' residuals in flight before they are examined
+            float rv[4], dv[4];   // four tiles in flight before they are examined
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const long long v = (t0 + k * nwarps) * 32 + lane;
                 rv[k] = v < a.n ? a.r[v] : 0.f;
+                dv[k] = v < a.n ? a.d[v] : 0.f;
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const long long v = (t0 + k * nwarps) * 32 + lane;
                 if (v >= a.n) continue;
-                const bool take = fabsf(rv[k]) > a.eps;
-                a.d[v] = take ? rv[k] : 0.f;
-                if (take) {
-                    a.r[v] = 0.f;
-                    a.x[v] += rv[k];
+                if (dv[k] != 0.f) a.x[v] += dv[k];
+                const bool above = fabsf(rv[k]) > a.eps;
+                const float d = above || pull ? rv[k] : 0.f;
+                if (d != 0.f) a.r[v] = 0.f;
+                if (d != 0.f || dv[k] != 0.f) a.d[v] = d;
+                if (above) {
                     pv++;
                     pe += a.out.idx[v + 1] - a.out.idx[v];
                 }
@@ -137,18 +147,19 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
             s_next = 0;
             ull tv = 0, te = 0;
             for (int i = 0; i < WP / 32; i++) { tv += s_v[i]; te += s_e[i]; }
-            if (tv) atomicAdd(&a.ctrl->taken[par], tv);
+            if (tv) atomicAdd(&a.ctrl->above[par], tv);
             if (te) atomicAdd(&a.ctrl->demand[par], te);
         }
         if (!grid_sync(&a.ctrl->bar, epoch)) return;
-        const ull taken = a.ctrl->taken[par], demand = a.ctrl->demand[par];
+        const ull above = a.ctrl->above[par], demand = a.ctrl->demand[par];
+        if (!above) break;
         if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next pass's counters: nobody uses them before the barrier
-            a.ctrl->taken[par ^ 1] = 0;
+            a.ctrl->above[par ^ 1] = 0;
             a.ctrl->demand[par ^ 1] = 0;
-            a.ctrl->total_e += demand;
-            if (taken) a.ctrl->pass = pass + 1;
+            a.ctrl->total_e += pull ? a.m : demand;
+            a.ctrl->pass = pass + 1;
         }
-        if (demand >= a.pull_min && demand) {
+        if (pull) {
             gather_phase<float>(a.n, a.in.idx, a.in.seg, a.in.nseg, gather, [&](unsigned v, float sum, bool part) {
                 if (sum == 0.f) return;
                 if (part) atomicAdd(&a.r[v], a.s * sum);
@@ -220,15 +231,22 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
                 __syncwarp();
             }
         }
-        if (!taken || pass + 1 >= max_passes) break;
+        pull = demand >= a.pull_min;
         if (!grid_sync(&a.ctrl->bar, epoch)) return;
+        if (pass + 1 >= max_passes) {   // out of passes: x gets what this one has taken
+            for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < a.n;
+                 v += (long long)gridDim.x * blockDim.x)
+                a.x[v] += a.d[v];
+            break;
+        }
     }
 }
 
-// x = 0, r = c0 * t (t NULL: all ones).
-__global__ void k_wseed(int n, const float* t, float c0, float* x, float* r) {
+// x = d = 0, r = c0 * t (t NULL: all ones).
+__global__ void k_wseed(int n, const float* t, float c0, float* x, float* r, float* d) {
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
         x[v] = 0.f;
+        d[v] = 0.f;
         r[v] = c0 * (t ? t[v] : 1.f);
     }
 }
@@ -593,7 +611,7 @@ extern "C" int excent_wgraph_set_weights(excent_wgraph* g, const float* d_w) {
 
 static WArgs wargs(excent_wgraph* g, bool transposed, float s, float eps, float* x, float* r) {
     WArgs a{};
-    a.n = g->n;
+    a.n = g->n; a.m = g->m;
     const WLists fwd{g->d_idx, g->d_adj, g->d_wn, g->d_rowseg, g->n_rowseg};
     const WLists tr{g->d_idxT, g->d_adjT, g->d_wt, g->d_colseg, g->n_colseg};
     a.out = transposed ? tr : fwd;
@@ -601,7 +619,7 @@ static WArgs wargs(excent_wgraph* g, bool transposed, float s, float eps, float*
     // a gather reads every list, at about four times the scatter's rate; where one direction's
     // lists lie in host memory, the solve stays with the other
     a.pull_min = g->host_t ? (transposed ? 0 : ~0ull) : g->m / 4;
-    a.s = s; a.eps = eps; a.x = x; a.r = r; a.d = g->d_d;
+    a.s = s; a.eps = a.pull_min <= g->m && 0.5f * eps > 0.f ? 0.5f * eps : eps; a.x = x; a.r = r; a.d = g->d_d;
     a.ctrl = g->d_ctrl;
     return a;
 }
@@ -610,7 +628,7 @@ static WArgs wargs(excent_wgraph* g, bool transposed, float s, float eps, float*
 // (forward lists) or W (transposed lists). Result in x.
 static int wg_push(excent_wgraph* g, bool transposed, float s, float eps, int max_passes, const float* seed, float c0,
                    float* x, int* passes, ull* pushed) {
-    k_wseed<<<g->sms * 8, WB, 0, g->st>>>(g->n, seed, c0, x, g->d_r);
+    k_wseed<<<g->sms * 8, WB, 0, g->st>>>(g->n, seed, c0, x, g->d_r, g->d_d);
     WCtrl c{};
     c.max_passes = max_passes;
     EX_CUDA(cudaMemcpyAsync(g->d_ctrl, &c, sizeof c, cudaMemcpyHostToDevice, g->st));
