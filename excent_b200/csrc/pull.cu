@@ -8,6 +8,7 @@ __global__ void k_list_segs(int n, const ull* idx, ListSeg* out, ull* cnt) {
         const ull b = idx[u], deg = idx[u + 1] - b;
         if (deg <= PULL_LONG) continue;
         const ull k = (deg + PULL_SEG - 1) / PULL_SEG, at = atomicAdd(cnt, k);
+        if (!out) continue;
         for (ull i = 0; i < k; i++)
             out[at + i] = ListSeg{b + i * PULL_SEG, (unsigned)min((ull)PULL_SEG, deg - i * PULL_SEG), (unsigned)u};
     }

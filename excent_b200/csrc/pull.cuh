@@ -156,7 +156,7 @@ __device__ __forceinline__ void gather_phase(int n, const ull* idx, const ListSe
     }
 }
 
-// The lists longer than PULL_LONG as segments, in any order.
+// The lists longer than PULL_LONG as segments, in any order (out null: their number alone).
 __global__ void k_list_segs(int n, const ull* idx, ListSeg* out, ull* cnt);
 // At most this many segments in a graph of m entries.
 static inline ull list_seg_cap(ull m) { return m / PULL_SEG + m / PULL_LONG + 1; }
