@@ -20,6 +20,7 @@
 
 #include "common.h"
 #include "device.cuh"
+#include "gridsync.cuh"
 
 namespace excent {
 
@@ -54,6 +55,16 @@ struct PushQueue {
 static constexpr int TILE_BATCH = 32;           // at most this many tiles (of 32 items) per claim
 static constexpr unsigned SPIN_LIMIT = 1u << 24; // bounded polls of an mbarrier
 
+// What a snapshot of the persistent solve adds up, and the queue counters of
+// one of its take phases.
+struct SnapAcc {
+    double rsum[MAXM];
+    double ev_dot;
+};
+struct WaveCount {
+    unsigned small, big, claim, pad;
+};
+
 // Device control block: counters that live across kernels of one pass.
 struct Ctrl {
     ull hotpend;
@@ -69,9 +80,12 @@ struct Ctrl {
     double ev_dot;     // FP64 (r_ev . v1) accumulated by the snapshot
     double ev_corr;    // component removed from r_ev by the next snapshot
     ull host_pushed;   // entries pushed from lists read in place in host memory
-    ull chunk_runs;    // chunk launches a sweeping solve ran (chunks with items, summed over passes)
+    ull sweeps;        // passes that went chunk by chunk
     ull lanes;         // sum over pushed lists of entries x measures carrying a nonzero weight
     ull taken;         // sum over pushed vertices of the measures taken
+    SnapAcc acc[2];    // persistent solve: by pass parity
+    WaveCount wave[3]; // by take phase
+    GridBar bar;
 };
 
 struct PassRec {
@@ -203,32 +217,33 @@ __device__ __forceinline__ int chunk_of(long long v, const int* cv0, int nc) {
     return lo;
 }
 
-// Demand snapshot. Each warp owns a contiguous run of 16-word groups; per
-// group it ballots 512 vertices (one bitmap word per 32), writes the words
+// Demand snapshot of groups [g0, g1) of `group` words by one warp. Per
+// group it ballots its vertices (one bitmap word per 32), writes the words
 // coalesced, and adds the group's pending count and degree sum to its chunk
 // with one atomic pair (per-lane atomics only where a group straddles a chunk
 // boundary). The same atomic returns the offset at which the group's pending
 // ids are appended to the chunk's list region list[cv0[c] ..]. Integer
 // outputs equal src/excent.cu:69-98 exactly; list order is not defined.
+struct SnapSums {
+    double rs0 = 0, rs1 = 0, rs2 = 0, evd = 0;
+    unsigned hp = 0;
+};
 template <int L>
-__global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
+__device__ __forceinline__ void snapshot_scan(const SnapArgs& a, ull* cnt, int group, long long g0, long long g1,
+                                              double evc_in, SnapSums& sums, int lane) {
     typedef typename Lane<L>::T T;
     T* r = reinterpret_cast<T*>(a.r);
-    const int lane = threadIdx.x & 31;
-    const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long ngroups = (a.words + SNAP_GROUP - 1) / SNAP_GROUP;
-    long long g0 = gw * a.groups_per_warp, g1 = g0 + a.groups_per_warp;
+    const long long ngroups = (a.words + group - 1) / group;
     if (g1 > ngroups) g1 = ngroups;
     double rs0 = 0, rs1 = 0, rs2 = 0, evd = 0;
     // the v1 component measured by the previous snapshot is removed here only once it
     // matters (|c| max|v1| above a thousandth of eps); until then the residuals stay as
     // stored and the next dot product measures the component again, carried over
-    const double evc_in = a.v1 ? a.ctrl->ev_corr : 0.0;
     const double evc = fabs(evc_in) > a.ev_skip ? evc_in : 0.0;
     unsigned hp = 0;
     for (long long g = g0; g < g1; g++) {
-        const long long w0 = g * SNAP_GROUP;
-        const int nw = (int)min((long long)SNAP_GROUP, (long long)a.words - w0);
+        const long long w0 = g * group;
+        const int nw = (int)min((long long)group, (long long)a.words - w0);
         uint32_t myb = 0;
         ull mydeg = 0;
         for (int j4 = 0; j4 < nw; j4 += 4) {
@@ -292,8 +307,8 @@ __global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
             const ull dsum = warp_sum(mydeg);
             unsigned base = 0;
             if (lane == 0) {
-                base = (unsigned)atomicAdd(&a.cnt[2 * c], (ull)tot);
-                atomicAdd(&a.cnt[2 * c + 1], dsum);
+                base = (unsigned)atomicAdd(&cnt[2 * c], (ull)tot);
+                atomicAdd(&cnt[2 * c + 1], dsum);
             }
             base = __shfl_sync(FULL, base, 0);
             const unsigned excl = warp_incl_scan(cl, lane) - cl;
@@ -320,8 +335,8 @@ __global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
                     const ull ds = __shfl_sync(FULL, warp_sum(d), 0);
                     unsigned base = 0;
                     if (lane == leader) {
-                        base = (unsigned)atomicAdd(&a.cnt[2 * cl2], (ull)__popc(mm));
-                        atomicAdd(&a.cnt[2 * cl2 + 1], ds);
+                        base = (unsigned)atomicAdd(&cnt[2 * cl2], (ull)__popc(mm));
+                        atomicAdd(&cnt[2 * cl2 + 1], ds);
                     }
                     base = __shfl_sync(FULL, base, leader);
                     if ((mm >> lane) & 1u) a.list[a.cv0[cl2] + base + __popc(mm & ((1u << lane) - 1u))] = (int)v;
@@ -330,6 +345,18 @@ __global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
             }
         }
     }
+    sums.rs0 += rs0; sums.rs1 += rs1; sums.rs2 += rs2; sums.evd += evd; sums.hp += hp;
+}
+
+template <int L>
+__global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
+    const int lane = threadIdx.x & 31;
+    const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    SnapSums sums;
+    snapshot_scan<L>(a, a.cnt, SNAP_GROUP, gw * a.groups_per_warp, (gw + 1) * a.groups_per_warp,
+                     a.v1 ? a.ctrl->ev_corr : 0.0, sums, lane);
+    double rs0 = sums.rs0, rs1 = sums.rs1, rs2 = sums.rs2, evd = sums.evd;
+    unsigned hp = sums.hp;
     // FP64 termination residual and hot pending count: block reduction, one atomic each
     __shared__ double s_rs[4][BLOCK / 32];
     __shared__ unsigned s_hp[BLOCK / 32];
@@ -351,21 +378,20 @@ __global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
     }
 }
 
-// On-device fetch plan for a fully cached graph: per chunk with pending
+// On-device fetch plan of the host-driven loop: per chunk with pending
 // vertices choose its pending list (cnt < list_frac * vertices) or its whole
 // range (src/excent.cu:639), build the item prefix, log the pass, decide
-// termination (src/excent.cu:680, max passes :656), reset the counters the
-// next snapshot accumulates into, and set the graph's loop condition.
+// termination (src/excent.cu:680, max passes :656), and reset the counters the
+// next snapshot accumulates into.
 __global__ void k_plan(int nc, const int* cv0, int n, ull* cnt, const uint8_t* cmode, double list_frac, int max_passes,
                        uint8_t* wt_type, unsigned* wt_prefix, Ctrl* ctrl, PushQueue* q0, PassRec* log, int log_cap,
-                       cudaGraphConditionalHandle cond, int use_cond, const cudaGraphConditionalHandle* chunk_if,
                        int sweep, ull sweep_min) {
     __shared__ ull s_pend, s_dem;
     __shared__ unsigned s_carry;
-    __shared__ int s_nl, s_nr, s_runs;
+    __shared__ int s_nl, s_nr;
     __shared__ unsigned s_scan[1024];
     const int t = threadIdx.x;
-    if (t == 0) { s_pend = 0; s_dem = 0; s_carry = 0; s_nl = 0; s_nr = 0; s_runs = 0; }
+    if (t == 0) { s_pend = 0; s_dem = 0; s_carry = 0; s_nl = 0; s_nr = 0; }
     __syncthreads();
     ull lp = 0, ld = 0;
     for (int c = t; c < nc; c += blockDim.x) { lp += cnt[2 * c]; ld += cnt[2 * c + 1]; }
@@ -404,8 +430,6 @@ __global__ void k_plan(int nc, const int* cv0, int n, ull* cnt, const uint8_t* c
         if (c < nc) {
             wt_type[c] = ty;
             wt_prefix[c + 1] = s_carry + s_scan[t];
-            if (chunk_if) cudaGraphSetConditional(chunk_if[c], sweep_pass && items ? 1u : 0u);   // launch it?
-            if (sweep_pass && items) atomicAdd(&s_runs, 1);
         }
         if (c == 0) wt_prefix[0] = 0;
         __syncthreads();
@@ -422,17 +446,13 @@ __global__ void k_plan(int nc, const int* cv0, int n, ull* cnt, const uint8_t* c
             R.n_list = s_nl; R.n_range = s_nr;
         }
         ctrl->items = stop ? 0 : s_carry;
-        // pushes launched this pass: one per chunk with items, or the one whole-table push
-        ctrl->chunk_runs += sweep_pass ? s_runs : (sweep && !stop && s_carry ? 1 : 0);
         ctrl->sweep_pass = sweep_pass ? 1 : 0;
-        if (chunk_if) cudaGraphSetConditional(chunk_if[nc], sweep && !stop && !sweep_pass && s_carry ? 1u : 0u);
         if (stop) ctrl->done = 1; else ctrl->pass = p + 1;
         q0->tail = 0; q0->claim = 0;
         ctrl->hotpend = 0;
         ctrl->ev_corr = ctrl->ev_dot;
         ctrl->ev_dot = 0;
         if (!stop) for (int k = 0; k < MAXM; k++) ctrl->rsum[k] = 0;
-        if (use_cond) cudaGraphSetConditional(cond, stop ? 0u : 1u);
     }
     // zero the demand table for the next snapshot (after everyone read it)
     __syncthreads();
@@ -752,20 +772,47 @@ __global__ void k_fill_hot(int lo, int hi, const int* hids, const ull* hoff, con
 }
 
 
-// Vertices whose lists are longer than HUB_MIN, appended in any order.
-__global__ void k_hub_list(int n, const ull* idx, int* out, ull* cnt) {
-    const int lane = threadIdx.x & 31;
-    for (long long v0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) & ~31ll; v0 < n;
-         v0 += (long long)gridDim.x * blockDim.x) {
-        const long long v = v0 + lane;
-        const bool h = v < n && idx[v + 1] - idx[v] > HUB_MIN;
+// Vertices whose lists are longer than HUB_MIN, in ascending order: each block
+// counts a contiguous range (out null), k_hub_scan turns the counts into
+// offsets, and each block writes its range's from there.
+static constexpr int HUB_BLOCKS = 1024;
+__global__ void __launch_bounds__(BLOCK) k_hub_list(int n, const ull* idx, ull* counts, int* out) {
+    __shared__ unsigned s_w[BLOCK / 32];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const long long per = ((long long)n + HUB_BLOCKS - 1) / HUB_BLOCKS;
+    const long long v0 = blockIdx.x * per, v1 = min(v0 + per, (long long)n);
+    ull at = out ? counts[blockIdx.x] : 0;
+    for (long long base = v0; base < v1; base += BLOCK) {
+        const long long v = base + threadIdx.x;
+        const bool h = v < v1 && idx[v + 1] - idx[v] > HUB_MIN;
         const unsigned b = __ballot_sync(FULL, h);
-        if (!b) continue;
-        ull base = 0;
-        if (lane == 0) base = atomicAdd(cnt, (ull)__popc(b));
-        base = __shfl_sync(FULL, base, 0);
-        if (h && out) out[base + __popc(b & ((1u << lane) - 1u))] = (int)v;
+        if (lane == 0) s_w[wib] = __popc(b);
+        __syncthreads();
+        unsigned before = 0, all = 0;
+        for (int w = 0; w < BLOCK / 32; w++) {
+            if (w < wib) before += s_w[w];
+            all += s_w[w];
+        }
+        if (h && out) out[at + before + __popc(b & ((1u << lane) - 1u))] = (int)v;
+        at += all;
+        __syncthreads();
     }
+    if (!out && threadIdx.x == 0) counts[blockIdx.x] = at;
+}
+__global__ void __launch_bounds__(HUB_BLOCKS) k_hub_scan(ull* counts, ull* total) {
+    __shared__ ull s_w[HUB_BLOCKS / 32];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const ull c = counts[threadIdx.x];
+    ull v = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const ull t = __shfl_up_sync(FULL, v, o);
+        if (lane >= o) v += t;
+    }
+    if (lane == 31) s_w[wib] = v;
+    __syncthreads();
+    for (int w = 0; w < wib; w++) v += s_w[w];
+    counts[threadIdx.x] = v - c;
+    if (threadIdx.x == HUB_BLOCKS - 1) *total = v;
 }
 
 // Encode / decode the edge cache for hub-target aggregation.
@@ -808,6 +855,8 @@ __global__ void k_insert(int n, float4* s, int i, const float* in) {
 }
 
 }  // namespace excent
+
+#include "passes.cuh"
 
 using namespace excent;
 
@@ -871,8 +920,10 @@ struct excent_engine {
     int claim_tiles = 0;     // tiles per claim of k_push (0: by the launch's size)
     int sweep_mode = -1;     // cached pushes chunk by chunk (1), in one launch (0), -1 by the chunk count
     double sweep_frac = 0.5; // ... only in passes whose pending entries reach sweep_frac * m
-    cudaGraphConditionalHandle* d_chunk_if = nullptr;  // per chunk: does this pass push it (graph IF nodes)
-    std::vector<cudaGraphConditionalHandle> h_chunk_if;
+    ull* d_hub_counts = nullptr;   // scratch of the high-degree list
+    ull* d_cnt2 = nullptr;         // persistent solve: the second demand table
+    HubSeg* d_small = nullptr;     // and the short lists taken together
+    int wave = 0;                  // items its passes take together
     bool hubv_stale = true;
     bool ev_proj = false;
     double ev_skip = 0;      // carry (do not write) a v1 correction of at most this size
@@ -962,7 +1013,7 @@ static int free_engine(excent_engine* e) {
     cudaDeviceSynchronize();
     if (e->gexec) cudaGraphExecDestroy(e->gexec);
     if (e->graph) cudaGraphDestroy(e->graph);
-    void* dptrs[] = {e->d_chunk_if, e->d_hub_id, e->d_hubv, e->d_hubv_cnt, e->d_v1, e->d_idx, e->d_x, e->d_r, e->d_bitmap, e->d_cnt, e->d_cv0, e->d_list, e->d_ctrl, e->d_cmode,
+    void* dptrs[] = {e->d_hub_counts, e->d_cnt2, e->d_small, e->d_hub_id, e->d_hubv, e->d_hubv_cnt, e->d_v1, e->d_idx, e->d_x, e->d_r, e->d_bitmap, e->d_cnt, e->d_cv0, e->d_list, e->d_ctrl, e->d_cmode,
                      e->d_wt_type, e->d_wt_prefix, e->d_hubq[0], e->d_hubq[1], e->d_hubq[2], e->d_queue, e->d_log, e->d_trace, e->d_tmp, e->d_cache,
                      e->d_hids, e->d_hoff, e->d_hedges, e->d_hot, e->d_hlist};
     for (void* p : dptrs) if (p) cudaFree(p);
@@ -991,6 +1042,21 @@ static int free_engine(excent_engine* e) {
     ::excent::set_error("device allocation of %llu bytes failed (%s)", (ull)(bytes), #ptr); return EXCENT_ERR_NOMEM; } } while (0)
 #define EX_HALLOC(ptr, bytes) do { if (cudaMallocHost((void**)&(ptr), (bytes)) != cudaSuccess) { cudaGetLastError(); \
     ::excent::set_error("pinned allocation of %llu bytes failed (%s)", (ull)(bytes), #ptr); return EXCENT_ERR_NOMEM; } } while (0)
+
+// Segments of a wave's longer lists: short ones spread a small graph's lists over more warps;
+// on a large one they only cost queue memory.
+static constexpr ull wave_seg(ull m) { return m < (1ull << 26) ? 256 : HUB_SEG; }
+// Most items of a wave, whatever the occupancy (148 SMs x 2048 threads).
+static constexpr int WAVE_MAX = 1 << 18;
+
+// Blocks of k_push resident at once with `smem` bytes of hub-target slots.
+static int push_blocks(excent_engine* e, size_t smem, int* grid) {
+    int occ = 0;
+    if (e->L == 1) EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push<1, SRC_TABLE>, BLOCK, smem));
+    else EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push<4, SRC_TABLE>, BLOCK, smem));
+    *grid = e->sms * std::max(1, occ);
+    return EXCENT_OK;
+}
 
 static int engine_setup(excent_engine* e, int device, int n, ull m, const excent_measures* ms, int nc,
                         const int* chunk_v0, const ull* chunk_e) {
@@ -1031,7 +1097,8 @@ static int engine_setup(excent_engine* e, int device, int n, ull m, const excent
     EX_ALLOC(e->d_cmode, (size_t)nc);
     EX_ALLOC(e->d_wt_type, (size_t)nc);
     EX_ALLOC(e->d_wt_prefix, ((size_t)nc + 1) * sizeof(unsigned));
-    e->hub_cap[0] = m / HUB_SEG + m / HUB_MIN + 64;
+    // every long list of the graph as segments, and one segment per list of a wave
+    e->hub_cap[0] = m / wave_seg(m) + m / HUB_MIN + WAVE_MAX + 64;
     EX_ALLOC(e->d_hubq[0], e->hub_cap[0] * sizeof(HubSeg));
     EX_ALLOC(e->d_queue, 3 * sizeof(PushQueue));
     e->log_cap = 1 << 17;
@@ -1046,10 +1113,10 @@ static int engine_setup(excent_engine* e, int device, int n, ull m, const excent
     EX_CUDA(cudaMemset(e->d_cnt, 0, 2 * (size_t)nc * sizeof(ull)));
     EX_CUDA(cudaMemset(e->d_cmode, 0, (size_t)nc));
     EX_CUDA(cudaMemset(e->d_queue, 0, 3 * sizeof(PushQueue)));
-    int occ = 0;
-    if (e->L == 1) EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push<1, SRC_TABLE>, BLOCK, 0));
-    else EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push<4, SRC_TABLE>, BLOCK, 0));
-    e->grid_push = e->sms * std::max(1, occ);
+    EX_TRY(push_blocks(e, 0, &e->grid_push));
+    e->wave = std::min(e->grid_push * BLOCK, WAVE_MAX);
+    EX_ALLOC(e->d_cnt2, 2 * (size_t)nc * sizeof(ull));
+    EX_ALLOC(e->d_small, (size_t)std::min(n, WAVE_MAX) * sizeof(HubSeg));
     int occs = 0;
     if (e->L == 1) EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occs, k_snapshot<1>, BLOCK, 0));
     else EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occs, k_snapshot<4>, BLOCK, 0));
@@ -1209,6 +1276,7 @@ static int reset_counters(excent_engine* e) {
     EX_CUDA(cudaMemsetAsync(e->d_ctrl, 0, sizeof(Ctrl), e->s_main));
     EX_CUDA(cudaMemsetAsync(e->d_queue, 0, 3 * sizeof(PushQueue), e->s_main));
     EX_CUDA(cudaMemsetAsync(e->d_cnt, 0, 2 * (size_t)e->nc * sizeof(ull), e->s_main));
+    EX_CUDA(cudaMemsetAsync(e->d_cnt2, 0, 2 * (size_t)e->nc * sizeof(ull), e->s_main));
     if (e->d_trace && e->trace_on) EX_CUDA(cudaMemsetAsync(e->d_trace, 0, (size_t)e->n * sizeof(uint16_t), e->s_main));
     e->hot_skip = false;
     e->n_list = e->n_range = 0;
@@ -1389,7 +1457,7 @@ extern "C" int excent_engine_push_cached(excent_engine* e, const unsigned char* 
     bool all_cached = true;
     for (int c = 0; c < e->nc; c++) all_cached &= cnt[2 * c] == 0 || mode[c] == 1;
     int order = 0;
-    if (order_of(e) == 3) order = 3;
+    if (order_of(e) == 3) order = 3;   // inside each launch: needs no high-degree list
     else if (all_cached && order_of(e) && !sweep_of(e)) {
         EX_TRY(ensure_hubv(e));
         order = effective_order(e);
@@ -1627,9 +1695,9 @@ extern "C" int excent_engine_sync(excent_engine* e) {
     return EXCENT_OK;
 }
 
-// Open an IF node on the stream being captured (condition `h`, set per pass
-// by k_plan) and start capturing its body on `body`; close_if ends the body.
-static cudaError_t open_if(cudaStream_t st, cudaStream_t body, cudaGraphConditionalHandle* h) {
+// Open an IF node with condition `h` on the stream being captured and start
+// capturing its body on `body`; close_if ends the body.
+static cudaError_t open_if(cudaStream_t st, cudaStream_t body, cudaGraphConditionalHandle h) {
     cudaStreamCaptureStatus status;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -1637,11 +1705,9 @@ static cudaError_t open_if(cudaStream_t st, cudaStream_t body, cudaGraphConditio
     cudaError_t rc = cudaStreamGetCaptureInfo(st, &status, nullptr, &g, &deps, &nd);
     if (rc != cudaSuccess) return rc;
     if (status != cudaStreamCaptureStatusActive) return cudaErrorStreamCaptureInvalidated;
-    rc = cudaGraphConditionalHandleCreate(h, g, 0, cudaGraphCondAssignDefault);
-    if (rc != cudaSuccess) return rc;
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = *h;
+    cp.conditional.handle = h;
     cp.conditional.type = cudaGraphCondTypeIf;
     cp.conditional.size = 1;
     cudaGraphNode_t node;
@@ -1657,153 +1723,130 @@ static cudaError_t close_if(cudaStream_t body) {
     return cudaStreamEndCapture(body, &g);
 }
 
-// Kernels of one pass outside the per-chunk launches of a chunk sweep, and per
-// chunk launch (for the launch count of a graph solve).
-static void pass_kernels(const excent_engine* e, int order, ull* fixed, ull* per_chunk) {
-    // kernels of one table push: with segments 2, short lists only 1 (no k_segments)
-    const ull table = order == 3 ? 3 : (order == 1 || order == 2 ? 1 : 2);
-    *fixed = 2 + (order == 1 || order == 2 ? 2 : 0) + (sweep_of(e) ? 0 : table);
-    *per_chunk = sweep_of(e) ? table : 0;
-}
-
-
-// One pass of the device solve: snapshot -> plan -> push -> hub segments.
-// With ev, events are recorded between the kernels. chunk_body (a second
-// stream) is given while the pass is captured into a graph with a chunk
-// sweep: each chunk's launches then sit in an IF node that k_plan switches
-// on for chunks with something to push in a sweeping pass, and the
-// whole-table launch sits in one more IF node, switched on in the other
-// passes; e->h_chunk_if receives the nc + 1 handles.
-static void enqueue_plan(excent_engine* e, double list_frac, int max_passes, cudaGraphConditionalHandle cond,
-                         int use_cond, cudaStream_t st, cudaEvent_t* ev, bool use_if) {
+// One pass of the host-driven loop: snapshot and plan (read back), then the
+// pushes the plan chose. With ev, events are recorded between the kernels.
+static void enqueue_plan(excent_engine* e, double list_frac, int max_passes, cudaStream_t st, cudaEvent_t* ev) {
     if (ev) cudaEventRecord(ev[0], st);
     launch_snapshot(e, false, st);
     if (ev) cudaEventRecord(ev[1], st);
     k_plan<<<1, 1024, 0, st>>>(e->nc, e->d_cv0, e->n, e->d_cnt, e->d_cmode, list_frac, max_passes, e->d_wt_type,
-                               e->d_wt_prefix, e->d_ctrl, e->d_queue, e->d_log, e->log_cap, cond, use_cond,
-                               use_if ? e->d_chunk_if : nullptr, sweep_of(e) ? 1 : 0, sweep_min_entries(e));
+                               e->d_wt_prefix, e->d_ctrl, e->d_queue, e->d_log, e->log_cap, sweep_of(e) ? 1 : 0,
+                               sweep_min_entries(e));
     e->launches++;
     if (ev) cudaEventRecord(ev[2], st);
 }
-
-// The pushes of a pass. sweep_pass: whether k_plan chose a chunk-by-chunk pass
-// (known to the host-driven loop, which reads it back first); ignored while
-// capturing with IF nodes, which hold both forms.
-static cudaError_t enqueue_push(excent_engine* e, cudaStream_t st, cudaEvent_t* ev, cudaStream_t chunk_body,
-                                bool sweep_pass) {
+static cudaError_t enqueue_push(excent_engine* e, cudaStream_t st, cudaEvent_t* ev, bool sweep_pass) {
     PushArgs a = push_args(e, 0);
-    const bool use_if = chunk_body && sweep_of(e);
     // high-degree order: 1 = the lists longer than HUB_MIN first, so their (large) share of the
     // pass's residual reaches every other vertex before that vertex is taken; 2 = last, so they
     // collect the pass's residual and push it once; 0 = in table order with the rest
-    const int order = effective_order(e);
-    auto table1 = [&](cudaStream_t s) { launch_push<SRC_TABLE>(e, a, e->grid_push, s); };
+    const int order = order_of(e) == 3 ? 3 : effective_order(e);
+    auto table1 = [&]() { launch_push<SRC_TABLE>(e, a, e->grid_push, st); };
     // order 3: each launch's long lists first, then its short ones
-    auto table = [&](cudaStream_t s) {
+    auto table = [&]() {
         if (order == 3) {
             a.lists = LISTS_LONG;
-            table1(s);
+            table1();
             a.lists = LISTS_SHORT;
-            table1(s);
+            table1();
             a.lists = LISTS_ALL;
         } else {
-            table1(s);
+            table1();
         }
     };
-    auto hub_phase = [&]() {
-        cudaMemsetAsync(a.q, 0, sizeof(PushQueue), st);
-        if (e->L == 1) {
-            k_push<1, SRC_HUBS><<<e->grid_push, BLOCK, hub_smem(e), st>>>(a);
-            k_segments<1><<<e->grid_push, BLOCK, hub_smem(e), st>>>(e->d_r, a);
-        } else {
-            k_push<4, SRC_HUBS><<<e->grid_push, BLOCK, hub_smem(e), st>>>(a);
-            k_segments<4><<<e->grid_push, BLOCK, hub_smem(e), st>>>(e->d_r, a);
-        }
-        e->launches += 2;
-    };
-    // one launch under an IF node (c = -1: the whole table)
-    auto guarded = [&](int c) -> cudaError_t {
-        a.chunk = c;
-        cudaError_t rc = open_if(st, chunk_body, &e->h_chunk_if[c >= 0 ? c : e->nc]);
-        if (rc != cudaSuccess) return rc;
-        table(chunk_body);
-        rc = close_if(chunk_body);
-        a.chunk = -1;
-        return rc;
-    };
-    if (order == 1) hub_phase();
+    if (order == 1) launch_push<SRC_HUBS>(e, a, e->grid_push, st);
     a.lists = order == 1 || order == 2 ? LISTS_SHORT : LISTS_ALL;   // the table push skips the high-degree vertices
-    if (use_if) {
-        // chunk by chunk: each chunk's push (with its long lists) completes before the next
-        // chunk's vertices are taken, so they see everything pushed so far; or the whole table
-        for (int c = 0; c < e->nc; c++) {
-            const cudaError_t rc = guarded(c);
-            if (rc != cudaSuccess) return rc;
-        }
-        const cudaError_t rc = guarded(-1);
-        if (rc != cudaSuccess) return rc;
-    } else if (sweep_of(e) && sweep_pass) {
+    if (sweep_of(e) && sweep_pass) {
         for (int c = 0; c < e->nc; c++) {
             a.chunk = c;
-            table(st);
+            table();
         }
         a.chunk = -1;
     } else {
-        table(st);
+        table();
     }
     a.lists = LISTS_ALL;
     if (ev) cudaEventRecord(ev[3], st);
-    if (order == 2) hub_phase();
+    if (order == 2) launch_push<SRC_HUBS>(e, a, e->grid_push, st);
     if (ev) cudaEventRecord(ev[4], st);
     return cudaGetLastError();
 }
 
-static cudaError_t enqueue_pass(excent_engine* e, double list_frac, int max_passes, cudaGraphConditionalHandle cond,
-                                int use_cond, cudaStream_t st, cudaStream_t chunk_body) {
-    enqueue_plan(e, list_frac, max_passes, cond, use_cond, st, nullptr, chunk_body && sweep_of(e));
-    return enqueue_push(e, st, nullptr, chunk_body, true);
+static SolveArgs solve_args(excent_engine* e, double list_frac, int max_passes) {
+    SolveArgs a{};
+    a.snap = snap_args(e, false);
+    a.push = push_args(e, 0);
+    a.cnt2 = e->d_cnt2;
+    // a word per warp step while there are warps for it, up to SNAP_GROUP
+    a.snap_group = std::max(1, std::min(SNAP_GROUP, a.snap.words / (e->sms * PW)));
+    a.cmode = e->d_cmode;
+    a.list_frac = list_frac;
+    a.max_passes = max_passes;
+    a.sweep = sweep_of(e) ? 1 : 0;
+    a.sweep_min = sweep_min_entries(e);
+    a.log = e->d_log;
+    a.log_cap = e->log_cap;
+    a.order = effective_order(e);
+    a.wave = e->wave;
+    a.seg = (unsigned)wave_seg(e->m);
+    a.small = e->d_small;
+    return a;
 }
 
+// One block per SM, fewer where there is not a word of 32 vertices for each.
+static int solve_grid(const excent_engine* e) { return std::max(1, std::min(e->sms, (e->n + 31) / 32)); }
+static cudaError_t launch_passes(excent_engine* e, SolveArgs& a, cudaStream_t st) {
+    return launch_grid(e->L == 1 ? k_passes<1> : k_passes<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
+}
+static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st) {
+    return launch_grid(e->L == 1 ? k_sweep<1> : k_sweep<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
+}
+
+// The solve of a sweeping engine: while { k_passes; if (a swept pass is due) k_sweep }.
 static int build_graph(excent_engine* e, double list_frac, int max_passes) {
     if (e->gexec && e->graph_max_passes == max_passes && e->graph_list_frac == list_frac) return EXCENT_OK;
     invalidate_graph(e);
-    if (sweep_of(e) && !e->d_chunk_if)
-        EX_ALLOC(e->d_chunk_if, (size_t)(e->nc + 1) * sizeof(cudaGraphConditionalHandle));
-    e->h_chunk_if.assign(e->nc + 1, 0);
+    SolveArgs a = solve_args(e, list_frac, max_passes);
+    a.use_cond = 1;
     cudaGraph_t g;
     EX_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle h;
-    EX_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
+    cudaStream_t cs = nullptr, cb = nullptr;
     cudaGraphNodeParams cp = {};
+    cudaGraphNode_t node;
+    cudaGraph_t captured;
+    cudaError_t rc = cudaGraphConditionalHandleCreate(&a.again, g, 1, cudaGraphCondAssignDefault);
     cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
+    cp.conditional.handle = a.again;
     cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    EX_CUDA(cudaGraphAddNode(&node, g, nullptr, 0, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    // capture one pass into the body graph
-    cudaStream_t cs, cb;
-    EX_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    EX_CUDA(cudaStreamCreateWithFlags(&cb, cudaStreamNonBlocking));
-    EX_CUDA(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const ull before = e->launches;
-    const cudaError_t pe = enqueue_pass(e, list_frac, max_passes, h, 1, cs, sweep_of(e) ? cb : nullptr);
-    e->launches = before;
-    cudaGraph_t captured;
-    const cudaError_t ce = cudaStreamEndCapture(cs, &captured);
-    cudaStreamDestroy(cs);
-    cudaStreamDestroy(cb);
-    if (pe != cudaSuccess || ce != cudaSuccess) {
+    if (rc == cudaSuccess) rc = cudaGraphAddNode(&node, g, nullptr, 0, &cp);
+    if (rc == cudaSuccess) rc = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
+    if (rc == cudaSuccess) rc = cudaStreamCreateWithFlags(&cb, cudaStreamNonBlocking);
+    if (rc == cudaSuccess) {
+        cudaGraph_t body = cp.conditional.phGraph_out[0];
+        rc = cudaGraphConditionalHandleCreate(&a.go_sweep, body, 0, cudaGraphCondAssignDefault);
+        if (rc == cudaSuccess) rc = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (rc == cudaSuccess) {
+            rc = launch_passes(e, a, cs);
+            if (rc == cudaSuccess) rc = open_if(cs, cb, a.go_sweep);
+            if (rc == cudaSuccess) {
+                rc = launch_sweep(e, a, cb);
+                const cudaError_t ci = close_if(cb);
+                if (rc == cudaSuccess) rc = ci;
+            }
+            const cudaError_t ce = cudaStreamEndCapture(cs, &captured);
+            if (rc == cudaSuccess) rc = ce;
+        }
+    }
+    if (cs) cudaStreamDestroy(cs);
+    if (cb) cudaStreamDestroy(cb);
+    if (rc == cudaSuccess) rc = cudaGraphInstantiate(&e->gexec, g, 0);
+    if (rc != cudaSuccess) {
+        e->gexec = nullptr;
         cudaGraphDestroy(g);
         cudaGetLastError();
-        EX_CUDA(pe != cudaSuccess ? pe : ce);
+        EX_CUDA(rc);
     }
-    if (sweep_of(e))
-        EX_CUDA(cudaMemcpy(e->d_chunk_if, e->h_chunk_if.data(), (size_t)(e->nc + 1) * sizeof(cudaGraphConditionalHandle),
-                           cudaMemcpyHostToDevice));
-    const cudaError_t ie = cudaGraphInstantiate(&e->gexec, g, 0);
-    if (ie != cudaSuccess) { cudaGraphDestroy(g); e->gexec = nullptr; EX_CUDA(ie); }
     e->graph = g;
     e->graph_max_passes = max_passes;
     e->graph_list_frac = list_frac;
@@ -1859,7 +1902,6 @@ extern "C" int excent_engine_seed(excent_engine* e, int k, const int32_t* vids, 
 // The vertices whose lists are longer than HUB_MIN (for a high-degree order),
 // listed once per graph; without room for the list the solve runs in table order.
 static int effective_order(const excent_engine* e) {
-    if (order_of(e) == 3) return 3;   // inside each launch: needs no high-degree list
     return order_of(e) && e->d_hubv && !e->hubv_stale ? order_of(e) : 0;
 }
 
@@ -1867,8 +1909,10 @@ static int ensure_hubv(excent_engine* e) {
     if (e->hubv_stale) {
         // count the high-degree vertices, then list them in a buffer of that size
         if (!e->d_hubv_cnt) EX_ALLOC(e->d_hubv_cnt, sizeof(ull));
-        EX_CUDA(cudaMemsetAsync(e->d_hubv_cnt, 0, sizeof(ull), e->s_main));
-        k_hub_list<<<e->sms * 8, BLOCK, 0, e->s_main>>>(e->n, e->d_idx, nullptr, e->d_hubv_cnt);
+        if (!e->d_hub_counts) EX_ALLOC(e->d_hub_counts, HUB_BLOCKS * sizeof(ull));
+        k_hub_list<<<HUB_BLOCKS, BLOCK, 0, e->s_main>>>(e->n, e->d_idx, e->d_hub_counts, nullptr);
+        k_hub_scan<<<1, HUB_BLOCKS, 0, e->s_main>>>(e->d_hub_counts, e->d_hubv_cnt);
+        e->launches += 2;
         ull h = 0;
         EX_CUDA(cudaMemcpyAsync(&h, e->d_hubv_cnt, sizeof(ull), cudaMemcpyDeviceToHost, e->s_main));
         EX_CUDA(cudaStreamSynchronize(e->s_main));
@@ -1885,9 +1929,8 @@ static int ensure_hubv(excent_engine* e) {
             }
         }
         if (e->d_hubv) {
-            EX_CUDA(cudaMemsetAsync(e->d_hubv_cnt, 0, sizeof(ull), e->s_main));
-            k_hub_list<<<e->sms * 8, BLOCK, 0, e->s_main>>>(e->n, e->d_idx, e->d_hubv, e->d_hubv_cnt);
-            e->launches += 2;
+            k_hub_list<<<HUB_BLOCKS, BLOCK, 0, e->s_main>>>(e->n, e->d_idx, e->d_hub_counts, e->d_hubv);
+            e->launches++;
             EX_CUDA(cudaGetLastError());
             e->hubv_stale = false;
         }
@@ -1908,24 +1951,28 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
     EX_CUDA(cudaMemcpy(e->d_cmode, cm.data(), e->nc, cudaMemcpyHostToDevice));
     if (init) EX_TRY(init_state(e));
     else EX_TRY(reset_counters(e));
-    if (order_of(e) == 1 || order_of(e) == 2) EX_TRY(ensure_hubv(e));
+    if (order_of(e)) EX_TRY(ensure_hubv(e));
     if (use_graph) {
-        EX_TRY(build_graph(e, list_frac, max_passes));
-        EX_CUDA(cudaGraphLaunch(e->gexec, e->s_main));
+        if (sweep_of(e)) {
+            EX_TRY(build_graph(e, list_frac, max_passes));
+            EX_CUDA(cudaGraphLaunch(e->gexec, e->s_main));
+        } else {   // every pass in one launch
+            SolveArgs a = solve_args(e, list_frac, max_passes);
+            EX_CUDA(launch_passes(e, a, e->s_main));
+        }
+        EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
         EX_CUDA(cudaStreamSynchronize(e->s_main));
-        EX_CUDA(cudaMemcpy(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost));
-        ull fixed = 0, per_chunk = 0;
-        pass_kernels(e, effective_order(e), &fixed, &per_chunk);
-        e->launches += fixed * (e->h_ctrl->pass + 1) + per_chunk * e->h_ctrl->chunk_runs;
+        e->launches += 1 + 2 * e->h_ctrl->sweeps;
+        if (e->h_ctrl->bar.failed) EX_FAIL(EXCENT_ERR_STATE, "a wait between the blocks of a solve timed out");
     } else {
         // snapshot and plan, read the plan back (one sync per pass), then the pushes it chose
         for (int p = 0; p <= max_passes; p++) {
             cudaEvent_t* ev = e->prof ? e->ev : nullptr;
-            enqueue_plan(e, list_frac, max_passes, 0, 0, e->s_main, ev, false);
+            enqueue_plan(e, list_frac, max_passes, e->s_main, ev);
             EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
             EX_CUDA(cudaStreamSynchronize(e->s_main));
             if (e->h_ctrl->done) break;
-            EX_CUDA(enqueue_push(e, e->s_main, ev, nullptr, e->h_ctrl->sweep_pass != 0));
+            EX_CUDA(enqueue_push(e, e->s_main, ev, e->h_ctrl->sweep_pass != 0));
             if (ev) {
                 EX_CUDA(cudaStreamSynchronize(e->s_main));
                 for (int k = 0; k < 4; k++) {
@@ -2047,18 +2094,27 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
         EX_CUDA(cudaGetLastError());
     }
     e->hub_k = 0;
+    const size_t asked = (size_t)k * (e->L == 1 ? sizeof(float) : sizeof(float4));
+    std::vector<int> ids;
     if (k > 0) {
         EX_CHECK_ARG(e->d_cache && e->cache_edges, "reserve the edge cache before choosing hub targets");
         std::vector<ull> idx((size_t)e->n + 1);
         EX_CUDA(cudaMemcpy(idx.data(), e->d_idx, idx.size() * sizeof(ull), cudaMemcpyDeviceToHost));
-        std::vector<int> ids(e->n);
+        ids.resize(e->n);
         for (int v = 0; v < e->n; v++) ids[v] = v;
         auto deg = [&](int v) { return idx[v + 1] - idx[v]; };
         std::nth_element(ids.begin(), ids.begin() + (k - 1), ids.end(), [&](int a, int b) {
             return deg(a) > deg(b) || (deg(a) == deg(b) && a < b);
         });
-        ids.resize(k);
+        // a slot pays where a block adds to it more than once before it flushes it: entries of
+        // targets of a lower degree stay plain (65k vertices, 16384 slots asked for: 2.00 ms a
+        // solve with all of them, 1.83 ms with those that pay)
+        const ull pays = 2ull * e->sms * (sweep_of(e) ? e->nc : 1);
+        ids.resize(std::partition(ids.begin(), ids.begin() + k, [&](int v) { return deg(v) >= pays; }) - ids.begin());
+        k = (int)ids.size();
         std::sort(ids.begin(), ids.end());
+    }
+    if (k > 0) {
         if (!e->d_hub_id) EX_ALLOC(e->d_hub_id, (size_t)kmax * sizeof(int));
         EX_CUDA(cudaMemcpy(e->d_hub_id, ids.data(), (size_t)k * sizeof(int), cudaMemcpyHostToDevice));
         e->hub_k = k;
@@ -2071,8 +2127,8 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
         EX_CUDA(cudaGetLastError());
     }
     const size_t smem = hub_smem(e);
-    if (smem > 0) {   // static + dynamic above 48 KiB needs the opt-in, per kernel (the staged kernels hold ~40 KiB)
-        const int sz = (int)smem;
+    if (asked > 0) {   // static + dynamic above 48 KiB needs the opt-in, per kernel (the staged kernels hold ~40 KiB)
+        const int sz = (int)asked;
         cudaFuncSetAttribute(k_push<1, SRC_TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_push<1, SRC_CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_push<1, SRC_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
@@ -2083,14 +2139,20 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
         cudaFuncSetAttribute(k_push<4, SRC_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_push<4, SRC_HOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_push<4, SRC_HUBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
+        cudaFuncSetAttribute(k_passes<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
+        cudaFuncSetAttribute(k_passes<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
+        cudaFuncSetAttribute(k_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
+        cudaFuncSetAttribute(k_sweep<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_segments<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_segments<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         EX_CUDA(cudaGetLastError());
     }
-    int occ = 0;
-    if (e->L == 1) EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push<1, SRC_TABLE>, BLOCK, smem));
-    else EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push<4, SRC_TABLE>, BLOCK, smem));
-    e->grid_push = e->sms * std::max(1, occ);
+    // a wave keeps the size that the slots asked for give it: what a solve of a few waves
+    // leaves below eps depends on it
+    int grid_asked = 0;
+    EX_TRY(push_blocks(e, asked, &grid_asked));
+    e->wave = std::min(grid_asked * BLOCK, WAVE_MAX);
+    EX_TRY(push_blocks(e, smem, &e->grid_push));
     return EXCENT_OK;
 }
 

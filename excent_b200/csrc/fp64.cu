@@ -329,7 +329,6 @@ extern "C" int excent_ppr_fp64(int device, int n, const unsigned long long* d_id
     EX_CUDA(cudaSetDevice(device));
     int sms = 0;
     EX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int G = sms * 8;
     const unsigned wb = (unsigned)(((long long)n * 32 + 255) / 256);
     Bufs B;
     double* t = nullptr;
