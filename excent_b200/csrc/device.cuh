@@ -49,6 +49,11 @@ __device__ __forceinline__ float4 shfl(float4 v, int src) {
     return make_float4(__shfl_sync(FULL, v.x, src), __shfl_sync(FULL, v.y, src), __shfl_sync(FULL, v.z, src),
                        __shfl_sync(FULL, v.w, src));
 }
+__device__ __forceinline__ float shfl_up(float v, int o) { return __shfl_up_sync(FULL, v, o); }
+__device__ __forceinline__ double shfl_up(double v, int o) { return __shfl_up_sync(FULL, v, o); }
+__device__ __forceinline__ double shfl(double v, int src) { return __shfl_sync(FULL, v, src); }
+__device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(FULL, v, o); }
+__device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(FULL, v, o); }
 template <typename T> __device__ __forceinline__ const T* shfl_ptr(const T* p, int src) {
     return (const T*)__shfl_sync(FULL, (unsigned long long)p, src);
 }

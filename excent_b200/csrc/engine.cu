@@ -857,6 +857,7 @@ __global__ void k_insert(int n, float4* s, int i, const float* in) {
 }  // namespace excent
 
 #include "passes.cuh"
+#include "sweep.cuh"
 
 using namespace excent;
 
@@ -924,6 +925,10 @@ struct excent_engine {
     ull* d_cnt2 = nullptr;         // persistent solve: the second demand table
     HubSeg* d_small = nullptr;     // and the short lists taken together
     int wave = 0;                  // items its passes take together
+    SweepLists sweep{};            // swept passes as gathers: the split lists
+    void* d_sweep = nullptr;       // (one allocation)
+    bool sweep_stale = true;       // not tried for the loaded lists
+    bool sweep_ok = false;
     bool hubv_stale = true;
     bool ev_proj = false;
     double ev_skip = 0;      // carry (do not write) a v1 correction of at most this size
@@ -990,6 +995,17 @@ static const char* ctrl_error(int err) {
                     : "device capacity check failed (hub queue overflow)";
 }
 static int ensure_hubv(excent_engine* e);
+// The lists changed: their split for swept passes holds no more (its memory is used again).
+static void lists_changed(excent_engine* e) {
+    e->sweep_stale = true;
+    if (!e->sweep_ok) return;
+    invalidate_graph(e);
+    e->sweep_ok = false;
+}
+static void offsets_changed(excent_engine* e) {
+    e->hubv_stale = true;
+    lists_changed(e);
+}
 
 // Pass order. By default a graph cut into several chunks is pushed chunk by
 // chunk, which is how the reference launches its resident chunks
@@ -1013,7 +1029,7 @@ static int free_engine(excent_engine* e) {
     cudaDeviceSynchronize();
     if (e->gexec) cudaGraphExecDestroy(e->gexec);
     if (e->graph) cudaGraphDestroy(e->graph);
-    void* dptrs[] = {e->d_hub_counts, e->d_cnt2, e->d_small, e->d_hub_id, e->d_hubv, e->d_hubv_cnt, e->d_v1, e->d_idx, e->d_x, e->d_r, e->d_bitmap, e->d_cnt, e->d_cv0, e->d_list, e->d_ctrl, e->d_cmode,
+    void* dptrs[] = {e->d_sweep, e->d_hub_counts, e->d_cnt2, e->d_small, e->d_hub_id, e->d_hubv, e->d_hubv_cnt, e->d_v1, e->d_idx, e->d_x, e->d_r, e->d_bitmap, e->d_cnt, e->d_cv0, e->d_list, e->d_ctrl, e->d_cmode,
                      e->d_wt_type, e->d_wt_prefix, e->d_hubq[0], e->d_hubq[1], e->d_hubq[2], e->d_queue, e->d_log, e->d_trace, e->d_tmp, e->d_cache,
                      e->d_hids, e->d_hoff, e->d_hedges, e->d_hot, e->d_hlist};
     for (void* p : dptrs) if (p) cudaFree(p);
@@ -1197,7 +1213,7 @@ extern "C" int excent_engine_upload_offsets(excent_engine* e, const unsigned lon
     EX_CUDA(cudaSetDevice(e->dev));
     EX_CUDA(cudaMemcpyAsync(e->d_idx + v0, idx, count * sizeof(ull), cudaMemcpyHostToDevice, e->s_main));
     EX_CUDA(cudaStreamSynchronize(e->s_main));
-    e->hubv_stale = true;
+    offsets_changed(e);
     return EXCENT_OK;
 }
 
@@ -1210,7 +1226,7 @@ extern "C" int excent_engine_upload_device(excent_engine* e, const unsigned long
     hub_encode(e, 0, e->m, e->s_main);
     EX_CUDA(cudaStreamSynchronize(e->s_main));
     EX_CUDA(cudaGetLastError());
-    e->hubv_stale = true;
+    offsets_changed(e);
     std::fill(e->loaded.begin(), e->loaded.end(), 1);
     return EXCENT_OK;
 }
@@ -1220,6 +1236,8 @@ extern "C" int excent_engine_reserve_cache(excent_engine* e, unsigned long long 
     EX_CUDA(cudaSetDevice(e->dev));
     invalidate_graph(e);
     EX_CUDA(cudaDeviceSynchronize());
+    lists_changed(e);
+    if (e->d_sweep) { cudaFree(e->d_sweep); e->d_sweep = nullptr; }
     if (e->d_cache) { cudaFree(e->d_cache); e->d_cache = nullptr; e->cache_edges = 0; }
     e->hub_k = 0;   // a fresh cache holds plain ids
     free_host_cache(e);
@@ -1243,6 +1261,7 @@ extern "C" int excent_engine_load_cache(excent_engine* e, unsigned long long e0,
     hub_encode(e, e0, e1, e->s_main);
     EX_CUDA(cudaStreamSynchronize(e->s_main));
     EX_CUDA(cudaGetLastError());
+    lists_changed(e);
     for (int c = 0; c < e->nc; c++) if (e->ce[c] >= e0 && e->ce[c + 1] <= e1) e->loaded[c] = 1;
     return EXCENT_OK;
 }
@@ -1579,7 +1598,7 @@ extern "C" int excent_engine_push_stream(excent_engine* e, int s, int c, const u
     else { a.ctype = WT_RANGE; a.ccount = (unsigned)nv; e->n_range++; }
     if (a.ccount) launch_ordered<SRC_CHUNK>(e, a, grid_for(e, a.ccount), sl.st);
     EX_CUDA(cudaGetLastError());
-    if (to_cache) e->loaded[c] = 1;
+    if (to_cache) { lists_changed(e); e->loaded[c] = 1; }
     EX_CUDA(cudaEventRecord(sl.done, sl.st));
     sl.busy = true;
     return EXCENT_OK;
@@ -1799,7 +1818,116 @@ static cudaError_t launch_passes(excent_engine* e, SolveArgs& a, cudaStream_t st
     return launch_grid(e->L == 1 ? k_passes<1> : k_passes<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
 }
 static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st) {
+    if (e->sweep_ok && a.order == 3) {
+        SweepArgs s{a, e->sweep};
+        return launch_grid(e->L == 1 ? k_sweep_gather<1> : k_sweep_gather<4>, e->sms * G_PER_SM, GT, 0, s, &e->d_ctrl->bar, st);
+    }
     return launch_grid(e->L == 1 ? k_sweep<1> : k_sweep<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
+}
+
+// Split the lists for swept passes as gathers, once per loaded graph. It takes
+// a symmetric graph, wholly in the edge cache, of fewer than 2^31 entries, the
+// launch-first order, and an eighth of the free device memory at most (a copy
+// of the lists, a weight per vertex and the segment tables); otherwise swept
+// passes scatter.
+static int ensure_sweep(excent_engine* e) {
+    if (!e->sweep_stale) return EXCENT_OK;
+    if (!sweep_of(e) || effective_order(e) != 3 || e->d_hcache || e->cache_edges != e->m) return EXCENT_OK;   // may change
+    e->sweep_stale = false;
+    const size_t n = (size_t)e->n, tb = e->L == 1 ? sizeof(float) : sizeof(float4);
+    const ull m = e->m;
+    // short lists of a chunk are taken in phases of this many vertices: the scatter takes a wave at a
+    // time and delivers it before the next. With one phase a chunk, PageRank inside `all` on 16.8M
+    // vertices moved by 3.7e-4 of its norm (two runs of the scatter differ by 1.1e-4), with phases of
+    // 700k vertices, six waves, by 1.8e-4, for 8 % of the time; smaller ones change nothing more.
+    const int per_phase = 6 * e->wave;
+    std::vector<int> q_of(1, 0);
+    for (int c = 0; c < e->nc; c++) {
+        const int nv = (c + 1 < e->nc ? e->cv0[c + 1] : e->n) - e->cv0[c];
+        q_of.push_back(q_of.back() + (nv + per_phase - 1) / per_phase);
+    }
+    const size_t nq = q_of.back();
+    if (m == 0 || m >= (1ull << 31) || nq + e->nc >= 65535) return EXCENT_OK;
+    // segments at most: a list of more than PULL_LONG entries has one for each PULL_SEG entries and one more
+    const size_t hub_cap = m / PULL_SEG + m / HUB_MIN + 1, mid_cap = m / PULL_LONG + 1, late_cap = list_seg_cap(m);
+    const size_t words = (n + 31) / 32;
+    std::vector<size_t> parts = {m * sizeof(int), n * 4, (n + 1) * 4, n * 2, n * 4, (n + 1) * 4, words * 4, n * tb,
+                                 hub_cap * sizeof(HubPart), mid_cap * sizeof(ListSeg), late_cap * sizeof(ListSeg), hub_cap * 4,
+                                 (size_t)(e->nc + 1) * 4, (nq + 1) * 4, (nq + 1) * 4, (size_t)(e->nc + 1) * 4, C_KINDS * 4};
+    // what only the building needs: phase and early length of every vertex, where its parts go, the sums
+    const size_t first_temp = parts.size();
+    for (size_t bytes : {n * sizeof(uint16_t), n * 4, n * 4, n * 4, (size_t)C_KINDS * HUB_BLOCKS * 4, sizeof(ull)})
+        parts.push_back(bytes);
+    size_t total = 0;   // sizes to offsets, 256-byte aligned
+    for (size_t& p : parts) { const size_t bytes = (p + 255) / 256 * 256; p = total; total += bytes; }
+    if (!e->d_sweep) {
+        size_t fr = 0, all = 0;
+        EX_CUDA(cudaMemGetInfo(&fr, &all));
+        if (total > fr / 8) return EXCENT_OK;
+        if (cudaMalloc(&e->d_sweep, total) != cudaSuccess) {
+            cudaGetLastError();
+            e->d_sweep = nullptr;
+            return EXCENT_OK;
+        }
+    }
+    char* k = (char*)e->d_sweep;
+    SweepBuild b{};
+    b.n = e->n; b.nc = e->nc; b.idx = e->d_idx; b.adj = e->d_cache; b.hub_id = e->d_hub_id;
+    b.hubv = e->d_hubv; b.hubv_cnt = e->d_hubv_cnt;
+    b.cv0 = e->d_cv0; b.per_phase = per_phase;
+    b.out = (int*)(k + parts[0]);
+    b.e_v = (int*)(k + parts[1]);
+    b.e_off = (unsigned*)(k + parts[2]);
+    b.e_deg = (uint16_t*)(k + parts[3]);
+    b.l_v = (int*)(k + parts[4]);
+    b.l_off = (unsigned*)(k + parts[5]);
+    b.alone = (uint32_t*)(k + parts[6]);
+    void* weights = k + parts[7];
+    b.e_hub = (HubPart*)(k + parts[8]);
+    b.e_mid = (ListSeg*)(k + parts[9]);
+    b.l_seg = (ListSeg*)(k + parts[10]);
+    b.hub_done = (unsigned*)(k + parts[11]);
+    b.hub_at = (unsigned*)(k + parts[12]);
+    b.mid_at = (unsigned*)(k + parts[13]);
+    b.ev_at = (unsigned*)(k + parts[14]);
+    int* d_q_of = (int*)(k + parts[15]);
+    b.totals = (unsigned*)(k + parts[16]);
+    b.q_of = d_q_of;
+    uint16_t* phase = (uint16_t*)(k + parts[first_temp]);
+    b.phase = phase;
+    b.early = (unsigned*)(k + parts[first_temp + 1]);
+    b.e_dst = (unsigned*)(k + parts[first_temp + 2]);
+    b.l_dst = (unsigned*)(k + parts[first_temp + 3]);
+    b.counts = (unsigned*)(k + parts[first_temp + 4]);
+    b.asym = (ull*)(k + parts[first_temp + 5]);
+    ull asym = 1;
+    cudaStream_t st = e->s_main;
+    const int grid = e->sms * 6;
+    cudaMemsetAsync(b.alone, 0, words * 4, st);
+    cudaMemsetAsync(b.asym, 0, sizeof(ull), st);
+    cudaMemcpyAsync(d_q_of, q_of.data(), q_of.size() * 4, cudaMemcpyHostToDevice, st);
+    k_sweep_phase<<<e->sms * 8, BLOCK, 0, st>>>(e->n, e->d_idx, e->d_cv0, e->nc, d_q_of, per_phase, phase);
+    k_sweep_split<0><<<grid, BLOCK, 0, st>>>(b);
+    cudaMemcpyAsync(&asym, b.asym, sizeof asym, cudaMemcpyDeviceToHost, st);
+    cudaError_t rc = cudaStreamSynchronize(st);
+    e->launches += 2;
+    if (rc == cudaSuccess && !asym) {
+        k_sweep_layout<<<HUB_BLOCKS, BLOCK, 0, st>>>(b, 0);
+        k_sweep_scan<<<C_KINDS, HUB_BLOCKS, 0, st>>>(b.counts, b.totals);
+        k_sweep_layout<<<HUB_BLOCKS, BLOCK, 0, st>>>(b, 1);
+        k_sweep_split<1><<<grid, BLOCK, 0, st>>>(b);
+        rc = cudaGetLastError();
+        e->launches += 4;
+        if (rc == cudaSuccess) {
+            invalidate_graph(e);
+            e->sweep = SweepLists{b.out, b.e_v, b.e_off, b.e_deg, b.l_v, b.l_off, b.alone, b.e_hub, b.e_mid, b.l_seg,
+                                  b.totals, b.hub_at, b.mid_at, b.ev_at, d_q_of, b.hub_done, weights};
+            e->sweep_ok = true;
+        }
+    }
+    if (!e->sweep_ok) { cudaFree(e->d_sweep); e->d_sweep = nullptr; }
+    EX_CUDA(rc);
+    return EXCENT_OK;
 }
 
 // The solve of a sweeping engine: while { k_passes; if (a swept pass is due) k_sweep }.
@@ -1954,6 +2082,7 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
     if (order_of(e)) EX_TRY(ensure_hubv(e));
     if (use_graph) {
         if (sweep_of(e)) {
+            EX_TRY(ensure_sweep(e));
             EX_TRY(build_graph(e, list_frac, max_passes));
             EX_CUDA(cudaGraphLaunch(e->gexec, e->s_main));
         } else {   // every pass in one launch
@@ -2106,10 +2235,12 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
         std::nth_element(ids.begin(), ids.begin() + (k - 1), ids.end(), [&](int a, int b) {
             return deg(a) > deg(b) || (deg(a) == deg(b) && a < b);
         });
-        // a slot pays where a block adds to it more than once before it flushes it: entries of
-        // targets of a lower degree stay plain (65k vertices, 16384 slots asked for: 2.00 ms a
-        // solve with all of them, 1.83 ms with those that pay)
-        const ull pays = 2ull * e->sms * (sweep_of(e) ? e->nc : 1);
+        // targets of a lower degree stay plain: a block seldom adds to their slots twice before it
+        // flushes them (65k vertices, 16384 slots asked for: 2.00 ms a solve with all of them, 1.83
+        // without). Down to 64 entries they keep large residuals from being summed entry by entry,
+        // and with them Katz's error at eps 1e-6 (150k vertices: 6.2e-7, 8.5e-7 with slots from 296
+        // entries on, 6.0e-7 with all)
+        constexpr ull pays = 64;
         ids.resize(std::partition(ids.begin(), ids.begin() + k, [&](int v) { return deg(v) >= pays; }) - ids.begin());
         k = (int)ids.size();
         std::sort(ids.begin(), ids.end());

@@ -39,7 +39,7 @@ template <typename T> struct PullScratch {
 // each 32-entry window, summed per list by a segmented scan, so short lists (5
 // entries on average on the R-MAT graphs) keep every lane busy.
 template <typename T, typename F>
-__device__ __forceinline__ T warp_list_sums(ull b, unsigned ds, const F& f, PullScratch<T>& s, int lane) {
+__device__ __forceinline__ T warp_window_sums(ull b, unsigned ds, const F& f, PullScratch<T>& s, int lane) {
     const unsigned nz = __ballot_sync(FULL, ds != 0);
     if (!nz) return T(0);
     const unsigned incl = warp_incl_scan(ds, lane);
@@ -72,7 +72,7 @@ __device__ __forceinline__ T warp_list_sums(ull b, unsigned ds, const F& f, Pull
             const int first = 31 - __clz((starts[q] & le) | 1u);   // where this lane's list starts in the window
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const T up = __shfl_up_sync(FULL, val[q], o);
+                const T up = shfl_up(val[q], o);
                 if (lane - o >= first) val[q] += up;
             }
             const bool last = lane == 31 || j + 1 >= tot || ((starts[q] >> (lane + 1)) & 1u);
@@ -83,6 +83,58 @@ __device__ __forceinline__ T warp_list_sums(ull b, unsigned ds, const F& f, Pull
     const T sum = ds ? s.acc[rank] : T(0);
     __syncwarp();
     return sum;
+}
+
+// Each lane's sum of f over its list [b, b + ds), ds <= PULL_LONG. f.key(e)
+// loads what entry e names, f.value(key) gathers its value (0 for a default
+// key). Eight lanes walk a list, four lists at a time and four such rounds in
+// flight: on lists of 5 to 7 entries that keeps half of the lanes busy for
+// less than half the instructions of a segmented scan over the concatenated
+// lists (15 shuffles and as many additions per 32 float4 entries).
+template <typename T, int R = 4, typename O, typename F>
+__device__ __forceinline__ T warp_list_sums(O b, unsigned ds, const F& f, int lane) {
+    T mine = T(0);
+    if (!__any_sync(FULL, ds)) return mine;
+    const int sub = lane >> 3, l8 = lane & 7;
+#pragma unroll 1
+    for (int t = 0; t < 8; t += R) {   // R rounds of four lists in flight
+        O bb[R];
+        unsigned dd[R], most = 0;
+        T acc[R];
+        typename F::Key key[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            const int src = (t + k) * 4 + sub;
+            bb[k] = __shfl_sync(FULL, b, src);
+            dd[k] = __shfl_sync(FULL, ds, src);
+            most = max(most, dd[k]);
+            acc[k] = T(0);
+            key[k] = typename F::Key{};
+            if ((unsigned)l8 < dd[k]) key[k] = f.key(bb[k] + l8);
+        }
+        most = __reduce_max_sync(FULL, most);
+        for (unsigned j = 8; j < most + 8; j += 8) {   // the next entries' keys are loaded ahead
+            typename F::Key next[R];
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                next[k] = typename F::Key{};
+                if (j + l8 < dd[k]) next[k] = f.key(bb[k] + j + l8);
+            }
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                acc[k] += f.value(key[k]);
+                key[k] = next[k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) acc[k] += shfl_xor(acc[k], o);
+            const T v = shfl(acc[k], (lane & 3) * 8);   // list 4 * (t + k) + s is summed by lanes 8 s .. 8 s + 7
+            if ((lane >> 2) == t + k) mine = v;
+        }
+    }
+    return mine;
 }
 
 // The warp's sums of f over two segments (valid in lane 0).
@@ -151,7 +203,7 @@ __device__ __forceinline__ void gather_phase(int n, const ull* idx, const ListSe
             ds = dv > PULL_LONG ? 0u : (unsigned)dv;
         }
         if (!__any_sync(FULL, ds)) continue;
-        const T t = warp_list_sums<T>(b, ds, f, S, lane);
+        const T t = warp_window_sums<T>(b, ds, f, S, lane);
         if (ds) add((unsigned)v, t, false);
     }
 }
