@@ -13,10 +13,9 @@
 // "touched" bitmap of the previous pass (clearing it), checks each touched
 // row against eps, takes and pushes the pending lanes and marks every
 // receiving neighbour in the other touched bitmap (check before atomic OR).
-// The solve ends after a pass that pushed nothing. One persistent kernel does
-// the scan, take and push; lists longer than 512 entries are split into
-// segments handled by a second kernel; a one-thread kernel advances the pass
-// and sets the loop condition of the CUDA graph that runs all passes.
+// The solve ends after a pass that pushed nothing. One cooperative launch runs
+// all passes: scan, take and push, and, after a grid barrier, the segments of
+// the lists longer than 512 entries.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,10 +25,11 @@
 
 #include "common.h"
 #include "device.cuh"
+#include "gridsync.cuh"
 
 namespace excent {
 
-static constexpr int BB = 256;              // threads per block
+static constexpr int BB = 1024;             // threads per block, one block per SM
 static constexpr unsigned BHUB_MIN = 512;   // lists longer than this go to segments
 static constexpr unsigned BHUB_SEG = 512;
 
@@ -48,7 +48,8 @@ struct BCtrl {
     ull rows_checked;                    // touched rows examined, over the solve
     ull total_segs;                      // hub segments queued, over the solve
     int err;
-    int done;
+    int pad;
+    GridBar bar;
 };
 
 struct BArgs {
@@ -133,6 +134,8 @@ __device__ __forceinline__ ull scatter_rowpar(float4* R, int V, uint32_t* nxt, c
     return upd;
 }
 
+// Rows of short lists with more active 16-byte groups than this scatter over their groups.
+static constexpr int DENSE_ROW = 4;
 // Default: segments of rows with more active 16-byte groups than this scatter over their groups.
 static constexpr int DENSE_GROUPS = 4;
 
@@ -158,22 +161,41 @@ __device__ __forceinline__ int compact_groups(const float4 (&p)[NV], const bool 
     return base;
 }
 
-// One pass: scan touched words (interleaved over warps), check, take and push.
+// The whole solve in one cooperative launch, one block per SM. A pass is two
+// phases with a grid barrier after each: the touched rows are checked, taken
+// and pushed, lists longer than BHUB_MIN being queued as segments; then the
+// segments are scattered.
+//
+// What bounds it: in the dense passes the warps whose word holds 32 vertices
+// with long lists, one row after the other; in the others the latency of the
+// two phases. Neighbouring words go to different SMs, the next row's offsets
+// are loaded while a row is pushed, the values are added by reductions, which
+// nothing waits for, and rows with many active groups scatter over their
+// groups. 64 queries on 131k vertices to 1e-6: 9.8 ms as three kernels a pass
+// in a graph, 7.4 ms; 256 on 50k: 36 and 19 ms. Sharing a word's rows between
+// a block's warps as well gave 5.7 and 12 ms, but it moves the takes of those
+// vertices ahead of the others', and what a solve leaves below eps with them
+// (3e-4 of its norm, against 7e-5 between two runs).
 template <int LPR, int NV>
-__global__ void __launch_bounds__(BB, 4) k_bpass(BArgs a) {
+__global__ void __launch_bounds__(BB, 1) k_bsolve(BArgs a) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int j0 = lane % LPR;
-    const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const long long gw = (long long)wib * gridDim.x + blockIdx.x;   // neighbouring words (and their long lists) on different SMs
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     __shared__ float4 s_gp[BB / 32][LPR * NV];
     __shared__ int s_gi[BB / 32][LPR * NV];
-    const int par = a.ctrl->pass & 1;
-    uint32_t* cur = par ? a.touched[1] : a.touched[0];   // no run-time index into the parameters
-    uint32_t* nxt = par ? a.touched[0] : a.touched[1];
-    ull pushed_v = 0, pushed_e = 0, upd = 0, checked = 0;
+    __shared__ ull s_v[BB / 32];
+    const int max_passes = a.ctrl->max_passes;
+    unsigned epoch = 0;
+    ull pushed_e = 0, upd = 0, checked = 0;
     float4 eps[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) eps[k] = a.eps[j0 + LPR * k];
+    for (int pass = 0;; pass++) {
+    const int par = pass & 1;
+    uint32_t* cur = par ? a.touched[1] : a.touched[0];   // no run-time index into the parameters
+    uint32_t* nxt = par ? a.touched[0] : a.touched[1];
+    ull pushed_v = 0;
     for (long long jw = 0; gw + jw * nwarps < a.words; jw += 32) {
         // warp gw owns words gw + j * nwarps (interleaved, so dense regions spread over all
         // warps); it reads 32 of them per step, one per lane, then walks the nonzero ones
@@ -181,37 +203,49 @@ __global__ void __launch_bounds__(BB, 4) k_bpass(BArgs a) {
         const uint32_t mine = wl < a.words ? cur[wl] : 0u;
         if (mine) { cur[wl] = 0; checked += __popc(mine); }
         unsigned nzw = __ballot_sync(FULL, mine != 0);
-        while (nzw) {
-        const int src = __ffs(nzw) - 1;
-        nzw &= nzw - 1;
-        const long long w = gw + (jw + src) * nwarps;
-        uint32_t bits = __shfl_sync(FULL, mine, src);
-        while (bits) {
+        // the touched rows of these words in order: next_row() gives the next one, or -1
+        uint32_t bits = 0;
+        long long wbase = 0;
+        auto next_row = [&]() -> int {
+            if (!bits) {
+                if (!nzw) return -1;
+                const int src = __ffs(nzw) - 1;
+                nzw &= nzw - 1;
+                wbase = (gw + (jw + src) * nwarps) * 32;
+                bits = __shfl_sync(FULL, mine, src);
+            }
             const int b = __ffs(bits) - 1;
             bits &= bits - 1;
-            const int v = (int)(w * 32 + b);
+            return (int)(wbase + b);
+        };
+        float4 rv[NV];
+        ull b0 = 0, b1 = 0;
+        auto load_offsets = [&](int v) {
+            if (v >= 0) { b0 = a.idx[v]; b1 = a.idx[v + 1]; }
+        };
+        int v = next_row();
+        load_offsets(v);
+        while (v >= 0) {
             float4* rrow = a.R + (size_t)v * a.V;
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                rv[k] = v >= 0 && lane < LPR ? a.R[(size_t)v * a.V + j0 + LPR * k] : make_float4(0.f, 0.f, 0.f, 0.f);
             float4 d[NV];
-            bool any = false;
             // a row with any pending lane is pushed whole (greedy): every lane with a nonzero
             // residual is taken, since the one read of the list serves them all
-            float4 rv[NV];
-            bool pend = false;
+            bool pend = false, any = false;
 #pragma unroll
-            for (int k = 0; k < NV; k++) {
-                rv[k] = lane < LPR ? rrow[j0 + LPR * k] : make_float4(0.f, 0.f, 0.f, 0.f);
-                pend |= fabsf(rv[k].x) > eps[k].x || fabsf(rv[k].y) > eps[k].y || fabsf(rv[k].z) > eps[k].z ||
-                        fabsf(rv[k].w) > eps[k].w;
-            }
+            for (int k = 0; k < NV; k++)
+                pend |= lane < LPR && (fabsf(rv[k].x) > eps[k].x || fabsf(rv[k].y) > eps[k].y ||
+                                       fabsf(rv[k].z) > eps[k].z || fabsf(rv[k].w) > eps[k].w);
             const bool row_pend = __any_sync(FULL, pend);
-            const float4 floor0 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int k = 0; k < NV; k++) {
                 d[k] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < LPR && row_pend) {
                     if (a.greedy) {
                         // the whole 16-byte group in one exchange when any of its lanes is nonzero
-                        if (nonzero(rv[k])) d[k] = atomicExch(rrow + j0 + LPR * k, floor0);
+                        if (nonzero(rv[k])) d[k] = atomicExch(rrow + j0 + LPR * k, make_float4(0.f, 0.f, 0.f, 0.f));
                     } else {
                         const float4 th = eps[k];
                         float* rp = reinterpret_cast<float*>(rrow + j0 + LPR * k);
@@ -220,18 +254,20 @@ __global__ void __launch_bounds__(BB, 4) k_bpass(BArgs a) {
                         d[k].z = take_lane(rp + 2, rv[k].z, th.z);
                         d[k].w = take_lane(rp + 3, rv[k].w, th.w);
                     }
-                    if (nonzero(d[k])) {
-                        float4* xp = a.X + (size_t)v * a.V + j0 + LPR * k;
-                        float4 xv = *xp;
-                        xv.x += d[k].x; xv.y += d[k].y; xv.z += d[k].z; xv.w += d[k].w;
-                        *xp = xv;
-                        any = true;
-                    }
                 }
             }
+            const ull l0 = b0;
+            const unsigned deg = (unsigned)(b1 - b0);
+            const int vn = next_row();
+            load_offsets(vn);   // in flight while this row is pushed
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                if (nonzero(d[k])) {   // one writer per value: a reduction, for its load is not waited for
+                    red_add(a.X + (size_t)v * a.V, j0 + LPR * k, d[k]);
+                    any = true;
+                }
+            v = vn;
             if (!__any_sync(FULL, any)) continue;
-            const ull b0 = a.idx[v];
-            const unsigned deg = (unsigned)(a.idx[v + 1] - b0);
             if (lane == 0) { pushed_v++; pushed_e += deg; }
             if (deg == 0) continue;
             float4 p[NV];
@@ -249,7 +285,7 @@ __global__ void __launch_bounds__(BB, 4) k_bpass(BArgs a) {
                 p[k] = q;
                 act[k] = nonzero(q);
             }
-            const int* nb = a.adj + b0;
+            const int* nb = a.adj + l0;
             if (deg > BHUB_MIN) {
                 // queue: weight row into the hub buffer, segments of BHUB_SEG entries
                 ull slot = 0, sbase = 0;
@@ -276,43 +312,32 @@ __global__ void __launch_bounds__(BB, 4) k_bpass(BArgs a) {
                 }
                 continue;
             }
-            // (lists up to BHUB_MIN: lanes over entries measured faster here at any density)
             const int nact = compact_groups<LPR, NV>(p, act, s_gp[wib], s_gi[wib], lane);
-            upd += scatter_lanes(a.R, a.V, nxt, nb, deg, s_gp[wib], s_gi[wib], nact, lane);
+            if (nact > DENSE_ROW) upd += scatter_rowpar<LPR, NV>(a.R, a.V, nxt, nb, deg, p, act, lane);
+            else upd += scatter_lanes(a.R, a.V, nxt, nb, deg, s_gp[wib], s_gi[wib], nact, lane);
             __syncwarp();
         }
-        }
     }
-    __shared__ ull s_v[BB / 32], s_e[BB / 32], s_u[BB / 32], s_c[BB / 32];
     pushed_v = warp_sum(pushed_v);
-    pushed_e = warp_sum(pushed_e);
-    upd = warp_sum(upd);
-    checked = warp_sum(checked);
-    if (lane == 0) { s_v[wib] = pushed_v; s_e[wib] = pushed_e; s_u[wib] = upd; s_c[wib] = checked; }
+    if (lane == 0) s_v[wib] = pushed_v;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        ull tv = 0, te = 0, tu = 0, tc = 0;
-        for (int i = 0; i < BB / 32; i++) { tv += s_v[i]; te += s_e[i]; tu += s_u[i]; tc += s_c[i]; }
-        if (tv) atomicAdd(&a.ctrl->pushed_v[par], tv);
-        if (te) atomicAdd(&a.ctrl->total_e, te);
-        if (tu) atomicAdd(&a.ctrl->total_lane_e, tu);
-        if (tc) atomicAdd(&a.ctrl->rows_checked, tc);
+    if (wib == 0) {
+        const ull t = warp_sum(s_v[lane]);
+        if (lane == 0 && t) atomicAdd(&a.ctrl->pushed_v[par], t);
     }
-}
-
-template <int LPR, int NV>
-__global__ void __launch_bounds__(BB) k_bhub(BArgs a) {
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int j0 = lane % LPR;
-    const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const int par = a.ctrl->pass & 1;
-    uint32_t* nxt = par ? a.touched[0] : a.touched[1];
+    if (!grid_sync(&a.ctrl->bar, epoch)) return;
+    const ull pv = a.ctrl->pushed_v[par];
     ull nseg = a.ctrl->hub_segs[par];
+    const bool failed = nseg > a.seg_cap || a.ctrl->hub_rows[par] > a.prow_cap;   // err is set
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next pass's counters: nobody uses them before the barrier
+        a.ctrl->total_v += pv;
+        a.ctrl->total_segs += nseg;
+        a.ctrl->pushed_v[par ^ 1] = 0;
+        a.ctrl->hub_rows[par ^ 1] = 0;
+        a.ctrl->hub_segs[par ^ 1] = 0;
+        if (pv > 0) a.ctrl->pass = pass + 1;
+    }
     if (nseg > a.seg_cap) nseg = a.seg_cap;
-    __shared__ float4 s_gp[BB / 32][LPR * NV];
-    __shared__ int s_gi[BB / 32][LPR * NV];
-    ull upd = 0;
     for (long long s = gw; s < (long long)nseg; s += nwarps) {
         const BSeg sg = a.seg[s];
         float4 p[NV];
@@ -327,14 +352,16 @@ __global__ void __launch_bounds__(BB) k_bhub(BArgs a) {
         else upd += scatter_lanes(a.R, a.V, nxt, sg.nb, sg.len, s_gp[wib], s_gi[wib], nact, lane);
         __syncwarp();
     }
-    __shared__ ull s_u[BB / 32];
+    if (pv == 0 || failed || pass + 1 >= max_passes) break;
+    if (!grid_sync(&a.ctrl->bar, epoch)) return;
+    }
+    pushed_e = warp_sum(pushed_e);
     upd = warp_sum(upd);
-    if (lane == 0) s_u[wib] = upd;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ull tu = 0;
-        for (int i = 0; i < BB / 32; i++) tu += s_u[i];
-        if (tu) atomicAdd(&a.ctrl->total_lane_e, tu);
+    checked = warp_sum(checked);
+    if (lane == 0) {
+        if (pushed_e) atomicAdd(&a.ctrl->total_e, pushed_e);
+        if (upd) atomicAdd(&a.ctrl->total_lane_e, upd);
+        if (checked) atomicAdd(&a.ctrl->rows_checked, checked);
     }
 }
 
@@ -345,21 +372,6 @@ __global__ void k_bcount(int n, const ull* idx, unsigned thr, ull* out) {
         c += idx[v + 1] - idx[v] > thr;
     c = warp_sum(c);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
-}
-
-// End of a pass: totals, next pass's counters, loop condition.
-__global__ void k_bend(BCtrl* c, cudaGraphConditionalHandle cond, int use_cond) {
-    const int par = c->pass & 1;
-    const ull pv = c->pushed_v[par];
-    c->total_v += pv;
-    c->total_segs += c->hub_segs[par];
-    c->pushed_v[par ^ 1] = 0;
-    c->hub_rows[par ^ 1] = 0;
-    c->hub_segs[par ^ 1] = 0;
-    const bool more = pv > 0 && c->pass + 1 < c->max_passes && !c->err;
-    if (pv > 0) c->pass++;
-    if (!more) c->done = 1;
-    if (use_cond) cudaGraphSetConditional(cond, more ? 1u : 0u);
 }
 
 __global__ void k_bseed(int nq, const int* lane_off, const int* vids, const float* vals, float* R, int B,
@@ -403,10 +415,6 @@ struct excent_batch {
     size_t seed_cap = 0;
     float* d_col = nullptr;
     cudaStream_t st = nullptr;
-    cudaGraphExec_t gexec = nullptr;
-    cudaGraph_t graph = nullptr;
-    int graph_max = -1;
-    int grid = 0;
     ull launches = 0;
     int greedy = 1;
     int dense = DENSE_GROUPS;   // see excent_batch_set_dense
@@ -415,8 +423,6 @@ struct excent_batch {
 static void batch_free(excent_batch* b) {
     cudaSetDevice(b->dev);
     cudaDeviceSynchronize();
-    if (b->gexec) cudaGraphExecDestroy(b->gexec);
-    if (b->graph) cudaGraphDestroy(b->graph);
     void* ps[] = {b->d_R, b->d_X, b->d_eps, b->d_t[0], b->d_t[1], b->d_P, b->d_seg, b->d_ctrl,
                   b->d_seed_off, b->d_seed_v, b->d_seed_x, b->d_col};
     for (void* p : ps) if (p) cudaFree(p);
@@ -442,22 +448,13 @@ static BArgs bargs(excent_batch* b) {
     return a;
 }
 
-template <int LPR, int NV>
-static void launch_pass_t(excent_batch* b, cudaStream_t st, cudaGraphConditionalHandle cond, int use_cond) {
+static cudaError_t launch_solve(excent_batch* b) {
     BArgs a = bargs(b);
-    k_bpass<LPR, NV><<<b->grid, BB, 0, st>>>(a);
-    k_bhub<LPR, NV><<<b->grid, BB, 0, st>>>(a);
-    k_bend<<<1, 1, 0, st>>>(b->d_ctrl, cond, use_cond);
-}
-
-static void launch_pass(excent_batch* b, cudaStream_t st, cudaGraphConditionalHandle cond, int use_cond) {
-    switch (b->B) {
-        case 32: launch_pass_t<8, 1>(b, st, cond, use_cond); break;
-        case 64: launch_pass_t<16, 1>(b, st, cond, use_cond); break;
-        case 128: launch_pass_t<32, 1>(b, st, cond, use_cond); break;
-        default: launch_pass_t<32, 2>(b, st, cond, use_cond); break;
-    }
-    b->launches += 3;
+    // one block per SM, fewer where there is not a bitmap word for each
+    const int grid = std::max(1, std::min(b->sms, a.words));
+    auto kernel = b->B == 32 ? k_bsolve<8, 1> : b->B == 64 ? k_bsolve<16, 1> : b->B == 128 ? k_bsolve<32, 1> : k_bsolve<32, 2>;
+    b->launches++;
+    return launch_grid(kernel, grid, BB, 0, a, &b->d_ctrl->bar, b->st);
 }
 
 static int batch_setup(excent_batch* b, int device, int n, ull m, const ull* d_idx, const int* d_adj, int B, int kind,
@@ -480,7 +477,7 @@ static int batch_setup(excent_batch* b, int device, int n, ull m, const ull* d_i
         ull* d_cnt = nullptr;
         BX_ALLOC(d_cnt, sizeof(ull));
         cudaMemset(d_cnt, 0, sizeof(ull));
-        k_bcount<<<b->sms * 8, BB, 0, b->st>>>(n, d_idx, BHUB_MIN, d_cnt);
+        k_bcount<<<b->sms * 8, 256, 0, b->st>>>(n, d_idx, BHUB_MIN, d_cnt);
         ull cnt = 0;
         const cudaError_t err = cudaMemcpyAsync(&cnt, d_cnt, sizeof(ull), cudaMemcpyDeviceToHost, b->st);
         cudaStreamSynchronize(b->st);
@@ -493,14 +490,6 @@ static int batch_setup(excent_batch* b, int device, int n, ull m, const ull* d_i
     BX_ALLOC(b->d_seg, b->seg_cap * sizeof(BSeg));
     BX_ALLOC(b->d_ctrl, sizeof(BCtrl));
     BX_ALLOC(b->d_col, (size_t)n * sizeof(float));
-    int occ = 0;
-    switch (B) {
-        case 32: EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bpass<8, 1>, BB, 0)); break;
-        case 64: EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bpass<16, 1>, BB, 0)); break;
-        case 128: EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bpass<32, 1>, BB, 0)); break;
-        default: EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bpass<32, 2>, BB, 0)); break;
-    }
-    b->grid = b->sms * std::max(1, occ);
     return EXCENT_OK;
 }
 
@@ -568,59 +557,17 @@ extern "C" int excent_batch_seed(excent_batch* b, int nq, const int* lane_off, c
     return EXCENT_OK;
 }
 
-static int batch_graph(excent_batch* b, int max_passes) {
-    if (b->gexec && b->graph_max == max_passes) return EXCENT_OK;
-    if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
-    if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
-    cudaGraph_t g;
-    EX_CUDA(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle h;
-    EX_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    EX_CUDA(cudaGraphAddNode(&node, g, nullptr, 0, &cp));
-    cudaStream_t cs;
-    EX_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    EX_CUDA(cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal));
-    const ull before = b->launches;
-    launch_pass(b, cs, h, 1);
-    b->launches = before;
-    cudaGraph_t captured;
-    const cudaError_t ce = cudaStreamEndCapture(cs, &captured);
-    cudaStreamDestroy(cs);
-    EX_CUDA(ce);
-    EX_CUDA(cudaGraphInstantiate(&b->gexec, g, 0));
-    b->graph = g;
-    b->graph_max = max_passes;
-    return EXCENT_OK;
-}
-
 extern "C" int excent_batch_solve(excent_batch* b, int max_passes, int use_graph) {
     EX_CHECK_ARG(b && max_passes >= 1, "bad argument");
+    (void)use_graph;   // every pass runs in one launch either way
     EX_CUDA(cudaSetDevice(b->dev));
     BCtrl c{};
     c.max_passes = max_passes;
     EX_CUDA(cudaMemcpyAsync(b->d_ctrl, &c, sizeof c, cudaMemcpyHostToDevice, b->st));
-    if (use_graph) {
-        EX_TRY(batch_graph(b, max_passes));
-        EX_CUDA(cudaGraphLaunch(b->gexec, b->st));
-        EX_CUDA(cudaStreamSynchronize(b->st));
-        EX_CUDA(cudaMemcpy(&c, b->d_ctrl, sizeof c, cudaMemcpyDeviceToHost));
-        b->launches += 3ull * (c.pass + 1);
-    } else {
-        for (int p = 0; p < max_passes; p++) {
-            launch_pass(b, b->st, 0, 0);
-            EX_CUDA(cudaGetLastError());
-            EX_CUDA(cudaMemcpyAsync(&c, b->d_ctrl, sizeof c, cudaMemcpyDeviceToHost, b->st));
-            EX_CUDA(cudaStreamSynchronize(b->st));
-            if (c.done) break;
-        }
-    }
+    EX_CUDA(launch_solve(b));
+    EX_CUDA(cudaMemcpyAsync(&c, b->d_ctrl, sizeof c, cudaMemcpyDeviceToHost, b->st));
+    EX_CUDA(cudaStreamSynchronize(b->st));
+    if (c.bar.failed) EX_FAIL(EXCENT_ERR_STATE, "batch: a wait between the blocks of a solve timed out");
     if (c.err) EX_FAIL(EXCENT_ERR_STATE, "batch: hub buffer capacity exceeded");
     return EXCENT_OK;
 }
@@ -656,18 +603,12 @@ extern "C" int excent_batch_read(excent_batch* b, int lane, int residual, float*
 extern "C" int excent_batch_set_dense(excent_batch* b, int groups) {
     EX_CHECK_ARG(b && groups >= 0, "bad argument");
     b->dense = groups;
-    if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
-    if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
-    b->graph_max = -1;
     return EXCENT_OK;
 }
 
 extern "C" int excent_batch_set_greedy(excent_batch* b, int greedy) {
     EX_CHECK_ARG(b, "null batch");
     b->greedy = greedy != 0;
-    if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
-    if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
-    b->graph_max = -1;
     return EXCENT_OK;
 }
 
