@@ -15,6 +15,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -67,14 +68,12 @@ struct WaveCount {
 
 // Device control block: counters that live across kernels of one pass.
 struct Ctrl {
-    ull hotpend;
     ull pushed;        // adjacency entries pushed since init
     ull items;         // work items of the cached push in this pass
     int pass;          // passes that pushed so far
     int done;          // 1 once a snapshot found nothing pending (or max passes)
     int err;           // 1: a hub queue overflowed; 3: a bounded wait for a bulk copy gave up
     int sweep_pass;    // this pass is pushed chunk by chunk (set by k_plan)
-    double rsum[MAXM]; // FP64 sum |r| of the last snapshot
     unsigned hcount;   // hot pending list length
     unsigned pad2;
     double ev_dot;     // FP64 (r_ev . v1) accumulated by the snapshot
@@ -86,6 +85,10 @@ struct Ctrl {
     SnapAcc acc[2];    // persistent solve: by pass parity
     WaveCount wave[3]; // by take phase
     GridBar bar;
+    // what a snapshot of the host-driven loop adds up; the demand table follows the block in
+    // memory, so that one memset clears and one copy fetches it all
+    ull hotpend;
+    double rsum[MAXM]; // FP64 sum |r| of the last snapshot
 };
 
 struct PassRec {
@@ -97,6 +100,7 @@ struct PassRec {
 
 struct SnapArgs {
     int n, nc, words, groups_per_warp;
+    int group;         // bitmap words per warp step
     void* r;
     const float* v1;   // unit principal eigenvector (EV normalisation step) or null
     int ev;            // measure index of the eigenvector
@@ -353,7 +357,7 @@ __global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
     const int lane = threadIdx.x & 31;
     const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     SnapSums sums;
-    snapshot_scan<L>(a, a.cnt, SNAP_GROUP, gw * a.groups_per_warp, (gw + 1) * a.groups_per_warp,
+    snapshot_scan<L>(a, a.cnt, a.group, gw * a.groups_per_warp, (gw + 1) * a.groups_per_warp,
                      a.v1 ? a.ctrl->ev_corr : 0.0, sums, lane);
     double rs0 = sums.rs0, rs1 = sums.rs1, rs2 = sums.rs2, evd = sums.evd;
     unsigned hp = sums.hp;
@@ -961,7 +965,7 @@ struct excent_engine {
     double prof_ms[4] = {0, 0, 0, 0};  // snapshot, plan, push, hub
     ull prof_passes = 0;
     // launch grids
-    int grid_push = 0, grid_snap = 0, groups_per_warp = 1;
+    int grid_push = 0, grid_snap = 0, groups_per_warp = 1, snap_group = SNAP_GROUP;
     ull launches = 0;
     ull n_list = 0, n_range = 0;
 };
@@ -1029,11 +1033,11 @@ static int free_engine(excent_engine* e) {
     cudaDeviceSynchronize();
     if (e->gexec) cudaGraphExecDestroy(e->gexec);
     if (e->graph) cudaGraphDestroy(e->graph);
-    void* dptrs[] = {e->d_sweep, e->d_hub_counts, e->d_cnt2, e->d_small, e->d_hub_id, e->d_hubv, e->d_hubv_cnt, e->d_v1, e->d_idx, e->d_x, e->d_r, e->d_bitmap, e->d_cnt, e->d_cv0, e->d_list, e->d_ctrl, e->d_cmode,
+    void* dptrs[] = {e->d_sweep, e->d_hub_counts, e->d_small, e->d_hub_id, e->d_hubv, e->d_hubv_cnt, e->d_v1, e->d_idx, e->d_x, e->d_r, e->d_bitmap, e->d_cv0, e->d_list, e->d_ctrl, e->d_cmode,
                      e->d_wt_type, e->d_wt_prefix, e->d_hubq[0], e->d_hubq[1], e->d_hubq[2], e->d_queue, e->d_log, e->d_trace, e->d_tmp, e->d_cache,
                      e->d_hids, e->d_hoff, e->d_hedges, e->d_hot, e->d_hlist};
     for (void* p : dptrs) if (p) cudaFree(p);
-    void* hptrs[] = {e->h_cnt, e->h_ctrl, e->h_wt_type, e->h_wt_prefix};
+    void* hptrs[] = {e->h_ctrl, e->h_wt_type, e->h_wt_prefix};
     for (void* p : hptrs) if (p) cudaFreeHost(p);
     for (Slot& s : e->slot) {
         if (s.h_edges) cudaFreeHost(s.h_edges);
@@ -1106,10 +1110,11 @@ static int engine_setup(excent_engine* e, int device, int n, ull m, const excent
     EX_ALLOC(e->d_x, vbytes);
     EX_ALLOC(e->d_r, vbytes);
     EX_ALLOC(e->d_bitmap, words * sizeof(uint32_t));
-    EX_ALLOC(e->d_cnt, 2 * (size_t)nc * sizeof(ull));
     EX_ALLOC(e->d_cv0, (size_t)nc * sizeof(int));
     EX_ALLOC(e->d_list, (size_t)n * sizeof(int));
-    EX_ALLOC(e->d_ctrl, sizeof(Ctrl));
+    EX_ALLOC(e->d_ctrl, sizeof(Ctrl) + 4 * (size_t)nc * sizeof(ull));
+    e->d_cnt = reinterpret_cast<ull*>(e->d_ctrl + 1);
+    e->d_cnt2 = e->d_cnt + 2 * (size_t)nc;
     EX_ALLOC(e->d_cmode, (size_t)nc);
     EX_ALLOC(e->d_wt_type, (size_t)nc);
     EX_ALLOC(e->d_wt_prefix, ((size_t)nc + 1) * sizeof(unsigned));
@@ -1120,24 +1125,24 @@ static int engine_setup(excent_engine* e, int device, int n, ull m, const excent
     e->log_cap = 1 << 17;
     EX_ALLOC(e->d_log, (size_t)e->log_cap * sizeof(PassRec));
     if (e->L == 4) EX_ALLOC(e->d_tmp, (size_t)n * sizeof(float));
-    EX_HALLOC(e->h_cnt, 2 * (size_t)nc * sizeof(ull));
-    EX_HALLOC(e->h_ctrl, sizeof(Ctrl));
+    EX_HALLOC(e->h_ctrl, sizeof(Ctrl) + 2 * (size_t)nc * sizeof(ull));
+    e->h_cnt = reinterpret_cast<ull*>(e->h_ctrl + 1);
     EX_HALLOC(e->h_wt_type, (size_t)nc);
     EX_HALLOC(e->h_wt_prefix, ((size_t)nc + 1) * sizeof(unsigned));
     EX_CUDA(cudaMemcpy(e->d_cv0, chunk_v0, (size_t)nc * sizeof(int), cudaMemcpyHostToDevice));
-    EX_CUDA(cudaMemset(e->d_ctrl, 0, sizeof(Ctrl)));
-    EX_CUDA(cudaMemset(e->d_cnt, 0, 2 * (size_t)nc * sizeof(ull)));
+    EX_CUDA(cudaMemset(e->d_ctrl, 0, sizeof(Ctrl) + 4 * (size_t)nc * sizeof(ull)));
     EX_CUDA(cudaMemset(e->d_cmode, 0, (size_t)nc));
     EX_CUDA(cudaMemset(e->d_queue, 0, 3 * sizeof(PushQueue)));
     EX_TRY(push_blocks(e, 0, &e->grid_push));
     e->wave = std::min(e->grid_push * BLOCK, WAVE_MAX);
-    EX_ALLOC(e->d_cnt2, 2 * (size_t)nc * sizeof(ull));
     EX_ALLOC(e->d_small, (size_t)std::min(n, WAVE_MAX) * sizeof(HubSeg));
     int occs = 0;
     if (e->L == 1) EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occs, k_snapshot<1>, BLOCK, 0));
     else EX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occs, k_snapshot<4>, BLOCK, 0));
-    const long long groups = ((long long)words + SNAP_GROUP - 1) / SNAP_GROUP;
     const long long max_warps = (long long)e->sms * std::max(1, occs) * (BLOCK / 32);
+    // a word per warp step while there are warps for it, up to SNAP_GROUP
+    e->snap_group = (int)std::max(1LL, std::min((long long)SNAP_GROUP, (long long)words / max_warps));
+    const long long groups = ((long long)words + e->snap_group - 1) / e->snap_group;
     e->groups_per_warp = (int)std::max(1LL, (groups + max_warps - 1) / max_warps);
     const long long warps = (groups + e->groups_per_warp - 1) / e->groups_per_warp;
     e->grid_snap = (int)std::max(1LL, (warps + BLOCK / 32 - 1) / (BLOCK / 32));
@@ -1292,10 +1297,8 @@ extern "C" int excent_engine_read_trace(excent_engine* e, uint16_t* out) {
 }
 
 static int reset_counters(excent_engine* e) {
-    EX_CUDA(cudaMemsetAsync(e->d_ctrl, 0, sizeof(Ctrl), e->s_main));
+    EX_CUDA(cudaMemsetAsync(e->d_ctrl, 0, sizeof(Ctrl) + 4 * (size_t)e->nc * sizeof(ull), e->s_main));
     EX_CUDA(cudaMemsetAsync(e->d_queue, 0, 3 * sizeof(PushQueue), e->s_main));
-    EX_CUDA(cudaMemsetAsync(e->d_cnt, 0, 2 * (size_t)e->nc * sizeof(ull), e->s_main));
-    EX_CUDA(cudaMemsetAsync(e->d_cnt2, 0, 2 * (size_t)e->nc * sizeof(ull), e->s_main));
     if (e->d_trace && e->trace_on) EX_CUDA(cudaMemsetAsync(e->d_trace, 0, (size_t)e->n * sizeof(uint16_t), e->s_main));
     e->hot_skip = false;
     e->n_list = e->n_range = 0;
@@ -1330,6 +1333,7 @@ extern "C" int excent_engine_init(excent_engine* e) {
 static SnapArgs snap_args(excent_engine* e, bool use_hot) {
     SnapArgs a{};
     a.n = e->n; a.nc = e->nc; a.words = (int)(((size_t)e->n + 31) / 32); a.groups_per_warp = e->groups_per_warp;
+    a.group = e->snap_group;
     a.r = e->d_r; a.M = e->M; a.idx = e->d_idx; a.cv0 = e->d_cv0;
     a.v1 = e->ev_proj ? e->d_v1 : nullptr;
     a.ev = e->ev_index;
@@ -1353,14 +1357,13 @@ extern "C" int excent_engine_snapshot(excent_engine* e, int use_hot, unsigned lo
     EX_CHECK_ARG(e, "null engine");
     EX_CHECK_ARG(!use_hot || e->d_hot, "hot snapshot without a hot cache");
     EX_CUDA(cudaSetDevice(e->dev));
-    EX_CUDA(cudaMemsetAsync(e->d_cnt, 0, 2 * (size_t)e->nc * sizeof(ull), e->s_main));
-    EX_CUDA(cudaMemsetAsync(&e->d_ctrl->hotpend, 0, sizeof(ull), e->s_main));
-    EX_CUDA(cudaMemsetAsync(e->d_ctrl->rsum, 0, sizeof(double) * MAXM, e->s_main));
+    EX_CUDA(cudaMemsetAsync(&e->d_ctrl->hotpend, 0, sizeof(Ctrl) - offsetof(Ctrl, hotpend) + 2 * (size_t)e->nc * sizeof(ull),
+                            e->s_main));
     e->hot_skip = use_hot != 0;
     launch_snapshot(e, use_hot != 0, e->s_main);
     EX_CUDA(cudaGetLastError());
-    EX_CUDA(cudaMemcpyAsync(e->h_cnt, e->d_cnt, 2 * (size_t)e->nc * sizeof(ull), cudaMemcpyDeviceToHost, e->s_main));
-    EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
+    EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl) + 2 * (size_t)e->nc * sizeof(ull), cudaMemcpyDeviceToHost,
+                            e->s_main));
     EX_CUDA(cudaStreamSynchronize(e->s_main));
     if (e->ev_proj) {   // next snapshot removes the component measured by this one
         Ctrl* hc = e->h_ctrl;
@@ -1447,6 +1450,11 @@ static int grid_for(excent_engine* e, ull items) {
     return (int)std::max<ull>(1, std::min<ull>(blocks, (ull)e->grid_push));
 }
 
+static SolveArgs solve_args(excent_engine* e, double list_frac, int max_passes);
+static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st);
+static cudaError_t launch_table(excent_engine* e, SolveArgs& a, cudaStream_t st);
+static int ensure_sweep(excent_engine* e);
+
 extern "C" int excent_engine_push_cached(excent_engine* e, const unsigned char* mode, const unsigned long long* cnt,
                                          double list_frac) {
     EX_CHECK_ARG(e && mode && cnt, "null argument");
@@ -1471,16 +1479,29 @@ extern "C" int excent_engine_push_cached(excent_engine* e, const unsigned char* 
     EX_CUDA(cudaMemcpyAsync(e->d_wt_type, e->h_wt_type, e->nc, cudaMemcpyHostToDevice, e->s_main));
     EX_CUDA(cudaMemcpyAsync(e->d_wt_prefix, e->h_wt_prefix, ((size_t)e->nc + 1) * sizeof(unsigned),
                             cudaMemcpyHostToDevice, e->s_main));
+    ull demand = 0;
+    bool all_cached = true;
+    for (int c = 0; c < e->nc; c++) {
+        demand += cnt[2 * c + 1];
+        all_cached &= cnt[2 * c] == 0 || mode[c] == 1;
+    }
+    const bool sweep = sweep_of(e) && demand >= sweep_min_entries(e);
     // a high-degree order needs every chunk with work in the cache (the hub list spans the graph);
     // the hub list is built before the push arguments are taken, which point at it
-    bool all_cached = true;
-    for (int c = 0; c < e->nc; c++) all_cached &= cnt[2 * c] == 0 || mode[c] == 1;
+    if (all_cached && order_of(e)) EX_TRY(ensure_hubv(e));
+    // with every pending list in the cache, and none kept apart in the degree cache, the push is one
+    // launch; it was up to three kernels and two memsets a chunk
+    if (all_cached && !e->hot_skip && effective_order(e) == order_of(e)) {
+        if (sweep) EX_TRY(ensure_sweep(e));
+        SolveArgs s = solve_args(e, list_frac, 0);
+        s.standalone = 1;
+        EX_CUDA(sweep ? launch_sweep(e, s, e->s_main) : launch_table(e, s, e->s_main));
+        e->launches++;
+        return EXCENT_OK;
+    }
     int order = 0;
     if (order_of(e) == 3) order = 3;   // inside each launch: needs no high-degree list
-    else if (all_cached && order_of(e) && !sweep_of(e)) {
-        EX_TRY(ensure_hubv(e));
-        order = effective_order(e);
-    }
+    else if (all_cached && !sweep_of(e)) order = effective_order(e);
     PushArgs a = push_args(e, 0);
     a.hot = e->hot_skip ? e->d_hot : nullptr;
     if (order == 1) launch_push<SRC_HUBS>(e, a, e->grid_push, e->s_main);
@@ -1494,9 +1515,7 @@ extern "C" int excent_engine_push_cached(excent_engine* e, const unsigned char* 
         }
         launch_push<SRC_TABLE>(e, a, grid_for(e, items), e->s_main);
     };
-    ull demand = 0;
-    for (int c = 0; c < e->nc; c++) demand += cnt[2 * c + 1];
-    if (sweep_of(e) && demand >= sweep_min_entries(e)) {   // one launch per chunk, in chunk order
+    if (sweep) {   // one launch per chunk, in chunk order
         for (int c = 0; c < e->nc; c++) {
             const unsigned items = e->h_wt_prefix[c + 1] - e->h_wt_prefix[c];
             if (!items) continue;
@@ -1705,10 +1724,11 @@ extern "C" int excent_engine_hot_edges(excent_engine* e, int32_t* out) {
 extern "C" int excent_engine_sync(excent_engine* e) {
     EX_CHECK_ARG(e, "null engine");
     EX_CUDA(cudaSetDevice(e->dev));
-    EX_CUDA(cudaStreamSynchronize(e->s_main));
     if (e->slots_ok) for (Slot& s : e->slot) { EX_CUDA(cudaStreamSynchronize(s.st)); s.busy = false; }
-    int err = 0;
-    EX_CUDA(cudaMemcpy(&err, &e->d_ctrl->err, sizeof(int), cudaMemcpyDeviceToHost));
+    EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
+    EX_CUDA(cudaStreamSynchronize(e->s_main));
+    const int err = e->h_ctrl->err;
+    if (e->h_ctrl->bar.failed) EX_FAIL(EXCENT_ERR_STATE, "a wait between the blocks of a push timed out");
     if (err) scrub_queues(e);
     if (err) EX_FAIL(EXCENT_ERR_STATE, "%s", ctrl_error(err));
     return EXCENT_OK;
@@ -1817,6 +1837,9 @@ static int solve_grid(const excent_engine* e) { return std::max(1, std::min(e->s
 static cudaError_t launch_passes(excent_engine* e, SolveArgs& a, cudaStream_t st) {
     return launch_grid(e->L == 1 ? k_passes<1> : k_passes<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
 }
+static cudaError_t launch_table(excent_engine* e, SolveArgs& a, cudaStream_t st) {
+    return launch_grid(e->L == 1 ? k_table<1> : k_table<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
+}
 static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st) {
     if (e->sweep_ok && a.order == 3) {
         SweepArgs s{a, e->sweep};
@@ -1833,6 +1856,7 @@ static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st)
 static int ensure_sweep(excent_engine* e) {
     if (!e->sweep_stale) return EXCENT_OK;
     if (!sweep_of(e) || effective_order(e) != 3 || e->d_hcache || e->cache_edges != e->m) return EXCENT_OK;   // may change
+    for (uint8_t ok : e->loaded) if (!ok) return EXCENT_OK;
     e->sweep_stale = false;
     const size_t n = (size_t)e->n, tb = e->L == 1 ? sizeof(float) : sizeof(float4);
     const ull m = e->m;
@@ -2272,6 +2296,8 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
         cudaFuncSetAttribute(k_push<4, SRC_HUBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_passes<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_passes<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
+        cudaFuncSetAttribute(k_table<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
+        cudaFuncSetAttribute(k_table<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_sweep<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_segments<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);

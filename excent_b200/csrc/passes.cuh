@@ -41,6 +41,7 @@ struct SolveArgs {
     int wave;              // items taken together before they are scattered
     unsigned seg;          // entries per segment
     HubSeg* small;         // taken lists of at most WAVE_LONG entries (wave records)
+    int standalone;        // one push of the host-driven loop: its table and counts stay as they are
     cudaGraphConditionalHandle again, go_sweep;
     int use_cond;
 };
@@ -490,23 +491,41 @@ __global__ void __launch_bounds__(PT, 1) k_passes(SolveArgs a) {
     }
 }
 
+// One push of the whole table (host-driven loop).
+template <int L>
+__global__ void __launch_bounds__(PT, 1) k_table(SolveArgs a) {
+    typedef typename Lane<L>::T T;
+    __shared__ PassShared<L> s;
+    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        for (WaveCount& w : a.push.ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }
+    if (!P.sync()) return;
+    const long long nh = a.order ? (long long)*a.push.hubv_cnt : 0;
+    if ((a.order == 1 || a.order == 3) && !P.push_hubs(0, nh, false)) return;
+    if (!P.push_table(0, P.prefix[a.push.nc], -1, a.order ? LISTS_SHORT : LISTS_ALL)) return;
+    if (a.order == 2 && !P.push_hubs(0, nh, false)) return;
+    P.report();
+}
+
+// After a swept pass of a device solve: every table and sum of the passes, for the next k_passes.
+__device__ __forceinline__ void clear_tables(const SolveArgs& a, int threads) {
+    if (a.standalone || blockIdx.x) return;
+    for (int c = threadIdx.x; c < 2 * a.push.nc; c += threads) { a.snap.cnt[c] = 0; a.cnt2[c] = 0; }
+    if (threadIdx.x == 0) { a.push.ctrl->acc[0] = SnapAcc{}; a.push.ctrl->acc[1] = SnapAcc{}; }
+}
+
 // One pass chunk by chunk, in chunk order, per the table k_passes left.
 template <int L>
 __global__ void __launch_bounds__(PT, 1) k_sweep(SolveArgs a) {
     typedef typename Lane<L>::T T;
     __shared__ PassShared<L> s;
     Ctrl* ctrl = a.push.ctrl;
-    if (ctrl->done || !ctrl->sweep_pass) return;
+    if (!a.standalone && (ctrl->done || !ctrl->sweep_pass)) return;
     Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
     const int nc = a.push.nc;
-    if (blockIdx.x == 0) {   // every table and sum of the passes, for the next k_passes
-        for (int c = threadIdx.x; c < 2 * nc; c += PT) { a.snap.cnt[c] = 0; a.cnt2[c] = 0; }
-        if (threadIdx.x == 0) {
-            for (WaveCount& w : ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }
-            ctrl->acc[0] = SnapAcc{};
-            ctrl->acc[1] = SnapAcc{};
-        }
-    }
+    clear_tables(a, PT);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        for (WaveCount& w : ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }
     if (!P.sync()) return;
     const int order = a.order;
     if (order == 1 && !P.push_hubs(0, (long long)*a.push.hubv_cnt, false)) return;

@@ -455,13 +455,10 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(SweepArgs args) {
     __shared__ ull s_tot[3][GW];
     __shared__ unsigned s_next;
     Ctrl* ctrl = a.push.ctrl;
-    if (ctrl->done || !ctrl->sweep_pass) return;
+    if (!a.standalone && (ctrl->done || !ctrl->sweep_pass)) return;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nc = a.push.nc;
     unsigned epoch = 0;
-    if (blockIdx.x == 0) {   // every table and sum of the passes, for the next k_passes
-        for (int c = threadIdx.x; c < 2 * nc; c += GT) { a.snap.cnt[c] = 0; a.cnt2[c] = 0; }
-        if (threadIdx.x == 0) { ctrl->acc[0] = SnapAcc{}; ctrl->acc[1] = SnapAcc{}; }
-    }
+    clear_tables(a, GT);
     T* x = reinterpret_cast<T*>(a.push.x);
     T* r = reinterpret_cast<T*>(a.push.r);
     T* P = reinterpret_cast<T*>(g.P);
