@@ -232,9 +232,9 @@ struct SnapSums {
     double rs0 = 0, rs1 = 0, rs2 = 0, evd = 0;
     unsigned hp = 0;
 };
-template <int L>
+template <int L, typename F>
 __device__ __forceinline__ void snapshot_scan(const SnapArgs& a, ull* cnt, int group, long long g0, long long g1,
-                                              double evc_in, SnapSums& sums, int lane) {
+                                              double evc_in, SnapSums& sums, int lane, const F& on_pending) {
     typedef typename Lane<L>::T T;
     T* r = reinterpret_cast<T*>(a.r);
     const long long ngroups = (a.words + group - 1) / group;
@@ -292,7 +292,11 @@ __device__ __forceinline__ void snapshot_scan(const SnapArgs& a, ull* cnt, int g
                     pend = pending_of(rv, a.M);
                     if (a.trace && pend) a.trace[v]++;
                     if (a.hot && pend && bit_of(a.hot, v)) { hp++; pend = false; }
-                    if (pend) mydeg += a.idx[v + 1] - a.idx[v];
+                    if (pend) {
+                        const ull deg = a.idx[v + 1] - a.idx[v];
+                        mydeg += deg;
+                        on_pending(v, rv, deg);
+                    }
                 }
                 const uint32_t b = __ballot_sync(FULL, pend);
                 if (lane == j) myb = b;
@@ -358,7 +362,7 @@ __global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
     const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     SnapSums sums;
     snapshot_scan<L>(a, a.cnt, a.group, gw * a.groups_per_warp, (gw + 1) * a.groups_per_warp,
-                     a.v1 ? a.ctrl->ev_corr : 0.0, sums, lane);
+                     a.v1 ? a.ctrl->ev_corr : 0.0, sums, lane, [](long long, const typename Lane<L>::T&, ull) {});
     double rs0 = sums.rs0, rs1 = sums.rs1, rs2 = sums.rs2, evd = sums.evd;
     unsigned hp = sums.hp;
     // FP64 termination residual and hot pending count: block reduction, one atomic each

@@ -20,7 +20,10 @@
 
 namespace excent {
 
-static constexpr int PT = 1024;               // threads per block, one block per SM
+// Threads per block, one block per SM: 1024 leave 64 registers a thread and spill in the snapshot
+// (sample of 2000 vertices: 1.34 ms a solve, 1.23 with 768), 512 are too few for the large passes
+// (R-MAT 24 PageRank: 47.7, 48.0 and 49.7 ms with 1024, 768 and 512).
+static constexpr int PT = 768;
 static constexpr int PW = PT / 32;
 static constexpr unsigned WAVE_LONG = 32;     // longer lists of a wave are scattered as segments
 static constexpr int PLAN_LOCAL = PT;         // up to this many chunks every block plans for itself
@@ -46,12 +49,57 @@ struct SolveArgs {
     int use_cond;
 };
 
+// Take vertex v, whose residual is rv, in a phase in which nobody adds to
+// residuals: the take of device.cuh without its exchanges.
+__device__ __forceinline__ float take_alone(float* x, float* r, int v, float rv, ull deg, const DevMeasures& M) {
+    if (!(fabsf(rv) > M.eps[0])) return 0.f;
+    r[v] = 0.f;
+    x[v] += rv;
+    return weight(rv, deg, M, 0);
+}
+__device__ __forceinline__ float4 take_alone(float4* x, float4* r, int v, float4 rv, ull deg, const DevMeasures& M) {
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (fabsf(rv.x) > M.eps[0]) { d.x = rv.x; rv.x = 0.f; }
+    if (M.nm > 1 && fabsf(rv.y) > M.eps[1]) { d.y = rv.y; rv.y = 0.f; }
+    if (M.nm > 2 && fabsf(rv.z) > M.eps[2]) { d.z = rv.z; rv.z = 0.f; }
+    if (!nonzero(d)) return d;
+    r[v] = rv;
+    float4 xv = x[v];
+    xv.x += d.x; xv.y += d.y; xv.z += d.z;
+    x[v] = xv;
+    return make_float4(weight(d.x, deg, M, 0), weight(d.y, deg, M, 1), weight(d.z, deg, M, 2), 0.f);
+}
+
+// Take one hub vertex and queue its segments: called by one lane from the
+// snapshot, before the barrier that follows it (nobody adds to residuals
+// there). The measures its weight carries. Out of line: it would be unrolled
+// with the snapshot's loads and take their registers.
+template <int L>
+__device__ __noinline__ unsigned take_hub(const SolveArgs& a, WaveCount* w, int v, typename Lane<L>::T rv, unsigned deg) {
+    typedef typename Lane<L>::T T;
+    const T p = take_alone(reinterpret_cast<T*>(a.push.x), reinterpret_cast<T*>(a.push.r), v, rv, deg, a.push.M);
+    if (!nonzero(p)) return 0;
+    const unsigned nseg = (deg + a.seg - 1) / a.seg;
+    const ull at = atomicAdd(&w->big, nseg);
+    if (at + nseg > a.push.hub_cap) { atomicExch(&a.push.ctrl->err, 1); return 0; }
+    HubSeg h;
+    h.pad = 0;
+    if constexpr (L == 1) h.p = make_float4(p, 0.f, 0.f, 0.f); else h.p = p;
+    const int* nb = list_at(a.push, a.push.idx[v]);
+    for (unsigned k = 0; k < nseg; k++) {
+        h.nb = nb + (ull)k * a.seg;
+        h.len = min(a.seg, deg - k * a.seg);
+        a.push.hubq[at + k] = h;
+    }
+    return measures_in(p);
+}
+
 // Sum of (a, b) of every warp before this one in the block, and of the block.
 __device__ __forceinline__ void block_offsets(unsigned a, unsigned b, unsigned (&s)[2][PW], int wib, int lane,
                                               unsigned& oa, unsigned& ob, unsigned& ta, unsigned& tb) {
     if (lane == 0) { s[0][wib] = a; s[1][wib] = b; }
     __syncthreads();
-    const unsigned va = s[0][lane], vb = s[1][lane];
+    const unsigned va = lane < PW ? s[0][lane] : 0u, vb = lane < PW ? s[1][lane] : 0u;
     const unsigned ia = warp_incl_scan(va, lane), ib = warp_incl_scan(vb, lane);
     oa = __shfl_sync(FULL, ia - va, wib);
     ob = __shfl_sync(FULL, ib - vb, wib);
@@ -135,7 +183,7 @@ template <int L> struct Passes {
                 b = a.push.idx[v];
                 deg = a.push.idx[v + 1] - b;
                 if (!(which == LISTS_SHORT && deg > HUB_MIN) && !(which == LISTS_LONG && deg <= HUB_MIN))
-                    p = take(x, r, v, deg, a.push.M);
+                    p = take_alone(x, r, v, r[v], deg, a.push.M);
             }
             const bool act = nonzero(p) && deg > 0;
             if (act) count(p, deg, b);
@@ -211,7 +259,9 @@ template <int L> struct Passes {
     // Scatter what the last take phase queued: segments, one warp each, then
     // tiles of short lists; blocks share them interleaved, a block's warps claim.
     __device__ __forceinline__ void scatter_wave(ull nbig, unsigned nsmall) {
-        const ull ntiles = ((ull)nsmall + 31) / 32;
+        // 32 lists to a tile, down to 8 while there are warps for them
+        const unsigned per_tile = min(32u, max(8u, nsmall / (gridDim.x * PW)));
+        const ull ntiles = ((ull)nsmall + per_tile - 1) / per_tile;
         for (;;) {
             unsigned k = 0;
             if (lane == 0) k = atomicAdd(&s.next, 1u);
@@ -223,11 +273,11 @@ template <int L> struct Passes {
                 if constexpr (L == 1) p = p4.x; else p = p4;
                 warp_scatter(r, h->nb, h->len, p, lane, hacc);
             } else if (i - nbig < ntiles) {
-                const ull j = (i - nbig) * 32 + lane;
+                const ull j = (i - nbig) * per_tile + lane;
                 const int* nb = nullptr;
                 unsigned ds = 0;
                 T p{};
-                if (j < nsmall) {
+                if (lane < per_tile && j < nsmall) {
                     const HubSeg h = a.small[j];
                     nb = h.nb;
                     ds = h.len;
@@ -328,6 +378,15 @@ template <int L> struct Passes {
         return sync();
     }
 
+    // Scatter what the snapshot took (the phase after its barrier).
+    __device__ __forceinline__ bool push_taken_hubs() {
+        const ull nbig = min((ull)counts(phase).big, a.push.hub_cap);
+        phase++;
+        if (!nbig) return true;
+        scatter_wave(nbig, 0);
+        return sync();
+    }
+
     // The long lists of hub vertices [h0, h1), all taken before any is scattered.
     __device__ __forceinline__ bool push_hubs(long long h0, long long h1, bool listed) {
         if (h1 <= h0) return true;
@@ -354,7 +413,7 @@ template <int L> struct Passes {
         if (lane == 0) { s.tot[0][wib] = pushed; s.tot[1][wib] = lanes; s.tot[2][wib] = taken; s.tot[3][wib] = hpushed; }
         __syncthreads();
         if (wib < 4) {
-            const ull t = warp_sum(s.tot[wib][lane]);
+            const ull t = warp_sum(lane < PW ? s.tot[wib][lane] : 0ull);
             Ctrl* c = a.push.ctrl;
             if (lane == 0 && t) atomicAdd(wib == 0 ? &c->pushed : wib == 1 ? &c->lanes : wib == 2 ? &c->taken : &c->host_pushed, t);
         }
@@ -362,22 +421,23 @@ template <int L> struct Passes {
     }
 };
 
-// Snapshot of the whole graph by all blocks; sums into acc.
-template <int L>
+// Snapshot of the whole graph by all blocks; sums into acc. on_pending(v, residual, degree) for
+// every pending vertex.
+template <int L, typename F>
 __device__ __forceinline__ void solve_snapshot(const SolveArgs& a, PassShared<L>& s, ull* cnt, SnapAcc* acc, double ev_corr,
-                                               int lane, int wib) {
+                                               int lane, int wib, const F& on_pending) {
     const long long groups = (a.snap.words + a.snap_group - 1) / a.snap_group;
     const long long nwarps = (long long)gridDim.x * PW;
     // a contiguous run of groups per warp; with fewer groups than warps, neighbours on different SMs
     const long long per = (groups + nwarps - 1) / nwarps;
     const long long gw = per > 1 ? (long long)blockIdx.x * PW + wib : (long long)wib * gridDim.x + blockIdx.x;
     SnapSums q;
-    snapshot_scan<L>(a.snap, cnt, a.snap_group, gw * per, (gw + 1) * per, ev_corr, q, lane);
+    snapshot_scan<L>(a.snap, cnt, a.snap_group, gw * per, (gw + 1) * per, ev_corr, q, lane, on_pending);
     q.rs0 = warp_sum(q.rs0); q.rs1 = warp_sum(q.rs1); q.rs2 = warp_sum(q.rs2); q.evd = warp_sum(q.evd);
     if (lane == 0) { s.rs[0][wib] = q.rs0; s.rs[1][wib] = q.rs1; s.rs[2][wib] = q.rs2; s.rs[3][wib] = q.evd; }
     __syncthreads();
     if (wib < 4) {
-        const double t = warp_sum(s.rs[wib][lane]);
+        const double t = warp_sum(lane < PW ? s.rs[wib][lane] : 0.0);
         if (lane == 0 && t != 0.0) atomicAdd(wib < 3 ? &acc->rsum[wib] : &acc->ev_dot, t);
     }
 }
@@ -405,7 +465,7 @@ __device__ __forceinline__ unsigned solve_table(const SolveArgs& a, const ull* c
         const unsigned incl = warp_incl_scan(items, lane);
         if (lane == 31) scan[wib] = incl;
         __syncthreads();
-        const unsigned w = warp_incl_scan(scan[lane], lane);
+        const unsigned w = warp_incl_scan(lane < PW ? scan[lane] : 0u, lane);
         const unsigned before = wib ? __shfl_sync(FULL, w, wib - 1) : 0u;
         const unsigned all = __shfl_sync(FULL, w, 31);
         if (c < nc) { type[c] = ty; prefix[c + 1] = carry + before + incl; }
@@ -416,7 +476,7 @@ __device__ __forceinline__ unsigned solve_table(const SolveArgs& a, const ull* c
 }
 
 template <int L>
-__global__ void __launch_bounds__(PT, 1) k_passes(SolveArgs a) {
+__global__ void __launch_bounds__(PT, 1) k_passes(const __grid_constant__ SolveArgs a) {
     typedef typename Lane<L>::T T;
     __shared__ PassShared<L> s;
     __shared__ unsigned s_prefix[PLAN_LOCAL + 1];
@@ -428,12 +488,30 @@ __global__ void __launch_bounds__(PT, 1) k_passes(SolveArgs a) {
     Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
     const int lane = P.lane, wib = P.wib, nc = a.push.nc;
     const bool first_block = blockIdx.x == 0, lead = first_block && threadIdx.x == 0;
-    if (lead) for (WaveCount& w : ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }   // used after the first barrier
+    if (lead && a.sweep)   // what the sweep before left (otherwise the solve's reset cleared them)
+        for (WaveCount& w : ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }
     int pass = ctrl->pass;
     for (int k = 0;; k++, pass++) {
         ull* cnt = k & 1 ? a.cnt2 : a.snap.cnt;
         SnapAcc* acc = &ctrl->acc[k & 1];
-        solve_snapshot<L>(a, s, cnt, acc, a.snap.v1 ? ctrl->ev_corr : 0.0, lane, wib);
+        // without chunk-by-chunk passes the high-degree lists of this pass, which go first, can be taken
+        // right here (6.5 us less a pass than a phase of their own)
+        const bool take_hubs = a.order != 0 && a.order != 2 && !a.sweep && pass < a.max_passes;
+        WaveCount* taken_here = &P.counts(P.phase);
+        if (lead) {   // the next phase's counters: nobody uses them before the barrier
+            WaveCount& w = P.counts(P.phase + 1);
+            w.small = 0; w.big = 0; w.claim = 0;
+        }
+        solve_snapshot<L>(a, s, cnt, acc, a.snap.v1 ? ctrl->ev_corr : 0.0, lane, wib, [&](long long v, const T& rv, ull deg) {
+            if (!take_hubs || deg <= HUB_MIN) return;
+            const unsigned nz = take_hub<L>(a, taken_here, (int)v, rv, (unsigned)deg);
+            if (!nz) return;
+            P.pushed += deg;
+            P.lanes += deg * nz;
+            P.taken += nz;
+            if (a.push.hcache && a.push.idx[v] >= a.push.cache_edges) P.hpushed += deg;
+        });
+        if (threadIdx.x == 0) s.next = 0;
         if (!P.sync()) return;
         // pending vertices and entries of the whole graph, by every block
         if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
@@ -482,10 +560,13 @@ __global__ void __launch_bounds__(PT, 1) k_passes(SolveArgs a) {
         if (!local && !P.sync()) return;
         __syncthreads();
         const long long items = prefix[nc];
-        const long long nh = a.order ? (long long)*a.push.hubv_cnt : 0;
-        if (a.order == 1 || a.order == 3) { if (!P.push_hubs(0, nh, false)) return; }
+        if (take_hubs) {
+            if (!P.push_taken_hubs()) return;
+        } else if (a.order == 1 || a.order == 3) {
+            if (!P.push_hubs(0, (long long)*a.push.hubv_cnt, false)) return;
+        }
         if (!P.push_table(0, items, -1, a.order ? LISTS_SHORT : LISTS_ALL)) return;
-        if (a.order == 2) { if (!P.push_hubs(0, nh, false)) return; }
+        if (a.order == 2) { if (!P.push_hubs(0, (long long)*a.push.hubv_cnt, false)) return; }
         // the counters are read after the next snapshot's barrier
         P.report();
     }
@@ -493,7 +574,7 @@ __global__ void __launch_bounds__(PT, 1) k_passes(SolveArgs a) {
 
 // One push of the whole table (host-driven loop).
 template <int L>
-__global__ void __launch_bounds__(PT, 1) k_table(SolveArgs a) {
+__global__ void __launch_bounds__(PT, 1) k_table(const __grid_constant__ SolveArgs a) {
     typedef typename Lane<L>::T T;
     __shared__ PassShared<L> s;
     Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
@@ -516,7 +597,7 @@ __device__ __forceinline__ void clear_tables(const SolveArgs& a, int threads) {
 
 // One pass chunk by chunk, in chunk order, per the table k_passes left.
 template <int L>
-__global__ void __launch_bounds__(PT, 1) k_sweep(SolveArgs a) {
+__global__ void __launch_bounds__(PT, 1) k_sweep(const __grid_constant__ SolveArgs a) {
     typedef typename Lane<L>::T T;
     __shared__ PassShared<L> s;
     Ctrl* ctrl = a.push.ctrl;

@@ -447,7 +447,7 @@ struct SweepArgs {
     SweepLists g;
 };
 template <int L>
-__global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(SweepArgs args) {
+__global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_constant__ SweepArgs args) {
     const SolveArgs& a = args.a;
     const SweepLists& g = args.g;
     typedef typename Lane<L>::T T;
