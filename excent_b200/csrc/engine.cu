@@ -61,6 +61,7 @@ static constexpr unsigned SPIN_LIMIT = 1u << 24; // bounded polls of an mbarrier
 struct SnapAcc {
     double rsum[MAXM];
     double ev_dot;
+    ull pending, demand;   // (small graphs; elsewhere the demand table)
 };
 struct WaveCount {
     unsigned small, big, claim, pad;
@@ -866,6 +867,7 @@ __global__ void k_insert(int n, float4* s, int i, const float* in) {
 
 #include "passes.cuh"
 #include "sweep.cuh"
+#include "small.cuh"
 
 using namespace excent;
 
@@ -1838,6 +1840,20 @@ static SolveArgs solve_args(excent_engine* e, double list_frac, int max_passes) 
 
 // One block per SM, fewer where there is not a word of 32 vertices for each.
 static int solve_grid(const excent_engine* e) { return std::max(1, std::min(e->sms, (e->n + 31) / 32)); }
+// Whether a solve runs with every vertex in a thread's registers: one chunk whose vertices are taken
+// in one wave, the long lists first.
+static bool small_solve(const excent_engine* e, int order) {
+    return e->nc == 1 && !sweep_of(e) && (order == 1 || order == 3) && e->n <= e->wave &&
+           e->n <= e->sms * PT * SMALL_PER_THREAD && e->m < (1ull << 32);
+}
+static cudaError_t launch_small(excent_engine* e, SolveArgs& a, cudaStream_t st) {
+    const int per = e->n <= e->sms * PT ? 1 : 2;
+    auto kernel = e->L == 1 ? (per == 1 ? k_small<1, 1> : k_small<1, 2>) : (per == 1 ? k_small<4, 1> : k_small<4, 2>);
+    const size_t smem = (hub_smem(e) + 15) / 16 * 16 + (size_t)PT * per * (e->L == 1 ? sizeof(SmallRec<1>) : sizeof(SmallRec<4>));
+    const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (rc != cudaSuccess) return rc;
+    return launch_grid(kernel, solve_grid(e), PT, smem, a, &e->d_ctrl->bar, st);
+}
 static cudaError_t launch_passes(excent_engine* e, SolveArgs& a, cudaStream_t st) {
     return launch_grid(e->L == 1 ? k_passes<1> : k_passes<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
 }
@@ -2115,7 +2131,7 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
             EX_CUDA(cudaGraphLaunch(e->gexec, e->s_main));
         } else {   // every pass in one launch
             SolveArgs a = solve_args(e, list_frac, max_passes);
-            EX_CUDA(launch_passes(e, a, e->s_main));
+            EX_CUDA(small_solve(e, a.order) ? launch_small(e, a, e->s_main) : launch_passes(e, a, e->s_main));
         }
         EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
         EX_CUDA(cudaStreamSynchronize(e->s_main));
