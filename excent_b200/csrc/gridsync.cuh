@@ -27,8 +27,8 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, unsigned& epoch) {
     epoch += gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&b->arrived, 1u);
+        // release: what the block's threads wrote before (ordered by the block barrier) comes first
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&b->arrived) : "memory");
         int ok = 0;
         for (unsigned it = 0; it < GRID_SPIN_LIMIT; it++) {
             unsigned v;
@@ -37,7 +37,6 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, unsigned& epoch) {
             if ((it & 1023u) == 1023u && *(volatile unsigned*)&b->failed) break;
         }
         if (!ok) atomicExch(&b->failed, 1u);
-        __threadfence();
         s_ok = ok;
     }
     __syncthreads();
