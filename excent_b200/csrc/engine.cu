@@ -73,7 +73,7 @@ struct Ctrl {
     ull items;         // work items of the cached push in this pass
     int pass;          // passes that pushed so far
     int done;          // 1 once a snapshot found nothing pending (or max passes)
-    int err;           // 1: a hub queue overflowed; 3: a bounded wait for a bulk copy gave up
+    int err;           // 1: a hub queue overflowed; 3: a bounded wait for a bulk copy gave up; 4: one between blocks
     int sweep_pass;    // this pass is pushed chunk by chunk (set by k_plan)
     unsigned hcount;   // hot pending list length
     unsigned pad2;
@@ -85,7 +85,8 @@ struct Ctrl {
     ull taken;         // sum over pushed vertices of the measures taken
     SnapAcc acc[2];    // persistent solve: by pass parity
     WaveCount wave[3]; // by take phase
-    GridBar bar;
+    GridBar bar;       // barrier of k_passes, k_small and k_table, ...
+    GridBar sweep_bar; // ... and of the sweeps; in a solve each kernel clears the other's
     // what a snapshot of the host-driven loop adds up; the demand table follows the block in
     // memory, so that one memset clears and one copy fetches it all
     ull hotpend;
@@ -1001,7 +1002,8 @@ static void free_host_cache(excent_engine* e) {
     e->hcache_pinned = 0;
 }
 static const char* ctrl_error(int err) {
-    return err == 3 ? "a push kernel's wait for a bulk copy of its lists timed out"
+    return err == 4 ? "a wait between the blocks of a push timed out"
+           : err == 3 ? "a push kernel's wait for a bulk copy of its lists timed out"
                     : "device capacity check failed (hub queue overflow)";
 }
 static int ensure_hubv(excent_engine* e);
@@ -1734,38 +1736,9 @@ extern "C" int excent_engine_sync(excent_engine* e) {
     EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
     EX_CUDA(cudaStreamSynchronize(e->s_main));
     const int err = e->h_ctrl->err;
-    if (e->h_ctrl->bar.failed) EX_FAIL(EXCENT_ERR_STATE, "a wait between the blocks of a push timed out");
     if (err) scrub_queues(e);
     if (err) EX_FAIL(EXCENT_ERR_STATE, "%s", ctrl_error(err));
     return EXCENT_OK;
-}
-
-// Open an IF node with condition `h` on the stream being captured and start
-// capturing its body on `body`; close_if ends the body.
-static cudaError_t open_if(cudaStream_t st, cudaStream_t body, cudaGraphConditionalHandle h) {
-    cudaStreamCaptureStatus status;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    cudaError_t rc = cudaStreamGetCaptureInfo(st, &status, nullptr, &g, &deps, &nd);
-    if (rc != cudaSuccess) return rc;
-    if (status != cudaStreamCaptureStatusActive) return cudaErrorStreamCaptureInvalidated;
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    rc = cudaGraphAddNode(&node, g, deps, nd, &cp);
-    if (rc != cudaSuccess) return rc;
-    rc = cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies);
-    if (rc != cudaSuccess) return rc;
-    return cudaStreamBeginCaptureToGraph(body, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                         cudaStreamCaptureModeRelaxed);
-}
-static cudaError_t close_if(cudaStream_t body) {
-    cudaGraph_t g = nullptr;
-    return cudaStreamEndCapture(body, &g);
 }
 
 // One pass of the host-driven loop: snapshot and plan (read back), then the
@@ -1855,17 +1828,19 @@ static cudaError_t launch_small(excent_engine* e, SolveArgs& a, cudaStream_t st)
     return launch_grid(kernel, solve_grid(e), PT, smem, a, &e->d_ctrl->bar, st);
 }
 static cudaError_t launch_passes(excent_engine* e, SolveArgs& a, cudaStream_t st) {
-    return launch_grid(e->L == 1 ? k_passes<1> : k_passes<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
+    return launch_grid(e->L == 1 ? k_passes<1> : k_passes<4>, solve_grid(e), PT, hub_smem(e), a,
+                       a.use_cond ? nullptr : &e->d_ctrl->bar, st);
 }
 static cudaError_t launch_table(excent_engine* e, SolveArgs& a, cudaStream_t st) {
     return launch_grid(e->L == 1 ? k_table<1> : k_table<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
 }
 static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st) {
+    GridBar* bar = a.use_cond ? nullptr : &e->d_ctrl->sweep_bar;
     if (e->sweep_ok && a.order == 3) {
         SweepArgs s{a, e->sweep};
-        return launch_grid(e->L == 1 ? k_sweep_gather<1> : k_sweep_gather<4>, e->sms * G_PER_SM, GT, 0, s, &e->d_ctrl->bar, st);
+        return launch_grid(e->L == 1 ? k_sweep_gather<1> : k_sweep_gather<4>, e->sms * G_PER_SM, GT, 0, s, bar, st);
     }
-    return launch_grid(e->L == 1 ? k_sweep<1> : k_sweep<4>, solve_grid(e), PT, hub_smem(e), a, &e->d_ctrl->bar, st);
+    return launch_grid(e->L == 1 ? k_sweep<1> : k_sweep<4>, solve_grid(e), PT, hub_smem(e), a, bar, st);
 }
 
 // Split the lists for swept passes as gathers, once per loaded graph. It takes
@@ -1974,7 +1949,8 @@ static int ensure_sweep(excent_engine* e) {
     return EXCENT_OK;
 }
 
-// The solve of a sweeping engine: while { k_passes; if (a swept pass is due) k_sweep }.
+// The solve of a sweeping engine: while { k_passes; k_sweep }, a sweep leaving at once unless one is
+// due. (An IF node around it and memset nodes for the barriers cost 10 us a pass more.)
 static int build_graph(excent_engine* e, double list_frac, int max_passes) {
     if (e->gexec && e->graph_max_passes == max_passes && e->graph_list_frac == list_frac) return EXCENT_OK;
     invalidate_graph(e);
@@ -1982,7 +1958,7 @@ static int build_graph(excent_engine* e, double list_frac, int max_passes) {
     a.use_cond = 1;
     cudaGraph_t g;
     EX_CUDA(cudaGraphCreate(&g, 0));
-    cudaStream_t cs = nullptr, cb = nullptr;
+    cudaStream_t cs = nullptr;
     cudaGraphNodeParams cp = {};
     cudaGraphNode_t node;
     cudaGraph_t captured;
@@ -1993,25 +1969,16 @@ static int build_graph(excent_engine* e, double list_frac, int max_passes) {
     cp.conditional.size = 1;
     if (rc == cudaSuccess) rc = cudaGraphAddNode(&node, g, nullptr, 0, &cp);
     if (rc == cudaSuccess) rc = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
-    if (rc == cudaSuccess) rc = cudaStreamCreateWithFlags(&cb, cudaStreamNonBlocking);
+    if (rc == cudaSuccess)
+        rc = cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                           cudaStreamCaptureModeThreadLocal);
     if (rc == cudaSuccess) {
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        rc = cudaGraphConditionalHandleCreate(&a.go_sweep, body, 0, cudaGraphCondAssignDefault);
-        if (rc == cudaSuccess) rc = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-        if (rc == cudaSuccess) {
-            rc = launch_passes(e, a, cs);
-            if (rc == cudaSuccess) rc = open_if(cs, cb, a.go_sweep);
-            if (rc == cudaSuccess) {
-                rc = launch_sweep(e, a, cb);
-                const cudaError_t ci = close_if(cb);
-                if (rc == cudaSuccess) rc = ci;
-            }
-            const cudaError_t ce = cudaStreamEndCapture(cs, &captured);
-            if (rc == cudaSuccess) rc = ce;
-        }
+        rc = launch_passes(e, a, cs);
+        if (rc == cudaSuccess) rc = launch_sweep(e, a, cs);
+        const cudaError_t ce = cudaStreamEndCapture(cs, &captured);
+        if (rc == cudaSuccess) rc = ce;
     }
     if (cs) cudaStreamDestroy(cs);
-    if (cb) cudaStreamDestroy(cb);
     if (rc == cudaSuccess) rc = cudaGraphInstantiate(&e->gexec, g, 0);
     if (rc != cudaSuccess) {
         e->gexec = nullptr;
@@ -2135,8 +2102,8 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
         }
         EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
         EX_CUDA(cudaStreamSynchronize(e->s_main));
-        e->launches += 1 + 2 * e->h_ctrl->sweeps;
-        if (e->h_ctrl->bar.failed) EX_FAIL(EXCENT_ERR_STATE, "a wait between the blocks of a solve timed out");
+        // each iteration of the loop launches both kernels
+        e->launches += sweep_of(e) ? 2 * (e->h_ctrl->sweeps + 1) : 1;
     } else {
         // snapshot and plan, read the plan back (one sync per pass), then the pushes it chose
         for (int p = 0; p <= max_passes; p++) {

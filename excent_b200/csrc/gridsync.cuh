@@ -43,13 +43,15 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, unsigned& epoch) {
     return s_ok != 0;
 }
 
-// Launch `kernel` with one block of `threads` on every SM (or as many per SM
-// as `per_sm`) as a cooperative launch; `bar` is zeroed first, on the stream.
+// Launch `kernel` as a cooperative launch; `bar` is zeroed first, on the
+// stream (null: it is zero already).
 template <typename Args>
 static inline cudaError_t launch_grid(void (*kernel)(Args), int blocks, int threads, size_t smem, Args& a, GridBar* bar,
                                       cudaStream_t st) {
-    const cudaError_t rc = cudaMemsetAsync(bar, 0, sizeof(GridBar), st);
-    if (rc != cudaSuccess) return rc;
+    if (bar) {
+        const cudaError_t rc = cudaMemsetAsync(bar, 0, sizeof(GridBar), st);
+        if (rc != cudaSuccess) return rc;
+    }
     void* args[] = {&a};
     return cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)blocks), dim3((unsigned)threads), args, smem,
                                        st);

@@ -45,8 +45,8 @@ struct SolveArgs {
     unsigned seg;          // entries per segment
     HubSeg* small;         // taken lists of at most WAVE_LONG entries (wave records)
     int standalone;        // one push of the host-driven loop: its table and counts stay as they are
-    cudaGraphConditionalHandle again, go_sweep;
-    int use_cond;
+    int use_cond;          // in a loop with the sweep kernel: its condition, and the barriers cleared in turn
+    cudaGraphConditionalHandle again;
 };
 
 // Take vertex v, whose residual is rv, in a phase in which nobody adds to
@@ -107,6 +107,16 @@ __device__ __forceinline__ void block_offsets(unsigned a, unsigned b, unsigned (
     tb = __shfl_sync(FULL, ib, 31);
 }
 
+// A wait between blocks gave up: the solve ends with an error.
+__device__ __noinline__ bool gave_up(const SolveArgs& a) {
+    if (threadIdx.x == 0) {
+        atomicExch(&a.push.ctrl->err, 4);
+        a.push.ctrl->done = 1;
+        if (blockIdx.x == 0 && a.use_cond) cudaGraphSetConditional(a.again, 0u);
+    }
+    return false;
+}
+
 // Scratch of one block, and the counters it adds up over the kernel.
 template <int L> struct PassShared {
     typedef typename Lane<L>::T T;
@@ -134,12 +144,13 @@ template <int L> struct Passes {
     int phase;                 // take phases so far (ring of wave counters)
     ull pushed, hpushed, lanes, taken;
 
-    __device__ __forceinline__ Passes(const SolveArgs& a_, PassShared<L>& s_, T* hacc_)
+    __device__ __forceinline__ Passes(const SolveArgs& a_, PassShared<L>& s_, T* hacc_, GridBar* bar_)
         : a(a_), s(s_), x(reinterpret_cast<T*>(a_.push.x)), r(reinterpret_cast<T*>(a_.push.r)), hacc(hacc_),
           prefix(a_.push.wt_prefix), type(a_.push.wt_type), lane(threadIdx.x & 31), wib(threadIdx.x >> 5), epoch(0),
-          phase(0), pushed(0), hpushed(0), lanes(0), taken(0) {}
+          phase(0), pushed(0), hpushed(0), lanes(0), taken(0), bar(bar_) {}
 
-    __device__ __forceinline__ bool sync() { return grid_sync(&a.push.ctrl->bar, epoch); }
+    GridBar* bar;
+    __device__ __forceinline__ bool sync() { return grid_sync(bar, epoch) || gave_up(a); }
     __device__ __forceinline__ WaveCount& counts(int ph) const { return a.push.ctrl->wave[ph % 3]; }
 
     // Table item t: its vertex, in a chunk's list or range.
@@ -485,7 +496,7 @@ __global__ void __launch_bounds__(PT, 1) k_passes(const __grid_constant__ SolveA
     __shared__ ull s_sum[2];
     Ctrl* ctrl = a.push.ctrl;
     if (ctrl->done) return;
-    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
+    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k), &a.push.ctrl->bar);
     const int lane = P.lane, wib = P.wib, nc = a.push.nc;
     const bool first_block = blockIdx.x == 0, lead = first_block && threadIdx.x == 0;
     if (lead && a.sweep)   // what the sweep before left (otherwise the solve's reset cleared them)
@@ -549,7 +560,7 @@ __global__ void __launch_bounds__(PT, 1) k_passes(const __grid_constant__ SolveA
             ctrl->acc[(k & 1) ^ 1] = SnapAcc{};
             if (a.use_cond) {
                 cudaGraphSetConditional(a.again, stop ? 0u : 1u);
-                cudaGraphSetConditional(a.go_sweep, sweep ? 1u : 0u);
+                ctrl->sweep_bar = GridBar{};   // the sweep's, which is not running
             }
         }
         if (stop || sweep) return;   // k_sweep clears the tables of this pass
@@ -577,7 +588,7 @@ template <int L>
 __global__ void __launch_bounds__(PT, 1) k_table(const __grid_constant__ SolveArgs a) {
     typedef typename Lane<L>::T T;
     __shared__ PassShared<L> s;
-    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
+    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k), &a.push.ctrl->bar);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         for (WaveCount& w : a.push.ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }
     if (!P.sync()) return;
@@ -591,6 +602,7 @@ __global__ void __launch_bounds__(PT, 1) k_table(const __grid_constant__ SolveAr
 // After a swept pass of a device solve: every table and sum of the passes, for the next k_passes.
 __device__ __forceinline__ void clear_tables(const SolveArgs& a, int threads) {
     if (a.standalone || blockIdx.x) return;
+    if (threadIdx.x == 0) a.push.ctrl->bar = GridBar{};   // that of k_passes, which is not running
     for (int c = threadIdx.x; c < 2 * a.push.nc; c += threads) { a.snap.cnt[c] = 0; a.cnt2[c] = 0; }
     if (threadIdx.x == 0) { a.push.ctrl->acc[0] = SnapAcc{}; a.push.ctrl->acc[1] = SnapAcc{}; }
 }
@@ -602,7 +614,7 @@ __global__ void __launch_bounds__(PT, 1) k_sweep(const __grid_constant__ SolveAr
     __shared__ PassShared<L> s;
     Ctrl* ctrl = a.push.ctrl;
     if (!a.standalone && (ctrl->done || !ctrl->sweep_pass)) return;
-    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
+    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k), &ctrl->sweep_bar);
     const int nc = a.push.nc;
     clear_tables(a, PT);
     if (blockIdx.x == 0 && threadIdx.x == 0)

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
     __shared__ unsigned s_small, s_big;
     __shared__ ull s_cnt[2][PW];
     Ctrl* ctrl = a.push.ctrl;
-    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k));
+    Passes<L> P(a, s, hacc_init<T>(a.push.hub_k), &ctrl->bar);
     Rec* rec = reinterpret_cast<Rec*>(reinterpret_cast<char*>(s_dyn) + ((size_t)a.push.hub_k * sizeof(T) + 15) / 16 * 16);
     const int lane = P.lane, wib = P.wib, n = a.snap.n;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;

@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
     auto phase_end = [&]() -> bool {
         __syncthreads();
         if (threadIdx.x == 0) s_next = 0;
-        return grid_sync(&ctrl->bar, epoch);
+        return grid_sync(&ctrl->sweep_bar, epoch) || gave_up(a);
     };
     // segments [s0, s1) two at a time, `done(segment, sum)` in lane 0; returns the
     // warp's first claim past their pairs
