@@ -83,7 +83,7 @@ struct Ctrl {
     ull sweeps;        // passes that went chunk by chunk
     ull lanes;         // sum over pushed lists of entries x measures carrying a nonzero weight
     ull taken;         // sum over pushed vertices of the measures taken
-    SnapAcc acc[2];    // persistent solve: by pass parity
+    SnapAcc acc[3];    // persistent solve: by pass (parity)
     WaveCount wave[3]; // by take phase
     GridBar bar;       // barrier of k_passes, k_small and k_table, ...
     GridBar sweep_bar; // ... and of the sweeps; in a solve each kernel clears the other's

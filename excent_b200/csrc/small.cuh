@@ -9,8 +9,9 @@
 // long lists, belong to different blocks). The order is that of k_passes: the
 // snapshot, in which the high-degree lists are taken; their scatter; the takes
 // of the others; their scatter. R-MAT 16 PageRank, 49
-// passes: 4.2 ms as graph nodes, 1.46 by k_passes, 1.02 so; 2000 vertices, all three
-// measures, 42 passes: 2.6, 1.23 and 0.83 ms.
+// passes: 4.2 ms as graph nodes, 1.46 by k_passes, 0.95 so; 2000 vertices, all three
+// measures, 42 passes: 2.6, 1.23 and 0.74 ms. The pass log and the counters of what was taken
+// stay out of the chain of phases (by block 0 before its scatter and by every warp: 0.79 ms).
 #pragma once
 
 namespace excent {
@@ -62,12 +63,16 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
     __shared__ PassShared<L> s;
     __shared__ unsigned s_small, s_big;
     __shared__ ull s_cnt[2][PW];
+    __shared__ ull s_took[4][PW];   // entries, entries x measures, measures taken, entries from host memory
     Ctrl* ctrl = a.push.ctrl;
     Passes<L> P(a, s, hacc_init<T>(a.push.hub_k), &ctrl->bar);
     Rec* rec = reinterpret_cast<Rec*>(reinterpret_cast<char*>(s_dyn) + ((size_t)a.push.hub_k * sizeof(T) + 15) / 16 * 16);
     const int lane = P.lane, wib = P.wib, n = a.snap.n;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+    // the pass log is written off the critical path, by the last warp of the last block
+    const bool scribe = blockIdx.x == gridDim.x - 1 && threadIdx.x == PT - 32;
     T* r = P.r;
+    if (lane < 4) s_took[lane][wib] = 0;
     int v[V];
     unsigned deg[V];
     const int* nb[V];
@@ -91,10 +96,13 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
         }
     }
     for (int pass = 0;; pass++) {
-        SnapAcc* acc = &ctrl->acc[pass & 1];
+        SnapAcc* acc = &ctrl->acc[pass % 3];
         WaveCount* wave = &ctrl->wave[pass % 3];
         if (threadIdx.x == 0) { s_small = 0; s_big = 0; s.next = 0; }
-        if (lead) ctrl->wave[(pass + 1) % 3].big = 0;   // nobody uses it before the barrier
+        if (lead) {   // the next pass's: nobody uses them before the barrier
+            ctrl->wave[(pass + 1) % 3].big = 0;
+            ctrl->acc[(pass + 1) % 3] = SnapAcc{};
+        }
         // snapshot; the component along v1 as in snapshot_scan
         const double evc_in = a.snap.v1 ? ctrl->ev_corr : 0.0;
         const double evc = fabs(evc_in) > a.snap.ev_skip ? evc_in : 0.0;
@@ -154,6 +162,9 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
             } else if (wib < 6) {
                 const ull t = warp_sum(lane < PW ? s_cnt[wib - 4][lane] : 0ull);
                 if (lane == 0 && t) atomicAdd(wib == 4 ? &acc->pending : &acc->demand, t);
+            } else if (wib < 10) {   // what the pass before took
+                const ull t = warp_sum(lane < PW ? s_took[wib - 6][lane] : 0ull);
+                if (lane == 0 && t) atomicAdd(wib == 6 ? &ctrl->pushed : wib == 7 ? &ctrl->lanes : wib == 8 ? &ctrl->taken : &ctrl->host_pushed, t);
             }
         }
         if (!P.sync()) return;
@@ -161,19 +172,21 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
         const bool stop = pass >= a.max_passes || np == 0;
         const bool range = !((double)np < a.list_frac * n);   // (src/excent.cu:639)
         const unsigned nhub = (unsigned)min((ull)wave->big, a.push.hub_cap);
+        if (scribe && !stop && pass < a.log_cap) {
+            PassRec& R = a.log[pass];
+            R.pending = np; R.demand = acc->demand; R.hot_pending = 0; R.pushed_before = ctrl->pushed;
+            R.lanes_before = ctrl->lanes; R.taken_before = ctrl->taken;
+            for (int m = 0; m < MAXM; m++) R.rsum[m] = acc->rsum[m];
+            R.n_list = range ? 0 : 1; R.n_range = range ? 1 : 0;
+        }
         if (lead) {
-            if (!stop && pass < a.log_cap) {
-                PassRec& R = a.log[pass];
-                R.pending = np; R.demand = acc->demand; R.hot_pending = 0; R.pushed_before = ctrl->pushed;
-                R.lanes_before = ctrl->lanes; R.taken_before = ctrl->taken;
-                for (int m = 0; m < MAXM; m++) R.rsum[m] = acc->rsum[m];
-                R.n_list = range ? 0 : 1; R.n_range = range ? 1 : 0;
+            if (a.snap.v1) ctrl->ev_corr = acc->ev_dot;
+            if (stop) {
+                for (int m = 0; m < MAXM; m++) ctrl->rsum[m] = acc->rsum[m];
+                ctrl->done = 1;
+                ctrl->pass = pass;
+                a.snap.cnt[1] = acc->demand;
             }
-            for (int m = 0; m < MAXM; m++) ctrl->rsum[m] = acc->rsum[m];
-            ctrl->ev_corr = acc->ev_dot;
-            if (stop) ctrl->done = 1; else ctrl->pass = pass + 1;
-            ctrl->acc[(pass & 1) ^ 1] = SnapAcc{};
-            if (stop) a.snap.cnt[1] = acc->demand;
         }
         if (stop) {   // out of passes, perhaps: the pending list as a snapshot leaves it
 #pragma unroll
@@ -218,7 +231,21 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
                 t.p = p;
             }
         }
-        P.report();
+        {   // what this warp took in this pass, high-degree lists included
+            const unsigned lo = __reduce_add_sync(FULL, (unsigned)P.pushed & 0xffffu);
+            const unsigned hi = __reduce_add_sync(FULL, (unsigned)(P.pushed >> 16));
+            const unsigned llo = __reduce_add_sync(FULL, (unsigned)P.lanes & 0xffffu);
+            const unsigned lhi = __reduce_add_sync(FULL, (unsigned)(P.lanes >> 16));
+            const unsigned tk = __reduce_add_sync(FULL, (unsigned)P.taken);
+            const ull h = a.push.hcache ? warp_sum(P.hpushed) : 0;
+            if (lane == 0) {
+                s_took[0][wib] = lo + ((ull)hi << 16);
+                s_took[1][wib] = llo + ((ull)lhi << 16);
+                s_took[2][wib] = tk;
+                s_took[3][wib] = h;
+            }
+            P.pushed = P.lanes = P.taken = P.hpushed = 0;
+        }
         if (!P.sync()) return;
         const unsigned nsmall = s_small, nbig = s_big;
         const unsigned per_tile = min(32u, max(8u, nsmall / PW)), ntiles = (nsmall + per_tile - 1) / per_tile;
