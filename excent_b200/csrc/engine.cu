@@ -230,6 +230,11 @@ __device__ __forceinline__ int chunk_of(long long v, const int* cv0, int nc) {
 // boundary). The same atomic returns the offset at which the group's pending
 // ids are appended to the chunk's list region list[cv0[c] ..]. Integer
 // outputs equal src/excent.cu:69-98 exactly; list order is not defined.
+// Latency bounds it: the residuals of 16.8M vertices are 10 us of memory
+// traffic. With four words in flight and each pending word's degrees loaded by
+// themselves a solve's snapshot took 50 us a pass there; with eight (four, of
+// float4 residuals) and the degrees of four words at once, PageRank takes
+// 44.7 ms instead of 46.5, three measures 202.8 instead of 207.2.
 struct SnapSums {
     double rs0 = 0, rs1 = 0, rs2 = 0, evd = 0;
     unsigned hp = 0;
@@ -238,6 +243,7 @@ template <int L, typename F>
 __device__ __forceinline__ void snapshot_scan(const SnapArgs& a, ull* cnt, int group, long long g0, long long g1,
                                               double evc_in, SnapSums& sums, int lane, const F& on_pending) {
     typedef typename Lane<L>::T T;
+    constexpr int Q = L == 1 ? 8 : 4;
     T* r = reinterpret_cast<T*>(a.r);
     const long long ngroups = (a.words + group - 1) / group;
     if (g1 > ngroups) g1 = ngroups;
@@ -252,20 +258,21 @@ __device__ __forceinline__ void snapshot_scan(const SnapArgs& a, ull* cnt, int g
         const int nw = (int)min((long long)group, (long long)a.words - w0);
         uint32_t myb = 0;
         ull mydeg = 0;
-        for (int j4 = 0; j4 < nw; j4 += 4) {
-            // four words' residuals (and v1 entries) in flight before they are examined
-            T rq[4];
-            float qq[4];
+        for (int j0 = 0; j0 < nw; j0 += Q) {
+            // Q words' residuals (and v1 entries) in flight before they are examined
+            T rq[Q];
+            float qq[Q];
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const long long v = (w0 + j4 + k) * 32 + lane;
-                const bool in = j4 + k < nw && v < a.n;
+            for (int k = 0; k < Q; k++) {
+                const long long v = (w0 + j0 + k) * 32 + lane;
+                const bool in = j0 + k < nw && v < a.n;
                 if (in) rq[k] = r[v];
                 qq[k] = in && a.v1 ? a.v1[v] : 0.f;
             }
+            unsigned pm = 0;   // this lane's pending words
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int j = j4 + k;
+            for (int k = 0; k < Q; k++) {
+                const int j = j0 + k;
                 if (j >= nw) break;
                 const long long v = (w0 + j) * 32 + lane;
                 bool pend = false;
@@ -282,6 +289,7 @@ __device__ __forceinline__ void snapshot_scan(const SnapArgs& a, ull* cnt, int g
                             *rp = re;
                             if constexpr (L == 4) { if (a.ev == 0) rv.x = re; else if (a.ev == 1) rv.y = re; else rv.z = re; }
                             else rv = re;
+                            rq[k] = rv;
                         }
                         evd += (double)re * (double)q;
                     }
@@ -294,14 +302,31 @@ __device__ __forceinline__ void snapshot_scan(const SnapArgs& a, ull* cnt, int g
                     pend = pending_of(rv, a.M);
                     if (a.trace && pend) a.trace[v]++;
                     if (a.hot && pend && bit_of(a.hot, v)) { hp++; pend = false; }
-                    if (pend) {
-                        const ull deg = a.idx[v + 1] - a.idx[v];
-                        mydeg += deg;
-                        on_pending(v, rv, deg);
-                    }
+                    if (pend) pm |= 1u << k;
                 }
                 const uint32_t b = __ballot_sync(FULL, pend);
                 if (lane == j) myb = b;
+            }
+            // the pending vertices' degrees, four words' in flight
+#pragma unroll
+            for (int k0 = 0; k0 < Q; k0 += 4) {
+                if (!(pm >> k0 & 15u)) continue;
+                ull lo[4], hi[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    lo[k] = hi[k] = 0;
+                    if (pm >> (k0 + k) & 1u) {
+                        const ull* at = a.idx + (w0 + j0 + k0 + k) * 32 + lane;
+                        lo[k] = at[0];
+                        hi[k] = at[1];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (!(pm >> (k0 + k) & 1u)) continue;
+                    mydeg += hi[k] - lo[k];
+                    on_pending((w0 + j0 + k0 + k) * 32 + lane, rq[k0 + k], hi[k] - lo[k]);
+                }
             }
         }
         if (lane < nw) a.bitmap[w0 + lane] = myb;
@@ -1796,7 +1821,11 @@ static SolveArgs solve_args(excent_engine* e, double list_frac, int max_passes) 
     a.push = push_args(e, 0);
     a.cnt2 = e->d_cnt2;
     // a word per warp step while there are warps for it, up to SNAP_GROUP
-    a.snap_group = std::max(1, std::min(SNAP_GROUP, a.snap.words / (e->sms * PW)));
+    // the same number of words for every warp, in as few groups as that takes (with words / warps
+    // rounded down, half of the warps had two groups and the others none at 1M vertices: with this and
+    // the wider loads a query of 66 passes takes 3.98 ms instead of 4.21)
+    const int warps = e->sms * PW, runs = (a.snap.words + warps * SNAP_GROUP - 1) / (warps * SNAP_GROUP);
+    a.snap_group = std::max(1, (a.snap.words + warps * runs - 1) / (warps * runs));
     a.cmode = e->d_cmode;
     a.list_frac = list_frac;
     a.max_passes = max_passes;
