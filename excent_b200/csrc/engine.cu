@@ -1899,9 +1899,11 @@ static int ensure_sweep(excent_engine* e) {
     // segments at most: a list of more than PULL_LONG entries has one for each PULL_SEG entries and one more
     const size_t hub_cap = m / PULL_SEG + m / HUB_MIN + 1, mid_cap = m / PULL_LONG + 1, late_cap = list_seg_cap(m);
     const size_t words = (n + 31) / 32;
-    std::vector<size_t> parts = {m * sizeof(int), n * 4, (n + 1) * 4, n * 2, n * 4, (n + 1) * 4, words * 4, n * tb,
+    const size_t nt = n + 1, ns = std::min<ull>(n, m / (TINY_PART + 1)) + 1;   // listed vertices at most, and one more
+    std::vector<size_t> parts = {m * sizeof(int), nt * 4, nt * 4, nt * 2, nt * 4, nt * 4, words * 4, n * tb,
                                  hub_cap * sizeof(HubPart), mid_cap * sizeof(ListSeg), late_cap * sizeof(ListSeg), hub_cap * 4,
-                                 (size_t)(e->nc + 1) * 4, (nq + 1) * 4, (nq + 1) * 4, (size_t)(e->nc + 1) * 4, C_KINDS * 4};
+                                 (size_t)(e->nc + 1) * 4, (nq + 1) * 4, (nq + 1) * 4, (size_t)(e->nc + 1) * 4, C_KINDS * 4,
+                                 (nq + 1) * 4, ns * 4, ns * 4, ns * 2, ns * 4, ns * 4};
     // what only the building needs: phase and early length of every vertex, where its parts go, the sums
     const size_t first_temp = parts.size();
     for (size_t bytes : {n * sizeof(uint16_t), n * 4, n * 4, n * 4, (size_t)C_KINDS * HUB_BLOCKS * 4, sizeof(ull)})
@@ -1924,11 +1926,10 @@ static int ensure_sweep(excent_engine* e) {
     b.hubv = e->d_hubv; b.hubv_cnt = e->d_hubv_cnt;
     b.cv0 = e->d_cv0; b.per_phase = per_phase;
     b.out = (int*)(k + parts[0]);
-    b.e_v = (int*)(k + parts[1]);
-    b.e_off = (unsigned*)(k + parts[2]);
-    b.e_deg = (uint16_t*)(k + parts[3]);
-    b.l_v = (int*)(k + parts[4]);
-    b.l_off = (unsigned*)(k + parts[5]);
+    b.e_tiny = ListedParts{(int*)(k + parts[1]), (unsigned*)(k + parts[2]), (uint16_t*)(k + parts[3])};
+    b.l_tiny = ListedParts{(int*)(k + parts[4]), (unsigned*)(k + parts[5]), nullptr};
+    b.e_short = ListedParts{(int*)(k + parts[18]), (unsigned*)(k + parts[19]), (uint16_t*)(k + parts[20])};
+    b.l_short = ListedParts{(int*)(k + parts[21]), (unsigned*)(k + parts[22]), nullptr};
     b.alone = (uint32_t*)(k + parts[6]);
     void* weights = k + parts[7];
     b.e_hub = (HubPart*)(k + parts[8]);
@@ -1937,7 +1938,8 @@ static int ensure_sweep(excent_engine* e) {
     b.hub_done = (unsigned*)(k + parts[11]);
     b.hub_at = (unsigned*)(k + parts[12]);
     b.mid_at = (unsigned*)(k + parts[13]);
-    b.ev_at = (unsigned*)(k + parts[14]);
+    b.et_at = (unsigned*)(k + parts[14]);
+    b.es_at = (unsigned*)(k + parts[17]);
     int* d_q_of = (int*)(k + parts[15]);
     b.totals = (unsigned*)(k + parts[16]);
     b.q_of = d_q_of;
@@ -1968,8 +1970,8 @@ static int ensure_sweep(excent_engine* e) {
         e->launches += 4;
         if (rc == cudaSuccess) {
             invalidate_graph(e);
-            e->sweep = SweepLists{b.out, b.e_v, b.e_off, b.e_deg, b.l_v, b.l_off, b.alone, b.e_hub, b.e_mid, b.l_seg,
-                                  b.totals, b.hub_at, b.mid_at, b.ev_at, d_q_of, b.hub_done, weights};
+            e->sweep = SweepLists{b.out, b.e_tiny, b.e_short, b.l_tiny, b.l_short, b.alone, b.e_hub, b.e_mid, b.l_seg,
+                                  b.totals, b.hub_at, b.mid_at, b.et_at, b.es_at, d_q_of, b.hub_done, weights};
             e->sweep_ok = true;
         }
     }

@@ -85,14 +85,17 @@ __device__ __forceinline__ T warp_window_sums(ull b, unsigned ds, const F& f, Pu
     return sum;
 }
 
-// Each lane's sum of f over its list [b, b + ds), ds <= PULL_LONG. f.key(e)
-// loads what entry e names, f.value(key) gathers its value (0 for a default
-// key). Eight lanes walk a list, four lists at a time and four such rounds in
-// flight: on lists of 5 to 7 entries that keeps half of the lanes busy for
-// less than half the instructions of a segmented scan over the concatenated
-// lists (15 shuffles and as many additions per 32 float4 entries).
-template <typename T, int R = 4, typename O, typename F>
+// Each lane's sum of f over its list [b, b + ds), ds <= PULL_LONG (TINY: at
+// most 8). f.key(e) loads what entry e names, f.value(key) gathers its value (0
+// for a default key). Eight lanes walk a list, four lists at a time and R such
+// rounds in flight: on lists of 5 to 7 entries that keeps half of the lanes
+// busy for less than half the instructions of a segmented scan over the
+// concatenated lists (15 shuffles and as many additions per 32 float4
+// entries). A batch of 4 R lists takes a gather's latency for every eight
+// entries of its longest one, so lists of at most 8 entries go apart.
+template <typename T, bool TINY, typename O, typename F>
 __device__ __forceinline__ T warp_list_sums(O b, unsigned ds, const F& f, int lane) {
+    constexpr int R = TINY ? 8 : 4;
     T mine = T(0);
     if (!__any_sync(FULL, ds)) return mine;
     const int sub = lane >> 3, l8 = lane & 7;
@@ -112,18 +115,23 @@ __device__ __forceinline__ T warp_list_sums(O b, unsigned ds, const F& f, int la
             key[k] = typename F::Key{};
             if ((unsigned)l8 < dd[k]) key[k] = f.key(bb[k] + l8);
         }
-        most = __reduce_max_sync(FULL, most);
-        for (unsigned j = 8; j < most + 8; j += 8) {   // the next entries' keys are loaded ahead
-            typename F::Key next[R];
+        if constexpr (TINY) {
 #pragma unroll
-            for (int k = 0; k < R; k++) {
-                next[k] = typename F::Key{};
-                if (j + l8 < dd[k]) next[k] = f.key(bb[k] + j + l8);
-            }
+            for (int k = 0; k < R; k++) acc[k] = f.value(key[k]);
+        } else {
+            most = __reduce_max_sync(FULL, most);
+            for (unsigned j = 8; j < most + 8; j += 8) {   // the next entries' keys are loaded ahead
+                typename F::Key next[R];
 #pragma unroll
-            for (int k = 0; k < R; k++) {
-                acc[k] += f.value(key[k]);
-                key[k] = next[k];
+                for (int k = 0; k < R; k++) {
+                    next[k] = typename F::Key{};
+                    if (j + l8 < dd[k]) next[k] = f.key(bb[k] + j + l8);
+                }
+#pragma unroll
+                for (int k = 0; k < R; k++) {
+                    acc[k] += f.value(key[k]);
+                    key[k] = next[k];
+                }
             }
         }
 #pragma unroll

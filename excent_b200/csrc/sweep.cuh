@@ -2,25 +2,30 @@
 //
 // A swept pass pushes most of the graph, where a gather is faster than the
 // scatter (pull.cuh): on an R-MAT of 16.8M vertices and 263M entries a swept
-// pass takes 1.4 ms for one measure (scatter: 2.5) and 2.2 ms for three (3.4).
+// pass takes 1.3 ms for one measure (scatter: 2.5) and 2.1 ms for three (3.4).
 // What bounds it is one L1 lookup per entry (284 G/s for the GPU: 0.93 ms a
 // pass; the long late parts reach 85-100 % of that) and, for the many lists of
-// a few entries, chains of dependent loads in each of the phases. On a
-// symmetric graph the push of
-// vertex u is the same as every neighbour adding u's weight P[u] to its own
-// residual, once, at any time between u's take and the neighbour's next take
-// that has to see it. So each list is split, once per graph, by the order in
-// which a swept pass takes vertices: chunk by chunk, a chunk's lists longer
-// than HUB_MIN first, then its others. The early part of v's list holds the
+// a few entries, chains of dependent loads in each of the phases. (Filling the
+// ends of the phases with late segments, and keys loaded a batch ahead, gained
+// nothing.) On a symmetric graph the push of vertex u is the same as every
+// neighbour adding u's weight P[u] to its own residual, once, at any time
+// between u's take and the neighbour's next take that has to see it. So each
+// list is split, once per graph, by the order in which a swept pass takes
+// vertices: chunk by chunk, a chunk's lists longer than HUB_MIN first, then its
+// others. The early part of v's list holds the
 // neighbours taken in earlier phases than v; v gathers it and is taken in its
 // own phase. The late part holds the others; one last phase gathers it for
 // every vertex, after which the residuals are complete, as a push leaves them.
 //
 // Layout (one copy of the lists, plain ids): for the early and for the late
-// parts, those of at most PULL_LONG entries back to back in vertex order, with
-// the vertices that have them listed (more than half of an R-MAT graph's
-// vertices have no entry at all), and the longer ones, and every early part of
-// a hub vertex, apart with a segment table in vertex order.
+// parts, those of at most TINY_PART entries, then those of at most PULL_LONG,
+// each back to back in vertex order with the vertices that have them listed
+// (more than half of an R-MAT graph's vertices have no entry at all), and the
+// longer ones, and every early part of a hub vertex, apart with a segment table
+// in vertex order. Tiny parts go apart because a phase is a chain of a few
+// tiles a warp and a tile's time that of its longest list: with one class three
+// measures on 16.8M vertices took 202.6 ms a solve, with two 192, PageRank 44.8
+// and 43.0.
 #pragma once
 
 #include <type_traits>
@@ -60,14 +65,20 @@ struct HubPart {
 __device__ __forceinline__ ListSeg as_seg(const ListSeg& s) { return s; }
 __device__ __forceinline__ ListSeg as_seg(const HubPart& s) { return ListSeg{s.base, s.len_nseg & 1023u, s.row}; }
 
+// Vertices in ascending order, their parts back to back, their degrees (early parts only).
+struct ListedParts {
+    int* v;
+    unsigned* off;
+    uint16_t* deg;
+};
+
 // The split lists of one graph and the phases of its swept passes.
 struct SweepLists {
-    const int* adj;             // m entries: short early | long early | short late | long late parts
-    const int* e_v;             // vertices with entries and a short early part (it may be empty), not hubs
-    const unsigned* e_off;      // their parts
-    const uint16_t* e_deg;      // their degrees
-    const int* l_v;             // vertices with a short late part of at least one entry
-    const unsigned* l_off;
+    const int* adj;             // m entries: early parts tiny | short | long, then late parts tiny | short | long
+    ListedParts e_tiny;         // vertices with entries and a tiny early part (it may be empty), not hubs
+    ListedParts e_short;
+    ListedParts l_tiny;         // vertices with a tiny late part of at least one entry
+    ListedParts l_short;
     const uint32_t* alone;      // bitmap of the vertices without entries
     const HubPart* e_hub;       // early parts of hub vertices, in vertex order
     const ListSeg* e_mid;       // other early parts longer than PULL_LONG, one segment each, in vertex order
@@ -75,12 +86,15 @@ struct SweepLists {
     const unsigned* totals;     // [C_KINDS]: entries, segments and vertices of each kind
     const unsigned* hub_at;     // [nc + 1] first hub segment of each chunk
     const unsigned* mid_at;     // [nq + 1] first mid segment of each short phase
-    const unsigned* ev_at;      // [nq + 1] first of e_v of each short phase
+    const unsigned* et_at;      // [nq + 1] first of e_tiny of each short phase
+    const unsigned* es_at;      // [nq + 1] ... and of e_short
     const int* q_of;            // [nc + 1] first short phase of each chunk
     unsigned* hub_done;         // segments done, at the number of the vertex's first one
     void* P;                    // what each vertex pushed in this pass
 };
-enum SweepCount { C_E_SHORT, C_E_HUB_SEG, C_E_MID_SEG, C_E_LONG, C_L_SHORT, C_L_SEG, C_L_LONG, C_E_V, C_L_V, C_KINDS };
+static constexpr unsigned TINY_PART = 8;   // entries
+enum SweepCount { C_E_TINY, C_E_SHORT, C_E_HUB_SEG, C_E_MID_SEG, C_E_LONG, C_L_TINY, C_L_SHORT, C_L_SEG, C_L_LONG,
+                  C_ET_V, C_ES_V, C_LT_V, C_LS_V, C_KINDS };
 
 // ------------------------------------------------------------------ building
 
@@ -118,13 +132,11 @@ struct SweepBuild {
     ull* asym;              // 0: symmetric
     unsigned* counts;       // [C_KINDS][HUB_BLOCKS]
     unsigned* totals;
-    int *e_v, *l_v;
-    unsigned *e_off, *l_off;
-    uint16_t* e_deg;
+    ListedParts e_tiny, e_short, l_tiny, l_short;
     uint32_t* alone;
     HubPart* e_hub;
     ListSeg *e_mid, *l_seg;
-    unsigned *hub_at, *mid_at, *ev_at;
+    unsigned *hub_at, *mid_at, *et_at, *es_at;
     unsigned *e_dst, *l_dst;   // where each vertex's parts go
     unsigned* hub_done;
     int* out;
@@ -137,16 +149,21 @@ __device__ __forceinline__ void sweep_sizes(const SweepBuild& a, long long v, un
     ec = a.early[v];
     lc = deg - ec;
     hub = deg > HUB_MIN;
-    const bool es = !hub && ec <= PULL_LONG, ls = lc <= PULL_LONG;
+    const bool et = !hub && ec <= TINY_PART, es = !hub && !et && ec <= PULL_LONG;
+    const bool lt = lc <= TINY_PART, ls = !lt && lc <= PULL_LONG;
+    k[C_E_TINY] = et ? ec : 0u;
     k[C_E_SHORT] = es ? ec : 0u;
     k[C_E_HUB_SEG] = hub ? max(1u, (ec + PULL_SEG - 1) / PULL_SEG) : 0u;
-    k[C_E_MID_SEG] = !hub && !es ? 1u : 0u;
-    k[C_E_LONG] = es ? 0u : ec;
+    k[C_E_MID_SEG] = !hub && ec > PULL_LONG ? 1u : 0u;
+    k[C_E_LONG] = et || es ? 0u : ec;
+    k[C_L_TINY] = lt ? lc : 0u;
     k[C_L_SHORT] = ls ? lc : 0u;
-    k[C_L_SEG] = ls ? 0u : (lc + PULL_SEG - 1) / PULL_SEG;
-    k[C_L_LONG] = ls ? 0u : lc;
-    k[C_E_V] = es && deg ? 1u : 0u;
-    k[C_L_V] = ls && lc ? 1u : 0u;
+    k[C_L_SEG] = lt || ls ? 0u : (lc + PULL_SEG - 1) / PULL_SEG;
+    k[C_L_LONG] = lt || ls ? 0u : lc;
+    k[C_ET_V] = et && deg ? 1u : 0u;
+    k[C_ES_V] = es ? 1u : 0u;
+    k[C_LT_V] = lt && lc ? 1u : 0u;
+    k[C_LS_V] = ls ? 1u : 0u;
 }
 
 // Each block sums a contiguous range of vertices (write 0), then, from the
@@ -158,9 +175,12 @@ __global__ void __launch_bounds__(BLOCK) k_sweep_layout(SweepBuild a, int write)
     const long long v0 = blockIdx.x * per, v1 = min(v0 + per, (long long)a.n);
     unsigned at[C_KINDS];
     for (int q = 0; q < C_KINDS; q++) at[q] = write ? a.counts[q * HUB_BLOCKS + blockIdx.x] : 0u;
-    const unsigned base_el = write ? a.totals[C_E_SHORT] : 0u;
-    const unsigned base_ls = base_el + (write ? a.totals[C_E_LONG] : 0u);
-    const unsigned base_ll = base_ls + (write ? a.totals[C_L_SHORT] : 0u);
+    // where each kind of part begins in the entries
+    const unsigned at_es = write ? a.totals[C_E_TINY] : 0u;
+    const unsigned at_el = at_es + (write ? a.totals[C_E_SHORT] : 0u);
+    const unsigned at_lt = at_el + (write ? a.totals[C_E_LONG] : 0u);
+    const unsigned at_ls = at_lt + (write ? a.totals[C_L_TINY] : 0u);
+    const unsigned at_ll = at_ls + (write ? a.totals[C_L_SHORT] : 0u);
     for (long long b0 = v0; b0 < v1; b0 += BLOCK) {
         const long long v = b0 + threadIdx.x;
         unsigned k[C_KINDS], ec = 0, lc = 0, ex[C_KINDS];
@@ -185,16 +205,26 @@ __global__ void __launch_bounds__(BLOCK) k_sweep_layout(SweepBuild a, int write)
             at[q] += all;
         }
         if (write && v < v1) {
-            if (k[C_E_V]) {
-                a.e_v[ex[C_E_V]] = (int)v;
-                a.e_off[ex[C_E_V]] = ex[C_E_SHORT];
-                a.e_deg[ex[C_E_V]] = (uint16_t)(ec + lc);
+            unsigned ed = at_el + ex[C_E_LONG], ld = at_ll + ex[C_L_LONG];
+            if (k[C_ET_V]) {
+                const unsigned j = ex[C_ET_V];
+                ed = ex[C_E_TINY];
+                a.e_tiny.v[j] = (int)v; a.e_tiny.off[j] = ed; a.e_tiny.deg[j] = (uint16_t)(ec + lc);
             }
-            if (k[C_L_V]) { a.l_v[ex[C_L_V]] = (int)v; a.l_off[ex[C_L_V]] = base_ls + ex[C_L_SHORT]; }
+            if (k[C_ES_V]) {
+                const unsigned j = ex[C_ES_V];
+                ed = at_es + ex[C_E_SHORT];
+                a.e_short.v[j] = (int)v; a.e_short.off[j] = ed; a.e_short.deg[j] = (uint16_t)(ec + lc);
+            }
+            if (k[C_LT_V]) {
+                ld = at_lt + ex[C_L_TINY];
+                a.l_tiny.v[ex[C_LT_V]] = (int)v; a.l_tiny.off[ex[C_LT_V]] = ld;
+            }
+            if (k[C_LS_V]) {
+                ld = at_ls + ex[C_L_SHORT];
+                a.l_short.v[ex[C_LS_V]] = (int)v; a.l_short.off[ex[C_LS_V]] = ld;
+            }
             if (ec + lc == 0) atomicOr(&a.alone[v >> 5], 1u << (v & 31));
-            const bool es = k[C_E_MID_SEG] == 0 && !hub, ls = k[C_L_SEG] == 0;
-            const unsigned ed = es ? ex[C_E_SHORT] : base_el + ex[C_E_LONG];
-            const unsigned ld = ls ? base_ls + ex[C_L_SHORT] : base_ll + ex[C_L_LONG];
             a.e_dst[v] = ed;
             a.l_dst[v] = ld;
             if (hub) a.hub_done[ex[C_E_HUB_SEG]] = 0;
@@ -210,14 +240,18 @@ __global__ void __launch_bounds__(BLOCK) k_sweep_layout(SweepBuild a, int write)
             if (in_chunk == 0) a.hub_at[c] = ex[C_E_HUB_SEG];
             if (in_chunk % a.per_phase == 0) {
                 a.mid_at[a.q_of[c] + in_chunk / a.per_phase] = ex[C_E_MID_SEG];
-                a.ev_at[a.q_of[c] + in_chunk / a.per_phase] = ex[C_E_V];
+                a.et_at[a.q_of[c] + in_chunk / a.per_phase] = ex[C_ET_V];
+                a.es_at[a.q_of[c] + in_chunk / a.per_phase] = ex[C_ES_V];
             }
             if (v == a.n - 1) {
                 a.hub_at[a.nc] = a.totals[C_E_HUB_SEG];
                 a.mid_at[a.q_of[a.nc]] = a.totals[C_E_MID_SEG];
-                a.ev_at[a.q_of[a.nc]] = a.totals[C_E_V];
-                a.e_off[a.totals[C_E_V]] = base_el;
-                a.l_off[a.totals[C_L_V]] = base_ll;
+                a.et_at[a.q_of[a.nc]] = a.totals[C_ET_V];
+                a.es_at[a.q_of[a.nc]] = a.totals[C_ES_V];
+                a.e_tiny.off[a.totals[C_ET_V]] = at_es;
+                a.e_short.off[a.totals[C_ES_V]] = at_el;
+                a.l_tiny.off[a.totals[C_LT_V]] = at_ls;
+                a.l_short.off[a.totals[C_LS_V]] = at_ll;
             }
         }
         __syncthreads();
@@ -502,26 +536,32 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
         return i;
     };
     // tiles of 32 of the listed vertices [t0, t1), the warp's first claim being `i`, `before` claims taken by
-    // segments; done(number in the list, vertex, sum). The next tile's records are loaded ahead.
-    auto tiles = [&](ull i, ull before, unsigned t0, unsigned t1, const int* vs, const unsigned* off, auto&& done) {
+    // segments and other tiles; done(number in the list, vertex, sum); returns the warp's first claim past
+    // them. The next tile's records are loaded ahead.
+    auto tiles = [&](auto tiny, ull i, ull& before, unsigned t0, unsigned t1, const ListedParts& l, auto&& done) -> ull {
         const ull ntiles = ((ull)(t1 - t0) + 31) / 32;
         int v = -1, nv = -1;
         unsigned b = 0, e = 0, nb = 0, ne = 0;
         auto load = [&](ull t, int& lv, unsigned& lb, unsigned& le) {
             const ull j = t0 + t * 32 + lane;
             lv = -1; lb = 0; le = 0;
-            if (t < ntiles && j < t1) { lv = vs[j]; lb = off[j]; le = off[j + 1]; }
+            if (t < ntiles && j < t1) { lv = l.v[j]; lb = l.off[j]; le = l.off[j + 1]; }
         };
         ull t = i - before;
         load(t, v, b, e);
         while (t < ntiles) {
             const ull nt = claim() - before;
             load(nt, nv, nb, ne);
-            const S sum = warp_list_sums<S>(b, e - b, f, lane);
+            const S sum = warp_list_sums<S, decltype(tiny)::value>(b, e - b, f, lane);
             if (v >= 0) done((unsigned)(t0 + t * 32 + lane), v, sum);
             t = nt; v = nv; b = nb; e = ne;
         }
+        t += before;
+        before += ntiles;
+        return t;
     };
+    constexpr std::true_type TINY{};
+    constexpr std::false_type SHORT{};
     for (int c = 0; c < nc; c++) {
         const uint8_t ty = a.push.wt_type[c];
         auto allowed = [&](int v) { return ty == WT_RANGE || (ty == WT_LIST && bit_of(a.snap.bitmap, v)); };
@@ -548,25 +588,30 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
         }
         for (int q = g.q_of[c]; q < g.q_of[c + 1]; q++) {
             const unsigned m0 = g.mid_at[q], m1 = g.mid_at[q + 1];
-            const ull i = segments(g.e_mid, m0, m1, [&](const ListSeg& sg, const S& sum) {
+            ull i = segments(g.e_mid, m0, m1, [&](const ListSeg& sg, const S& sum) {
                 const int v = (int)sg.row;
                 take_here<L>(x, r, P, v, add_sum(r[v], sum), idx[v + 1] - idx[v], allowed(v), nonzero(sum), a.push.M,
                              pushed, lanes, taken);
             });
-            const unsigned t0 = g.ev_at[q], t1 = g.ev_at[q + 1];
-            tiles(i, (m1 - m0 + 1) / 2, t0, t1, g.e_v, g.e_off, [&](unsigned j, int v, const S& sum) {
-                take_here<L>(x, r, P, v, add_sum(r[v], sum), g.e_deg[j], allowed(v), nonzero(sum), a.push.M, pushed, lanes,
-                             taken);
-            });
+            ull before = (m1 - m0 + 1) / 2;
+            auto listed = [&](const ListedParts& l) {
+                return [&](unsigned j, int v, const S& sum) {
+                    take_here<L>(x, r, P, v, add_sum(r[v], sum), l.deg[j], allowed(v), nonzero(sum), a.push.M, pushed, lanes,
+                                 taken);
+                };
+            };
+            i = tiles(SHORT, i, before, g.es_at[q], g.es_at[q + 1], g.e_short, listed(g.e_short));
+            tiles(TINY, i, before, g.et_at[q], g.et_at[q + 1], g.e_tiny, listed(g.e_tiny));
             if (!phase_end()) return;
         }
     }
     // the late parts of every list
     const unsigned nl = g.totals[C_L_SEG];
-    const ull i = segments(g.l_seg, 0, nl, [&](const ListSeg& sg, const S& sum) { red_sum(r, sg.row, sum); });
-    tiles(i, (nl + 1) / 2, 0, g.totals[C_L_V], g.l_v, g.l_off, [&](unsigned, int v, const S& sum) {
-        if (nonzero(sum)) r[v] = add_sum(r[v], sum);
-    });
+    ull i = segments(g.l_seg, 0, nl, [&](const ListSeg& sg, const S& sum) { red_sum(r, sg.row, sum); });
+    ull before = (nl + 1) / 2;
+    auto rest = [&](unsigned, int v, const S& sum) { if (nonzero(sum)) r[v] = add_sum(r[v], sum); };
+    i = tiles(SHORT, i, before, 0, g.totals[C_LS_V], g.l_short, rest);
+    tiles(TINY, i, before, 0, g.totals[C_LT_V], g.l_tiny, rest);
     // a vertex without entries is pending until it is taken, and nobody adds to it
     for (long long w = blockIdx.x * (long long)GT + threadIdx.x; w < a.snap.words; w += (long long)gridDim.x * GT) {
         uint32_t bits = a.snap.bitmap[w] & g.alone[w];

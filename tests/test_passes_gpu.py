@@ -130,3 +130,45 @@ def test_swept_passes_gather_only_on_symmetric_graphs(n, kind):
         got.append(eng.read(0).astype(np.float64))
         eng.close()
     assert np.abs(got[0] - got[1]).sum() <= 2 * n * EPS / 0.15 + 1e-5 * got[1].sum()
+
+
+@pytest.mark.parametrize("measure", ["pr", "all"])
+@pytest.mark.parametrize("passes", [1, 2])
+def test_swept_pass_of_every_part_length(passes, measure):
+    """The parts of a split list (neighbours taken before the vertex, and the others) at the edges of
+    their classes, both ways: the passes step by step in FP64, chunk by chunk, lists longer than 256
+    entries first; a chunk takes what is pending by then, unless the pass began with less than
+    list_frac of it pending, which are then the ones taken. FP32 sums of up to some 600 terms."""
+    n = 4000
+    rng = np.random.default_rng(11)
+    src, dst = [], []
+    for i, k in enumerate([1, 7, 8, 9, 31, 32, 33, 64, 257, 600]):
+        for v, lo in ((n - 1 - i, 0), (i, n // 2)):   # neighbours in the first quarter, or in the third
+            src.append(np.full(k, v))
+            dst.append(lo + 100 + rng.choice(n // 4, k, replace=False))
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    keys = np.unique(np.concatenate([src * n + dst, dst * n + src]))
+    src, dst = keys // n, keys % n
+    idx = np.zeros(n + 1, dtype=np.uint64)
+    np.cumsum(np.bincount(src, minlength=n), out=idx[1:])
+    adj = dst.astype(np.int32)
+    deg = np.diff(idx.astype(np.int64))
+    eng = engine(n, idx, adj, measure, len(adj) // 8 + 1, alpha=0.01, lam=25.0)
+    assert eng.nc > 4
+    eng.set_chunk_sweep(True)
+    eng.set_sweep_demand(0.01)
+    assert eng.solve(max_passes=passes, list_frac=0.5).passes == passes
+    chunk = np.searchsorted(np.asarray(eng.chunk_v0)[:eng.nc], np.arange(n), side="right") - 1
+    r, x = np.full(n, float(np.float32(1) - np.float32(0.85))), np.zeros(n)
+    for _ in range(passes):
+        first = np.abs(r) > EPS
+        few = np.bincount(chunk, first, eng.nc) < 0.5 * np.bincount(chunk, minlength=eng.nc)
+        for c in range(eng.nc):
+            for long in (True, False):
+                d = np.where((chunk == c) & ((deg > 256) == long) & (np.abs(r) > EPS) & (first | ~few[chunk]), r, 0.0)
+                x += d
+                r -= d
+                np.add.at(r, adj, (0.85 * d / np.maximum(deg, 1))[src])
+    assert np.allclose(eng.read(0), x, rtol=1e-5, atol=1e-6)
+    assert np.allclose(eng.read(0, residual=True), r, rtol=1e-5, atol=1e-6)
+    eng.close()
