@@ -75,7 +75,7 @@ def parse():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--errors", default="on", choices=["on", "off"],
                     help="error against the FP64 oracle solution, like-for-like run and the reference engine's error")
-    ap.add_argument("--no-graph", action="store_true", help="host-driven pass loop instead of the CUDA graph")
+    ap.add_argument("--no-graph", action="store_true", help="host-driven pass loop instead of the device's")
     ap.add_argument("--ev-project", default="on", choices=["on", "off"],
                     help="FP64 eigenvector normalisation step (remove the principal-eigenvector component of the "
                          "eigenvector residual each pass); the `all` run does not reach eps 1e-6 at scale 24 without it")
@@ -461,7 +461,7 @@ def run_ours(a, world, rank, local, dist):
         "e2e": {"value": round(e_pushed / te / 1e9, 4), "unit": "GTEPS", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": round(te / a.steps * 1e3, 3),
                 "wall_ms_per_step": round(te_wall / a.steps * 1e3, 3)},
-        "roofline": {"bound": "hbm", "kernel": "k_push + k_segments (one logical push: the takes, the short lists, then the queued long-list segments)",
+        "roofline": {"bound": "hbm", "kernel": "k_push + k_segments of a profiled solve by the host-driven loop (one logical push: the takes, the short lists, then the queued long-list segments); the timed solves run k_passes and k_sweep_gather, inside a graph whose kernels cannot be timed one by one",
                      "achieved": round(achieved, 1), "peak": peak, "peak_source": peak_kind, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": traffic,
                      "traffic_note": traffic_note,

@@ -54,9 +54,6 @@ __device__ __forceinline__ double shfl_up(double v, int o) { return __shfl_up_sy
 __device__ __forceinline__ double shfl(double v, int src) { return __shfl_sync(FULL, v, src); }
 __device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(FULL, v, o); }
 __device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(FULL, v, o); }
-template <typename T> __device__ __forceinline__ const T* shfl_ptr(const T* p, int src) {
-    return (const T*)__shfl_sync(FULL, (unsigned long long)p, src);
-}
 
 template <typename T> __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

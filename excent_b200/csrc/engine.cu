@@ -1,7 +1,8 @@
 // engine.cu -- the device engine of libexcent_b200: per-vertex state in HBM,
 // the demand-snapshot kernel, the on-device fetch plan for cached chunks, the
 // degree-dispatched push kernels, the hot (degree) cache kernels, staging
-// slots, and the C entry points of include/excent_b200.h that drive them.
+// slots, and the C entry points of include/excent_b200.h that drive them. The
+// kernels of the device solve are in passes.cuh, small.cuh and sweep.cuh.
 //
 // Reference seams replaced (SPADE-IITJ/ExCent, paths relative to the project):
 //   k_init                         src/excent.cu:41-47
@@ -74,7 +75,7 @@ struct Ctrl {
     int pass;          // passes that pushed so far
     int done;          // 1 once a snapshot found nothing pending (or max passes)
     int err;           // 1: a hub queue overflowed; 3: a bounded wait for a bulk copy gave up; 4: one between blocks
-    int sweep_pass;    // this pass is pushed chunk by chunk (set by k_plan)
+    int sweep_pass;    // this pass is pushed chunk by chunk (set by k_plan or k_passes)
     unsigned hcount;   // hot pending list length
     unsigned pad2;
     double ev_dot;     // FP64 (r_ev . v1) accumulated by the snapshot

@@ -177,8 +177,10 @@ int excent_engine_sync(excent_engine* e);
 
 /* Device solve of a fully cached graph (every chunk resident and loaded):
  * init, then passes of snapshot -> on-device fetch plan -> push until no
- * vertex is pending or max_passes, with no host round trip per pass. With
- * use_graph the pass is one CUDA graph with a conditional while node.
+ * vertex is pending or max_passes. With use_graph there is no host round trip
+ * per pass: all passes are one cooperative launch, or, where passes are swept
+ * chunk by chunk, one CUDA graph with a conditional while node; without it the
+ * host reads each pass's plan back and launches its pushes.
  * Per-pass log and totals are kept for excent_engine_stats. */
 int excent_engine_solve(excent_engine* e, double list_frac, int max_passes, int use_graph);
 
@@ -454,8 +456,8 @@ int excent_batch_destroy(excent_batch* b);
  * absolute threshold. Lanes >= nq stay idle. */
 int excent_batch_seed(excent_batch* b, int nq, const int* lane_off, const int32_t* vids, const float* vals,
                       const float* eps);
-/* Passes until no lane of any vertex is pending (or max_passes); with
- * use_graph all passes run as one CUDA graph with a conditional while node. */
+/* Passes until no lane of any vertex is pending (or max_passes), in one
+ * cooperative launch (use_graph makes no difference). */
 int excent_batch_solve(excent_batch* b, int max_passes, int use_graph);
 /* Passes, pushed vertices, pushed adjacency entries, 16-byte lane-group
  * reductions issued, touched rows examined and segments of lists longer than
