@@ -2,7 +2,7 @@
 //
 // A swept pass pushes most of the graph, where a gather is faster than the
 // scatter (pull.cuh): on an R-MAT of 16.8M vertices and 263M entries a swept
-// pass takes 1.3 ms for one measure (scatter: 2.5) and 2.1 ms for three (3.4).
+// pass takes 1.3 ms for one measure (scatter: 2.5) and 2.0 ms for three (3.4).
 // What bounds it is one L1 lookup per entry (284 G/s for the GPU: 0.93 ms a
 // pass; the long late parts reach 85-100 % of that) and, for the many lists of
 // a few entries, chains of dependent loads in each of the phases. (Filling the
@@ -24,8 +24,9 @@
 // longer ones, and every early part of a hub vertex, apart with a segment table
 // in vertex order. Tiny parts go apart because a phase is a chain of a few
 // tiles a warp and a tile's time that of its longest list: with one class three
-// measures on 16.8M vertices took 202.6 ms a solve, with two 192, PageRank 44.8
-// and 43.0.
+// measures on 16.8M vertices took 202.6 ms a solve, with two 191.2, PageRank
+// 44.8 and 43.2. For the same reason the takes of a warp's two segments run side
+// by side and a tile's residuals are loaded before its sums: 186.3 and 41.9 ms.
 #pragma once
 
 #include <type_traits>
@@ -511,8 +512,8 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
         if (threadIdx.x == 0) s_next = 0;
         return grid_sync(&ctrl->sweep_bar, epoch) || gave_up(a);
     };
-    // segments [s0, s1) two at a time, `done(segment, sum)` in lane 0; returns the
-    // warp's first claim past their pairs
+    // segments [s0, s1) two at a time, `done(segment, sum)` side by side in lanes 0 and 1 (a take is a
+    // chain of some seven accesses); returns the warp's first claim past their pairs
     auto segments = [&](const auto* seg, unsigned s0, unsigned s1, auto&& done) -> ull {
         typedef typename std::decay<decltype(*seg)>::type R;
         const ull npairs = (s1 - s0 + 1) / 2;
@@ -527,10 +528,8 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
             if (s0 + 2 * next + 1 < s1) n1 = seg[s0 + 2 * next + 1];
             S a0, a1;
             warp_segment_sums<S>(as_seg(g0), as_seg(g1), f, lane, a0, a1);
-            if (lane == 0) {
-                done(g0, a0);
-                if (s0 + 2 * i + 1 < s1) done(g1, a1);
-            }
+            const S b1 = shfl(a1, 0);
+            if (lane == 0 || (lane == 1 && s0 + 2 * i + 1 < s1)) done(lane ? g1 : g0, lane ? b1 : a0);
             i = next; g0 = n0; g1 = n1;
         }
         return i;
@@ -552,8 +551,10 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
         while (t < ntiles) {
             const ull nt = claim() - before;
             load(nt, nv, nb, ne);
+            T rv{};
+            if (v >= 0) rv = r[v];   // (nobody else adds to it in this phase)
             const S sum = warp_list_sums<S, decltype(tiny)::value>(b, e - b, f, lane);
-            if (v >= 0) done((unsigned)(t0 + t * 32 + lane), v, sum);
+            if (v >= 0) done((unsigned)(t0 + t * 32 + lane), v, rv, sum);
             t = nt; v = nv; b = nb; e = ne;
         }
         t += before;
@@ -595,8 +596,8 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
             });
             ull before = (m1 - m0 + 1) / 2;
             auto listed = [&](const ListedParts& l) {
-                return [&](unsigned j, int v, const S& sum) {
-                    take_here<L>(x, r, P, v, add_sum(r[v], sum), l.deg[j], allowed(v), nonzero(sum), a.push.M, pushed, lanes,
+                return [&](unsigned j, int v, const T& rv, const S& sum) {
+                    take_here<L>(x, r, P, v, add_sum(rv, sum), l.deg[j], allowed(v), nonzero(sum), a.push.M, pushed, lanes,
                                  taken);
                 };
             };
@@ -609,7 +610,7 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
     const unsigned nl = g.totals[C_L_SEG];
     ull i = segments(g.l_seg, 0, nl, [&](const ListSeg& sg, const S& sum) { red_sum(r, sg.row, sum); });
     ull before = (nl + 1) / 2;
-    auto rest = [&](unsigned, int v, const S& sum) { if (nonzero(sum)) r[v] = add_sum(r[v], sum); };
+    auto rest = [&](unsigned, int v, const T& rv, const S& sum) { if (nonzero(sum)) r[v] = add_sum(rv, sum); };
     i = tiles(SHORT, i, before, 0, g.totals[C_LS_V], g.l_short, rest);
     tiles(TINY, i, before, 0, g.totals[C_LT_V], g.l_tiny, rest);
     // a vertex without entries is pending until it is taken, and nobody adds to it
