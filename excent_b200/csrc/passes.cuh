@@ -335,49 +335,68 @@ template <int L> struct Passes {
         WaveCount& w = counts(phase);
         if (blockIdx.x == 0 && threadIdx.x == 0) { WaveCount& n = counts(phase + 1); n.small = 0; n.big = 0; n.claim = 0; }
         const long long ntiles = (items + 31) / 32, nwarps = (long long)gridDim.x * PW;
-        const long long per_claim =
-            a.push.claim_tiles > 0 ? a.push.claim_tiles : max(1ll, min((long long)TILE_BATCH, ntiles / (4 * nwarps)));
-        for (;;) {
-            unsigned c = 0;
-            if (lane == 0) c = atomicAdd(&w.claim, 1u);
-            const long long t0 = (long long)__shfl_sync(FULL, c, 0) * per_claim;
-            if (t0 >= ntiles) break;
-            const long long t1 = min(t0 + per_claim, ntiles);
-            for (long long tile = t0; tile < t1; tile++) {
-                const long long t = tile * 32 + lane;
-                T p{};
-                const int* nb = nullptr;
-                ull b = 0, deg = 0;
-                if (t < items) {
-                    const int v = item_vertex(first + t, chunk);
-                    b = a.push.idx[v];
-                    deg = a.push.idx[v + 1] - b;
-                    if (!(which == LISTS_SHORT && deg > HUB_MIN)) p = take(x, r, v, deg, a.push.M);
-                }
-                const bool act = nonzero(p) && deg > 0;
-                if (act) { count(p, deg, b); nb = list_at(a.push, b); }
-                const unsigned nseg = act && deg > HUB_MIN ? (unsigned)((deg + a.seg - 1) / a.seg) : 0u;
-                const unsigned incl = warp_incl_scan(nseg, lane);
-                const unsigned tot = __shfl_sync(FULL, incl, 31);
-                if (tot) {
-                    ull at = 0;
-                    if (lane == 0) at = atomicAdd(&w.big, tot);
-                    at = __shfl_sync(FULL, at, 0) + (incl - nseg);
-                    if (at + nseg <= a.push.hub_cap) {
-                        HubSeg h;
-                        h.pad = 0;
-                        if constexpr (L == 1) h.p = make_float4(p, 0.f, 0.f, 0.f); else h.p = p;
-                        for (unsigned k = 0; k < nseg; k++) {
-                            h.nb = nb + (ull)k * a.seg;
-                            h.len = (unsigned)min((ull)a.seg, deg - (ull)k * a.seg);
-                            a.push.hubq[at + k] = h;
-                        }
-                    } else if (nseg) {
-                        atomicExch(&a.push.ctrl->err, 1);
-                    }
-                }
-                scatter_tile(nb, act && !nseg ? (unsigned)deg : 0u, p);
+        // as many tiles are in flight as the wave has warps: when it has twice as many as run here, each
+        // takes its next tile before it scatters the one before (without that PageRank with host lists, 1M vertices, moved 4.2 times as far
+        // from where a launch of all those warps takes it as that moves between runs)
+        const unsigned ahead = a.wave >= 64 * nwarps ? 2 : 1;
+        const long long per_claim = a.push.claim_tiles > 0
+            ? a.push.claim_tiles : max(1ll, min((long long)TILE_BATCH, ntiles / (4 * nwarps * ahead)));
+        auto take_tile = [&](long long tile, const int*& nb, unsigned& ds, T& p) {
+            const long long t = tile * 32 + lane;
+            p = T{};
+            nb = nullptr;
+            ull b = 0, deg = 0;
+            if (tile < ntiles && t < items) {
+                const int v = item_vertex(first + t, chunk);
+                b = a.push.idx[v];
+                deg = a.push.idx[v + 1] - b;
+                if (!(which == LISTS_SHORT && deg > HUB_MIN)) p = take(x, r, v, deg, a.push.M);
             }
+            const bool act = nonzero(p) && deg > 0;
+            if (act) { count(p, deg, b); nb = list_at(a.push, b); }
+            const unsigned nseg = act && deg > HUB_MIN ? (unsigned)((deg + a.seg - 1) / a.seg) : 0u;
+            const unsigned incl = warp_incl_scan(nseg, lane);
+            const unsigned tot = __shfl_sync(FULL, incl, 31);
+            if (tot) {
+                ull at = 0;
+                if (lane == 0) at = atomicAdd(&w.big, tot);
+                at = __shfl_sync(FULL, at, 0) + (incl - nseg);
+                if (at + nseg <= a.push.hub_cap) {
+                    HubSeg h;
+                    h.pad = 0;
+                    if constexpr (L == 1) h.p = make_float4(p, 0.f, 0.f, 0.f); else h.p = p;
+                    for (unsigned k = 0; k < nseg; k++) {
+                        h.nb = nb + (ull)k * a.seg;
+                        h.len = (unsigned)min((ull)a.seg, deg - (ull)k * a.seg);
+                        a.push.hubq[at + k] = h;
+                    }
+                } else if (nseg) {
+                    atomicExch(&a.push.ctrl->err, 1);
+                }
+            }
+            ds = act && !nseg ? (unsigned)deg : 0u;
+        };
+        long long tile = 0, end = 0;
+        T p0{};
+        const int* nb0 = nullptr;
+        unsigned ds0 = 0;
+        for (;;) {
+            if (tile == end) {
+                unsigned c = 0;
+                if (lane == 0) c = atomicAdd(&w.claim, 1u);
+                tile = min((long long)__shfl_sync(FULL, c, 0) * per_claim, ntiles);
+                end = min(tile + per_claim, ntiles);
+            }
+            const bool more = tile < ntiles;
+            T p1;
+            const int* nb1;
+            unsigned ds1;
+            take_tile(tile, nb1, ds1, p1);
+            if (ahead == 2) scatter_tile(nb0, ds0, p0);   // the tile before
+            else scatter_tile(nb1, ds1, p1);
+            if (!more) break;
+            p0 = p1; nb0 = nb1; ds0 = ds1;
+            tile++;
         }
         flush();
         if (threadIdx.x == 0) s.next = 0;
