@@ -2109,6 +2109,12 @@ static int ensure_hubv(excent_engine* e) {
     return EXCENT_OK;
 }
 
+// Without a chunk sweep a pass is one phase, and above some 2^25 entries its scatter outlasts what a
+// launch costs: k_push and k_segments, three blocks to an SM, then beat k_passes, one block to an SM,
+// in spite of a host round trip a pass (PageRank, 65M entries: 16.3 against 18.8 ms, 14.8 by launches in a
+// graph; 263M: 47.1, 57.1 and 45.3; 16M entries: 5.4 by k_passes and 6.9 in a graph).
+static constexpr ull ONE_LAUNCH_MAX = 1ull << 25;
+
 static int solve_impl(excent_engine* e, double list_frac, int max_passes, int use_graph, bool init) {
     EX_CHECK_ARG(e, "null engine");
     EX_CHECK_ARG(max_passes >= 0 && max_passes < e->log_cap, "max_passes must be < %d", e->log_cap);
@@ -2123,7 +2129,7 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
     if (init) EX_TRY(init_state(e));
     else EX_TRY(reset_counters(e));
     if (order_of(e)) EX_TRY(ensure_hubv(e));
-    if (use_graph) {
+    if (use_graph && (sweep_of(e) || e->m < ONE_LAUNCH_MAX)) {
         if (sweep_of(e)) {
             EX_TRY(ensure_sweep(e));
             EX_TRY(build_graph(e, list_frac, max_passes));
@@ -2139,7 +2145,7 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
     } else {
         // snapshot and plan, read the plan back (one sync per pass), then the pushes it chose
         for (int p = 0; p <= max_passes; p++) {
-            cudaEvent_t* ev = e->prof ? e->ev : nullptr;
+            cudaEvent_t* ev = e->prof && !use_graph ? e->ev : nullptr;
             enqueue_plan(e, list_frac, max_passes, e->s_main, ev);
             EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
             EX_CUDA(cudaStreamSynchronize(e->s_main));
