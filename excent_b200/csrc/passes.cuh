@@ -582,6 +582,8 @@ __global__ void __launch_bounds__(PT, 1) k_passes(const __grid_constant__ SolveA
                 ctrl->sweep_bar = GridBar{};   // the sweep's, which is not running
             }
         }
+        if (stop && first_block && cnt != a.snap.cnt)   // the lengths of the pending lists, where they are read from
+            for (int c = threadIdx.x; c < 2 * nc; c += PT) a.snap.cnt[c] = cnt[c];
         if (stop || sweep) return;   // k_sweep clears the tables of this pass
         if (first_block) {           // the next snapshot's table: nobody uses it before the next barrier
             ull* other = k & 1 ? a.snap.cnt : a.cnt2;
