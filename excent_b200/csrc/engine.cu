@@ -963,7 +963,8 @@ struct excent_engine {
     HubSeg* d_small = nullptr;     // and the short lists taken together
     int wave = 0;                  // items its passes take together
     SweepLists sweep{};            // swept passes as gathers: the split lists
-    void* d_sweep = nullptr;       // (one allocation)
+    void* d_sweep = nullptr;       // (one allocation ...
+    size_t sweep_bytes = 0;        // ... of this many bytes)
     bool sweep_stale = true;       // not tried for the loaded lists
     bool sweep_ok = false;
     bool hubv_stale = true;
@@ -1033,7 +1034,8 @@ static const char* ctrl_error(int err) {
                     : "device capacity check failed (hub queue overflow)";
 }
 static int ensure_hubv(excent_engine* e);
-// The lists changed: their split for swept passes holds no more (its memory is used again).
+// The lists, or the wave, changed: the split for swept passes holds no more (its memory is used again
+// where it suffices).
 static void lists_changed(excent_engine* e) {
     e->sweep_stale = true;
     if (!e->sweep_ok) return;
@@ -1911,6 +1913,8 @@ static int ensure_sweep(excent_engine* e) {
         parts.push_back(bytes);
     size_t total = 0;   // sizes to offsets, 256-byte aligned
     for (size_t& p : parts) { const size_t bytes = (p + 255) / 256 * 256; p = total; total += bytes; }
+    // the number of phases follows the wave: a split made with a larger one takes less room
+    if (e->d_sweep && e->sweep_bytes < total) { cudaFree(e->d_sweep); e->d_sweep = nullptr; }
     if (!e->d_sweep) {
         size_t fr = 0, all = 0;
         EX_CUDA(cudaMemGetInfo(&fr, &all));
@@ -1920,6 +1924,7 @@ static int ensure_sweep(excent_engine* e) {
             e->d_sweep = nullptr;
             return EXCENT_OK;
         }
+        e->sweep_bytes = total;
     }
     char* k = (char*)e->d_sweep;
     SweepBuild b{};
@@ -2333,7 +2338,9 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
     // leaves below eps depends on it
     int grid_asked = 0;
     EX_TRY(push_blocks(e, asked, &grid_asked));
-    e->wave = std::min(grid_asked * BLOCK, WAVE_MAX);
+    const int wave = std::min(grid_asked * BLOCK, WAVE_MAX);
+    if (wave != e->wave) lists_changed(e);   // the phases of a split are six waves
+    e->wave = wave;
     EX_TRY(push_blocks(e, smem, &e->grid_push));
     return EXCENT_OK;
 }

@@ -11,6 +11,8 @@ torch = pytest.importorskip("torch")
 if not torch.cuda.is_available():
     pytest.skip("needs a GPU", allow_module_level=True)
 
+import excent_b200 as X  # noqa: E402
+
 
 @pytest.mark.parametrize("sweep", [False, True])
 @pytest.mark.parametrize("n,cap", [(2500, 900), (2500, 1), (70001, 20000), (300007, 10 ** 9)])
@@ -32,3 +34,31 @@ def test_pending_lists_after_a_solve(n, cap, sweep):
             lo, hi = int(eng.chunk_v0[c]), int(ends[c])
             assert np.array_equal(np.sort(eng.chunk_list(c)), lo + np.nonzero(pending[lo:hi])[0]), (passes, c)
     eng.close()
+
+
+@pytest.mark.parametrize("how", ["set after a solve", "set after a solve, lists loaded anew"])
+@pytest.mark.parametrize("measure,slots", [("pr", 32768), ("all", 8192)])
+def test_swept_passes_follow_the_slots_set_last(measure, slots, how):
+    """The phases of a swept pass follow the wave, which follows the slots: a first chunk of more
+    vertices than six waves of one block to an SM is taken in one phase without slots and in two
+    with all of them, whichever was set first and whether or not the lists are loaded anew (63
+    chunks: the tables of the second split take more room than those of the first)."""
+    n = 300007
+    idx, adj = edged_graph(n, 6, symmetric=True)
+    v0 = np.array([0] + [240000 + 968 * k for k in range(62)], dtype=np.int32)
+    e = idx[np.append(v0, n)].astype(np.uint64)
+    got = []
+    for solved_before in (False, True):
+        eng = X.Engine(n, len(adj), X.measures(measure, eps_pr=EPS, eps_katz=EPS, eps_ev=EPS, alpha=0.01, lam=25.0), v0, e)
+        eng.upload_graph(idx, adj)
+        eng.set_sweep_demand(0.01)
+        if solved_before:
+            eng.solve(max_passes=1)
+        eng.set_hub_targets(slots)
+        if solved_before and how.endswith("anew"):
+            eng.load_cache(0, len(adj), adj)
+        eng.solve(max_passes=1)
+        got.append((eng.read(0), eng.read(0, residual=True)))
+        eng.close()
+    for a, b in zip(*got):   # the same takes in the same order: FP32 sums of up to 2049 terms apart
+        assert np.allclose(a, b, rtol=1e-5, atol=1e-6)
