@@ -1104,6 +1104,10 @@ static int free_engine(excent_engine* e) {
 static constexpr ull wave_seg(ull m) { return m < (1ull << 26) ? 256 : HUB_SEG; }
 // Most items of a wave, whatever the occupancy (148 SMs x 2048 threads).
 static constexpr int WAVE_MAX = 1 << 18;
+// Hub-target slots take at most this much shared memory of a block, in either layout. A kernel's limit
+// belongs to the process: it is only ever set to what every engine may need, never to one engine's size.
+static constexpr int SLOT_BYTES_MAX = 128 * 1024;
+static constexpr int slot_max(int L) { return SLOT_BYTES_MAX / (L == 1 ? (int)sizeof(float) : (int)sizeof(float4)); }
 
 // Blocks of k_push resident at once with `smem` bytes of hub-target slots.
 static int push_blocks(excent_engine* e, size_t smem, int* grid) {
@@ -1854,8 +1858,9 @@ static bool small_solve(const excent_engine* e, int order) {
 static cudaError_t launch_small(excent_engine* e, SolveArgs& a, cudaStream_t st) {
     const int per = e->n <= e->sms * PT ? 1 : 2;
     auto kernel = e->L == 1 ? (per == 1 ? k_small<1, 1> : k_small<1, 2>) : (per == 1 ? k_small<4, 1> : k_small<4, 2>);
-    const size_t smem = (hub_smem(e) + 15) / 16 * 16 + (size_t)PT * per * (e->L == 1 ? sizeof(SmallRec<1>) : sizeof(SmallRec<4>));
-    const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t recs = (size_t)PT * per * (e->L == 1 ? sizeof(SmallRec<1>) : sizeof(SmallRec<4>));
+    const size_t smem = (hub_smem(e) + 15) / 16 * 16 + recs;
+    const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SLOT_BYTES_MAX + (int)recs);
     if (rc != cudaSuccess) return rc;
     return launch_grid(kernel, solve_grid(e), PT, smem, a, &e->d_ctrl->bar, st);
 }
@@ -2260,7 +2265,7 @@ extern "C" int excent_device_info(int device, excent_device_info_t* out) {
 
 extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
     EX_CHECK_ARG(e && k >= 0, "bad argument");
-    const int kmax = e->L == 1 ? 32768 : 8192;   // 128 KiB of shared accumulators per block
+    const int kmax = slot_max(e->L);
     EX_CHECK_ARG(k <= kmax, "at most %d hub targets for this layout", kmax);
     EX_CHECK_ARG(k <= e->n, "more hub targets than vertices");
     EX_CUDA(cudaSetDevice(e->dev));
@@ -2305,7 +2310,7 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
         e->hub_k = k;
         if ((size_t)k * sizeof(int) > 48 * 1024)   // the encoder keeps the sorted ids in shared memory
             EX_CUDA(cudaFuncSetAttribute(k_hub_encode, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)((size_t)k * sizeof(int))));
+                                         slot_max(1) * (int)sizeof(int)));
         for (int c = 0; c < e->nc; c++)   // chunks loaded so far; later loads encode themselves
             if (e->loaded[c] && e->ce[c + 1] <= e->cache_edges) hub_encode(e, e->ce[c], e->ce[c + 1], e->s_main);
         EX_CUDA(cudaStreamSynchronize(e->s_main));
@@ -2313,7 +2318,7 @@ extern "C" int excent_engine_set_hub_targets(excent_engine* e, int k) {
     }
     const size_t smem = hub_smem(e);
     if (asked > 0) {   // static + dynamic above 48 KiB needs the opt-in, per kernel (the staged kernels hold ~40 KiB)
-        const int sz = (int)asked;
+        const int sz = SLOT_BYTES_MAX;
         cudaFuncSetAttribute(k_push<1, SRC_TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_push<1, SRC_CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
         cudaFuncSetAttribute(k_push<1, SRC_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, sz);
@@ -2398,8 +2403,8 @@ extern "C" int excent_engine_scatter_peak(excent_engine* e, double* entries_per_
     cudaEventCreate(&e1);
     float best = 0.f;
     if (hub_smem(e)) {
-        cudaFuncSetAttribute(k_scatter_probe<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hub_smem(e));
-        cudaFuncSetAttribute(k_scatter_probe<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hub_smem(e));
+        cudaFuncSetAttribute(k_scatter_probe<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SLOT_BYTES_MAX);
+        cudaFuncSetAttribute(k_scatter_probe<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SLOT_BYTES_MAX);
     }
     for (int rep = 0; rep < 4; rep++) {   // the first launch warms up; best of the other three
         cudaEventRecord(e0, e->s_main);

@@ -1,8 +1,11 @@
 """What a solve and a host-driven push leave behind, and what engines and
 streams share."""
+import threading
+
 import numpy as np
 import pytest
 
+import oracle as O
 from test_long_lists_gpu import edged_graph
 from test_passes_gpu import EPS, engine
 
@@ -62,3 +65,49 @@ def test_swept_passes_follow_the_slots_set_last(measure, slots, how):
         eng.close()
     for a, b in zip(*got):   # the same takes in the same order: FP32 sums of up to 2049 terms apart
         assert np.allclose(a, b, rtol=1e-5, atol=1e-6)
+
+
+def test_slots_of_another_engine_leave_an_engine_its_own(rmat16):
+    """Two engines of one process: the one with more slots solves and pushes as before after the other
+    has set fewer."""
+    n, idx, adj = rmat16
+    lam = float(O.params(n, idx, adj)["_lambda"])
+    many = engine(n, idx, adj, "all", len(adj) // 5, alpha=0.5 / lam, lam=lam)
+    many.set_hub_targets(8192)
+    few = engine(n, idx, adj, "all", len(adj) // 5, alpha=0.5 / lam, lam=lam)
+    few.set_hub_targets(64)
+    for sweep in (True, False):
+        many.set_chunk_sweep(sweep)
+        for use_graph in (True, False):
+            many.solve(max_passes=20, use_graph=use_graph)
+        many.init()
+        cnt, _, _ = many.snapshot()
+        many.push_cached((cnt[0::2] > 0).astype(np.uint8), cnt)
+        many.sync()
+    assert many.scatter_peak() > 0
+    many.close()
+    few.close()
+
+
+def test_small_solves_of_two_threads(rmat12):
+    """Two threads solve small graphs with different numbers of slots at the same time."""
+    n, idx, adj = rmat12
+    engines = [engine(n, idx, adj, "pr", len(adj)) for _ in range(2)]
+    for eng, k in zip(engines, (n, 8)):
+        eng.set_hub_targets(k)
+    bad = []
+
+    def solves(eng):
+        try:
+            for _ in range(300):
+                eng.solve(max_passes=3)
+        except Exception as ex:   # noqa: BLE001
+            bad.append(ex)
+    threads = [threading.Thread(target=solves, args=(eng,)) for eng in engines]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[0]
+    for eng in engines:
+        eng.close()
