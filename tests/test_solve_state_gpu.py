@@ -7,7 +7,7 @@ import pytest
 
 import oracle as O
 from test_long_lists_gpu import edged_graph
-from test_passes_gpu import EPS, engine
+from test_passes_gpu import EPS, close_enough, engine
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -111,3 +111,23 @@ def test_small_solves_of_two_threads(rmat12):
     assert not bad, bad[0]
     for eng in engines:
         eng.close()
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_one_chunk_of_lists_in_host_memory_goes_as_a_range(use_graph):
+    """A chunk read over the host link is pushed as a range in every pass, also by the solve of a
+    graph whose vertices fit the GPU's threads: one that turns pending in a pass is pushed in it."""
+    n = 2500
+    idx, adj = edged_graph(n, 8, symmetric=True)
+    meas = X.measures("pr", eps_pr=EPS)
+    eng = X.Engine(n, len(adj), meas, *X.plan_chunks(idx, len(adj)))
+    assert eng.nc == 1
+    eng.upload_offsets(idx)
+    eng.reserve_cache(0)
+    buf, first = eng.host_cache()
+    assert first == 0
+    buf[:] = adj
+    st = eng.solve(use_graph=use_graph)
+    assert (st.n_list, st.n_range) == (0, st.passes) and eng.host_pushed() == st.pushed
+    assert close_enough("pr", n, eng.read(0), O.reference_solution(n, idx, adj, "pr"))
+    eng.close()
