@@ -130,7 +130,8 @@ __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
                 if (v >= a.n) continue;
                 if (dv[k] != 0.f) a.x[v] += dv[k];
                 const bool above = fabsf(rv[k]) > a.eps;
-                const float d = above || pull ? rv[k] : 0.f;
+                // (a residual that is no number, from a row whose weights sum to 0, is never above eps: it stays)
+                const float d = above || (pull && rv[k] == rv[k]) ? rv[k] : 0.f;
                 if (d != 0.f) a.r[v] = 0.f;
                 if (d != 0.f || dv[k] != 0.f) a.d[v] = d;
                 if (above) {

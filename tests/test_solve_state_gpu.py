@@ -131,3 +131,45 @@ def test_one_chunk_of_lists_in_host_memory_goes_as_a_range(use_graph):
     assert (st.n_list, st.n_range) == (0, st.passes) and eng.host_pushed() == st.pushed
     assert close_enough("pr", n, eng.read(0), O.reference_solution(n, idx, adj, "pr"))
     eng.close()
+
+
+@pytest.mark.parametrize("kind,s", [("pr", 0.85), ("katz", 0.6)])
+def test_a_residual_that_is_not_a_number_stays_where_it_is(kind, s):
+    """A row whose weights are all 0 has no normalised weights. Its targets' residuals are no numbers
+    from its first push on: they are taken no more, and nothing of them reaches other vertices."""
+    from excent_b200.autograd import WeightedGraph
+    n, k = 2000, 4
+    rng = np.random.default_rng(3)
+    adj = np.concatenate([np.sort(rng.choice(n, k, replace=False)) for _ in range(n)]).astype(np.int32)
+    idx = (np.arange(n + 1) * k).astype(np.uint64)
+    w = rng.uniform(0.5, 1.5, len(adj)).astype(np.float32)
+    u = 77
+    w[u * k:(u + 1) * k] = 0
+    dev = torch.device("cuda")
+    G = WeightedGraph(n, torch.from_numpy(idx.view(np.int64)).to(dev), torch.from_numpy(adj).to(dev),
+                      torch.from_numpy(w).to(dev))
+    src = np.repeat(np.arange(n), k)
+    with np.errstate(all="ignore"):
+        wn = w / np.bincount(src, w, n)[src]
+
+    def push(frm, to, r):
+        x = np.zeros(n)
+        for _ in range(400):
+            d = np.where(np.abs(r) > 1e-12, r, 0.0)   # (no number is above nothing)
+            x += d
+            r = np.where(d != 0, 0.0, r)
+            np.add.at(r, to, np.where(d[frm] != 0, s * wn * d[frm], 0.0))
+        return x
+
+    c0 = 1 - s if kind == "pr" else 1.0
+    x, _, _ = G.forward(kind, s, None, 1e-7)
+    assert np.allclose(x.cpu().numpy(), push(src, adj, np.full(n, c0)), rtol=1e-4, atol=1e-5)
+    c = np.zeros(n)
+    c[rng.choice(n, 300, replace=False)] = 1
+    c[adj[u * k]] = 1
+    gt, gw = G.vjp(torch.from_numpy(c.astype(np.float32)).to(dev), 1e-7)
+    lam = push(adj, src, c)
+    assert np.allclose(gt.cpu().numpy(), c0 * lam, rtol=1e-4, atol=1e-5)
+    finite = np.isfinite(gw.cpu().numpy())
+    assert finite[src != u].all()
+    G.close()
