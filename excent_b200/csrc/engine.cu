@@ -1539,9 +1539,11 @@ extern "C" int excent_engine_push_cached(excent_engine* e, const unsigned char* 
         e->launches++;
         return EXCENT_OK;
     }
+    // SRC_HUBS goes through the graph's whole high-degree list, so every chunk has to be loaded
+    const bool all_loaded = std::all_of(e->loaded.begin(), e->loaded.end(), [](uint8_t ok) { return ok != 0; });
     int order = 0;
     if (order_of(e) == 3) order = 3;   // inside each launch: needs no high-degree list
-    else if (all_cached && !sweep_of(e)) order = effective_order(e);
+    else if (all_cached && all_loaded && !sweep_of(e)) order = effective_order(e);
     PushArgs a = push_args(e, 0);
     a.hot = e->hot_skip ? e->d_hot : nullptr;
     if (order == 1) launch_push<SRC_HUBS>(e, a, e->grid_push, e->s_main);

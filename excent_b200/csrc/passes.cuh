@@ -417,11 +417,13 @@ template <int L> struct Passes {
         return sync();
     }
 
-    // The long lists of hub vertices [h0, h1), all taken before any is scattered.
+    // The long lists of hub vertices [h0, h1), all taken before any is scattered. A host-driven push
+    // leaves the vertices of other chunks than it was asked for alone: their lists may not be loaded.
     __device__ __forceinline__ bool push_hubs(long long h0, long long h1, bool listed) {
         if (h1 <= h0) return true;
         return push_wave(h1 - h0, LISTS_LONG, [&](long long i) {
             const int v = a.push.hubv[h0 + i];
+            if (a.standalone && type[chunk_of(v, a.push.cv0, a.push.nc)] == WT_NONE) return -1;
             return listed && !bit_of(a.snap.bitmap, v) ? -1 : v;
         });
     }

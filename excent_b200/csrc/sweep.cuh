@@ -619,6 +619,7 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
         while (bits) {
             const int v = (int)w * 32 + __ffs(bits) - 1;
             bits &= bits - 1;
+            if (a.standalone && a.push.wt_type[chunk_of(v, a.push.cv0, nc)] == WT_NONE) continue;   // not asked for
             take_here<L>(x, r, P, v, r[v], 0, true, false, a.push.M, pushed, lanes, taken);
         }
     }

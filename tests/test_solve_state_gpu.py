@@ -15,6 +15,7 @@ if not torch.cuda.is_available():
     pytest.skip("needs a GPU", allow_module_level=True)
 
 import excent_b200 as X  # noqa: E402
+import excent_b200._capi as K  # noqa: E402
 
 
 @pytest.mark.parametrize("sweep", [False, True])
@@ -173,3 +174,46 @@ def test_a_residual_that_is_not_a_number_stays_where_it_is(kind, s):
     finite = np.isfinite(gw.cpu().numpy())
     assert finite[src != u].all()
     G.close()
+
+
+@pytest.mark.parametrize("order", ["first", "last", "launch-first"])
+@pytest.mark.parametrize("sweep,degree_cache", [(False, False), (True, False), (False, True)])
+def test_a_push_of_some_chunks_leaves_the_others_alone(order, sweep, degree_cache):
+    """Chunks without pending vertices at the snapshot are in no push: their vertices, high-degree
+    and without entries alike, keep what reaches them, also where their lists are not loaded."""
+    n = 2500
+    idx, adj = edged_graph(n, 9, symmetric=True)
+    deg = np.diff(idx.astype(np.int64))
+    eng = engine(n, idx, adj, "pr", 900)
+    ends = np.append(eng.chunk_v0[1:], n)
+    chunk = np.searchsorted(eng.chunk_v0, np.arange(n), side="right") - 1
+    asked = np.arange(eng.nc) >= eng.nc // 2
+    hubs = np.nonzero(deg > 256)[0]
+    assert eng.nc > 4 and len(hubs) > 5 and not asked[chunk[hubs]].all()
+    eng.set_hub_order(order)
+    eng.set_chunk_sweep(sweep)
+    eng.set_sweep_demand(0.0)
+    for c in np.nonzero(~asked)[0]:
+        eng.set_loaded(int(c), False)
+    eng.init()
+    x0 = np.zeros(n, dtype=np.float32)
+    r0 = np.where(asked[chunk], np.float32(0.5), np.float32(0)).astype(np.float32)
+    eng.write(0, x0, r0)
+    if degree_cache:   # one vertex in it: the pushes go chunk by chunk as launches of their own
+        v = int(np.nonzero((deg > 0) & (deg < 9) & ~asked[chunk])[0][0])
+        ids, off, bits = np.array([v], np.int32), np.array([0, deg[v]], np.uint64), np.zeros((n + 31) // 32, np.uint32)
+        bits[v >> 5] = 1 << (v & 31)
+        K.call("excent_engine_hot_setup", eng.h, 1, ids.ctypes.data_as(K.i32p), off.ctypes.data_as(K.u64p),
+               bits.ctypes.data_as(K.u32p))
+    cnt, _, _ = eng.snapshot(use_hot=degree_cache)
+    assert np.array_equal(cnt[0::2] > 0, asked)
+    eng.push_cached(asked.astype(np.uint8), cnt)
+    eng.sync()
+    x, r = eng.read(0), eng.read(0, residual=True)
+    rest = ~asked[chunk]
+    assert not x[rest].any()
+    assert r[hubs[rest[hubs]]].min() > EPS   # (something did reach them)
+    # what was taken is delivered: sum r + (1 - 0.85) sum x (vertices without entries keep all they take)
+    lost = np.where(deg == 0, 1.0, 0.15)
+    assert abs(r.astype(np.float64).sum() + (lost * x).sum() - r0.astype(np.float64).sum()) <= 1e-5 * r0.sum()
+    eng.close()
