@@ -986,6 +986,8 @@ struct excent_engine {
     cudaStream_t s_main = nullptr;
     Slot slot[2];
     bool slots_ok = false, zc = false;
+    cudaEvent_t alone = nullptr;   // after the last push whose takes have no exchange, which ...
+    bool alone_set = false;        // ... may still run
     ull max_chunk_edges = 0;
     int max_chunk_verts = 0;
     // graph
@@ -1088,6 +1090,7 @@ static int free_engine(excent_engine* e) {
         if (s.done) cudaEventDestroy(s.done);
     }
     for (cudaEvent_t ev : e->ev) if (ev) cudaEventDestroy(ev);
+    if (e->alone) cudaEventDestroy(e->alone);
     free_host_cache(e);
     if (e->s_main) cudaStreamDestroy(e->s_main);
     delete e;
@@ -1490,6 +1493,24 @@ static int grid_for(excent_engine* e, ull items) {
     return (int)std::max<ull>(1, std::min<ull>(blocks, (ull)e->grid_push));
 }
 
+// A push in one launch takes residuals without exchanges, in phases in which nobody adds to them:
+// it waits for what the slots push, and they wait for it.
+static int wait_for_slots(excent_engine* e) {
+    if (e->slots_ok)
+        for (Slot& s : e->slot) if (s.busy) EX_CUDA(cudaStreamWaitEvent(e->s_main, s.done, 0));
+    return EXCENT_OK;
+}
+static int mark_alone(excent_engine* e) {
+    if (!e->slots_ok) return EXCENT_OK;
+    EX_CUDA(cudaEventRecord(e->alone, e->s_main));
+    e->alone_set = true;
+    return EXCENT_OK;
+}
+static int wait_for_alone(excent_engine* e, Slot& s) {
+    if (e->alone_set) EX_CUDA(cudaStreamWaitEvent(s.st, e->alone, 0));
+    return EXCENT_OK;
+}
+
 static SolveArgs solve_args(excent_engine* e, double list_frac, int max_passes);
 static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st);
 static cudaError_t launch_table(excent_engine* e, SolveArgs& a, cudaStream_t st);
@@ -1532,12 +1553,13 @@ extern "C" int excent_engine_push_cached(excent_engine* e, const unsigned char* 
     // with every pending list in the cache, and none kept apart in the degree cache, the push is one
     // launch; it was up to three kernels and two memsets a chunk
     if (all_cached && !e->hot_skip && effective_order(e) == order_of(e)) {
+        EX_TRY(wait_for_slots(e));
         if (sweep) EX_TRY(ensure_sweep(e));
         SolveArgs s = solve_args(e, list_frac, 0);
         s.standalone = 1;
         EX_CUDA(sweep ? launch_sweep(e, s, e->s_main) : launch_table(e, s, e->s_main));
         e->launches++;
-        return EXCENT_OK;
+        return mark_alone(e);
     }
     // SRC_HUBS goes through the graph's whole high-degree list, so every chunk has to be loaded
     const bool all_loaded = std::all_of(e->loaded.begin(), e->loaded.end(), [](uint8_t ok) { return ok != 0; });
@@ -1603,6 +1625,7 @@ extern "C" int excent_engine_slots_create(excent_engine* e, unsigned long long m
         EX_CUDA(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
         EX_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
     }
+    if (!e->alone) EX_CUDA(cudaEventCreateWithFlags(&e->alone, cudaEventDisableTiming));
     for (int q = 1; q < 3; q++) {
         const ull me = std::max<ull>(max_chunk_edges, 1);
         e->hub_cap[q] = me / HUB_SEG + me / HUB_MIN + 64;
@@ -1657,6 +1680,7 @@ extern "C" int excent_engine_push_stream(excent_engine* e, int s, int c, const u
     a.stage = e->zc ? 0 : 1;   // mapped host slots are read in place
     if ((double)k < list_frac * nv) { a.ctype = WT_LIST; a.ccount = (unsigned)k; e->n_list++; }
     else { a.ctype = WT_RANGE; a.ccount = (unsigned)nv; e->n_range++; }
+    EX_TRY(wait_for_alone(e, sl));
     if (a.ccount) launch_ordered<SRC_CHUNK>(e, a, grid_for(e, a.ccount), sl.st);
     EX_CUDA(cudaGetLastError());
     if (to_cache) { lists_changed(e); e->loaded[c] = 1; }
@@ -1679,6 +1703,7 @@ extern "C" int excent_engine_push_gather(excent_engine* e, int s, int k, unsigne
         PushArgs a = push_args(e, 1 + s);
         a.vids = sl.d_vids; a.off = sl.d_off; a.gedges = sl.d_edges; a.gk = (unsigned)k;
         a.stage = e->zc ? 0 : 1;
+        EX_TRY(wait_for_alone(e, sl));
         launch_ordered<SRC_GATHER>(e, a, grid_for(e, (ull)k), sl.st);
         EX_CUDA(cudaGetLastError());
     }
@@ -1769,6 +1794,7 @@ extern "C" int excent_engine_sync(excent_engine* e) {
     if (e->slots_ok) for (Slot& s : e->slot) { EX_CUDA(cudaStreamSynchronize(s.st)); s.busy = false; }
     EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
     EX_CUDA(cudaStreamSynchronize(e->s_main));
+    e->alone_set = false;
     const int err = e->h_ctrl->err;
     if (err) scrub_queues(e);
     if (err) EX_FAIL(EXCENT_ERR_STATE, "%s", ctrl_error(err));
@@ -2138,6 +2164,7 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
     for (int c = 0; c < e->nc; c++)
         if (e->d_hcache && e->ce[c] >= e->cache_edges) cm[c] = 2;   // lists in host memory
     EX_CUDA(cudaMemcpy(e->d_cmode, cm.data(), e->nc, cudaMemcpyHostToDevice));
+    EX_TRY(wait_for_slots(e));
     if (init) EX_TRY(init_state(e));
     else EX_TRY(reset_counters(e));
     if (order_of(e)) EX_TRY(ensure_hubv(e));

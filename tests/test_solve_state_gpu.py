@@ -1,5 +1,6 @@
 """What a solve and a host-driven push leave behind, and what engines and
 streams share."""
+import ctypes as C
 import threading
 
 import numpy as np
@@ -217,3 +218,38 @@ def test_a_push_of_some_chunks_leaves_the_others_alone(order, sweep, degree_cach
     lost = np.where(deg == 0, 1.0, 0.15)
     assert abs(r.astype(np.float64).sum() + (lost * x).sum() - r0.astype(np.float64).sum()) <= 1e-5 * r0.sum()
     eng.close()
+
+
+def test_slots_and_one_launch_pushes_do_not_run_side_by_side():
+    """Gathered lists in the slots and cached pushes in one launch, in turn and without a wait of
+    the host between them: nothing of a residual is lost. What is taken is delivered, so sum r +
+    (1 - 0.85) sum x stays as it was (a vertex without entries keeps all that it takes)."""
+    n = 70001
+    idx, adj = edged_graph(n, 12, symmetric=True)
+    deg = np.diff(idx.astype(np.int64))
+    for cap, sweep in ((len(adj), False), (len(adj) // 5, True), (len(adj) // 5, False)):
+        eng = engine(n, idx, adj, "pr", cap)
+        eng.set_chunk_sweep(sweep)
+        eng.set_sweep_demand(0.0)
+        k = int(np.diff(np.append(eng.chunk_v0, n)).max())   # (a gather is of one chunk's size at most)
+        K.call("excent_engine_slots_create", eng.h, len(adj), k, 0)
+        for s in (0, 1):
+            ed, vi, of = C.POINTER(C.c_int32)(), C.POINTER(C.c_int32)(), C.POINTER(C.c_uint64)()
+            K.call("excent_engine_slot_buffers", eng.h, s, C.byref(ed), C.byref(vi), C.byref(of))
+            np.ctypeslib.as_array(ed, shape=(len(adj),))[:] = adj
+            np.ctypeslib.as_array(vi, shape=(k,))[:] = np.arange(k)
+            np.ctypeslib.as_array(of, shape=(k + 1,))[:] = idx[:k + 1]
+        eng.init()
+        cnt, _, _ = eng.snapshot()
+        mode = np.ones(eng.nc, dtype=np.uint8)
+        before = float(np.float32(1) - np.float32(0.85)) * n
+        for turn in range(12):
+            s = turn % 2
+            K.call("excent_engine_slot_wait", eng.h, s)
+            K.call("excent_engine_push_gather", eng.h, s, k, int(idx[k]))
+            eng.push_cached(mode, cnt)
+        eng.sync()
+        x, r = eng.read(0).astype(np.float64), eng.read(0, residual=True).astype(np.float64)
+        now = r.sum() + (np.where(deg == 0, 1.0, 0.15) * x).sum()
+        assert abs(now - before) <= 1e-5 * before, (cap, sweep, now / before)
+        eng.close()
