@@ -159,6 +159,7 @@ struct PushArgs {
     // (hubv[*hubv_cnt]) first; SRC_TABLE then skips them
     const int* hubv;
     const ull* hubv_cnt;
+    int until_done;     // SRC_HUBS: nothing to push once the solve is done
     int lists;          // LISTS_ALL, or only the lists of at most HUB_MIN entries, or only the longer ones
     int chunk;          // SRC_TABLE: only chunk `chunk`'s items (-1: every chunk's)
     int stage;          // SRC_CHUNK / SRC_GATHER: bulk-copy each tile's short lists into shared memory
@@ -414,14 +415,15 @@ __global__ void __launch_bounds__(BLOCK) k_snapshot(SnapArgs a) {
     }
 }
 
-// On-device fetch plan of the host-driven loop: per chunk with pending
+// On-device fetch plan of a pass whose push is separate launches, by the host or in a
+// graph's while node (whose condition it sets): per chunk with pending
 // vertices choose its pending list (cnt < list_frac * vertices) or its whole
 // range (src/excent.cu:639), build the item prefix, log the pass, decide
 // termination (src/excent.cu:680, max passes :656), and reset the counters the
 // next snapshot accumulates into.
 __global__ void k_plan(int nc, const int* cv0, int n, ull* cnt, const uint8_t* cmode, double list_frac, int max_passes,
                        uint8_t* wt_type, unsigned* wt_prefix, Ctrl* ctrl, PushQueue* q0, PassRec* log, int log_cap,
-                       int sweep, ull sweep_min) {
+                       int sweep, ull sweep_min, cudaGraphConditionalHandle again, int use_cond) {
     __shared__ ull s_pend, s_dem;
     __shared__ unsigned s_carry;
     __shared__ int s_nl, s_nr;
@@ -484,6 +486,7 @@ __global__ void k_plan(int nc, const int* cv0, int n, ull* cnt, const uint8_t* c
         ctrl->items = stop ? 0 : s_carry;
         ctrl->sweep_pass = sweep_pass ? 1 : 0;
         if (stop) ctrl->done = 1; else ctrl->pass = p + 1;
+        if (use_cond) cudaGraphSetConditional(again, stop ? 0u : 1u);
         q0->tail = 0; q0->claim = 0;
         ctrl->hotpend = 0;
         ctrl->ev_corr = ctrl->ev_dot;
@@ -566,7 +569,7 @@ __device__ __forceinline__ long long item_total(const PushArgs& a) {
     if constexpr (SRC == SRC_TABLE) return a.wt_prefix[a.chunk >= 0 ? a.chunk + 1 : a.nc];
     else if constexpr (SRC == SRC_CHUNK) return a.ccount;
     else if constexpr (SRC == SRC_GATHER) return a.gk;
-    else if constexpr (SRC == SRC_HUBS) return (long long)*a.hubv_cnt;
+    else if constexpr (SRC == SRC_HUBS) return a.until_done && a.ctrl->done ? 0 : (long long)*a.hubv_cnt;
     else return a.ctrl->hcount;
 }
 
@@ -994,6 +997,7 @@ struct excent_engine {
     cudaGraphExec_t gexec = nullptr;
     cudaGraph_t graph = nullptr;
     int graph_max_passes = -1;
+    int graph_launches = 0;        // kernels of one pass of separate launches
     double graph_list_frac = -1;
     // per-kernel timing of the host-driven device solve (excent_engine_profile)
     bool prof = false;
@@ -1803,18 +1807,20 @@ extern "C" int excent_engine_sync(excent_engine* e) {
 
 // One pass of the host-driven loop: snapshot and plan (read back), then the
 // pushes the plan chose. With ev, events are recorded between the kernels.
-static void enqueue_plan(excent_engine* e, double list_frac, int max_passes, cudaStream_t st, cudaEvent_t* ev) {
+static void enqueue_plan(excent_engine* e, double list_frac, int max_passes, cudaStream_t st, cudaEvent_t* ev,
+                         cudaGraphConditionalHandle again = 0, int use_cond = 0) {
     if (ev) cudaEventRecord(ev[0], st);
     launch_snapshot(e, false, st);
     if (ev) cudaEventRecord(ev[1], st);
     k_plan<<<1, 1024, 0, st>>>(e->nc, e->d_cv0, e->n, e->d_cnt, e->d_cmode, list_frac, max_passes, e->d_wt_type,
                                e->d_wt_prefix, e->d_ctrl, e->d_queue, e->d_log, e->log_cap, sweep_of(e) ? 1 : 0,
-                               sweep_min_entries(e));
+                               sweep_min_entries(e), again, use_cond);
     e->launches++;
     if (ev) cudaEventRecord(ev[2], st);
 }
 static cudaError_t enqueue_push(excent_engine* e, cudaStream_t st, cudaEvent_t* ev, bool sweep_pass) {
     PushArgs a = push_args(e, 0);
+    a.until_done = 1;   // (in a graph the pass that found the end launches its pushes as well)
     // high-degree order: 1 = the lists longer than HUB_MIN first, so their (large) share of the
     // pass's residual reaches every other vertex before that vertex is taken; 2 = last, so they
     // collect the pass's residual and push it once; 0 = in table order with the rest
@@ -2019,13 +2025,15 @@ static int ensure_sweep(excent_engine* e) {
     return EXCENT_OK;
 }
 
-// The solve of a sweeping engine: while { k_passes; k_sweep }, a sweep leaving at once unless one is
-// due. (An IF node around it and memset nodes for the barriers cost 10 us a pass more.)
+// The loop of a solve as a while node: of a sweeping engine { k_passes; k_sweep }, a sweep leaving at
+// once unless one is due (an IF node around it and memset nodes for the barriers cost 10 us a pass
+// more); of another { snapshot; plan; the pushes }, see one_launch.
 static int build_graph(excent_engine* e, double list_frac, int max_passes) {
     if (e->gexec && e->graph_max_passes == max_passes && e->graph_list_frac == list_frac) return EXCENT_OK;
     invalidate_graph(e);
     SolveArgs a = solve_args(e, list_frac, max_passes);
     a.use_cond = 1;
+    const ull launches = e->launches;
     cudaGraph_t g;
     EX_CUDA(cudaGraphCreate(&g, 0));
     cudaStream_t cs = nullptr;
@@ -2043,8 +2051,15 @@ static int build_graph(excent_engine* e, double list_frac, int max_passes) {
         rc = cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal);
     if (rc == cudaSuccess) {
-        rc = launch_passes(e, a, cs);
-        if (rc == cudaSuccess) rc = launch_sweep(e, a, cs);
+        if (sweep_of(e)) {
+            rc = launch_passes(e, a, cs);
+            if (rc == cudaSuccess) rc = launch_sweep(e, a, cs);
+        } else {
+            enqueue_plan(e, list_frac, max_passes, cs, nullptr, a.again, 1);
+            rc = enqueue_push(e, cs, nullptr, false);
+        }
+        e->graph_launches = (int)(e->launches - launches);
+        e->launches = launches;
         const cudaError_t ce = cudaStreamEndCapture(cs, &captured);
         if (rc == cudaSuccess) rc = ce;
     }
@@ -2147,11 +2162,17 @@ static int ensure_hubv(excent_engine* e) {
     return EXCENT_OK;
 }
 
-// Without a chunk sweep a pass is one phase, and above some 2^25 entries its scatter outlasts what a
-// launch costs: k_push and k_segments, three blocks to an SM, then beat k_passes, one block to an SM,
-// in spite of a host round trip a pass (PageRank, 65M entries: 16.3 against 18.8 ms, 14.8 by launches in a
-// graph; 263M: 47.1, 57.1 and 45.3; 16M entries: 5.4 by k_passes and 6.9 in a graph).
-static constexpr ull ONE_LAUNCH_MAX = 1ull << 25;
+// Without a chunk sweep a pass is one phase. Its scatter is slower by k_passes, one block to an SM, than
+// by k_push and k_segments with three, whose launches in turn cost a small graph more than its work: the
+// more entries, and the more memory their targets are spread over. Both were measured on R-MATs of 2^17
+// to 2^24 vertices (ms by k_passes and by launches in a graph): one measure, 8 MB of residuals, 8M
+// entries 5.4 and 6.4, 16M 6.5 and 6.9 (Katz 24.8 and 23.0), 24M 7.9 and 7.2; 4 MB, 30M 7.2 and 7.6, 61M 13.3
+// and 12.7; 16 MB, 4M 5.6 and 5.6, 16M 8.1 and 7.2; 64 MB, 17M 16.3 and 11.9. Three measures, 8 MB, 15M
+// 20.6 and 21.7; 16 MB, 4M 12.1 and 12.3, 12M 20.1 and 19.5; 32 MB, 16M 30.4 and 24.4.
+static bool one_launch(const excent_engine* e) {
+    const double residuals = (double)e->n * (e->L == 1 ? sizeof(float) : sizeof(float4));
+    return e->m < (1ull << 25) && residuals * residuals * (double)e->m < 1.1e21;
+}
 
 static int solve_impl(excent_engine* e, double list_frac, int max_passes, int use_graph, bool init) {
     EX_CHECK_ARG(e, "null engine");
@@ -2168,9 +2189,10 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
     if (init) EX_TRY(init_state(e));
     else EX_TRY(reset_counters(e));
     if (order_of(e)) EX_TRY(ensure_hubv(e));
-    if (use_graph && (sweep_of(e) || e->m < ONE_LAUNCH_MAX)) {
-        if (sweep_of(e)) {
-            EX_TRY(ensure_sweep(e));
+    if (use_graph) {
+        const bool loop = sweep_of(e) || !one_launch(e);
+        if (loop) {
+            if (sweep_of(e)) EX_TRY(ensure_sweep(e));
             EX_TRY(build_graph(e, list_frac, max_passes));
             EX_CUDA(cudaGraphLaunch(e->gexec, e->s_main));
         } else {   // every pass in one launch
@@ -2179,12 +2201,12 @@ static int solve_impl(excent_engine* e, double list_frac, int max_passes, int us
         }
         EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
         EX_CUDA(cudaStreamSynchronize(e->s_main));
-        // each iteration of the loop launches both kernels
-        e->launches += sweep_of(e) ? 2 * (e->h_ctrl->sweeps + 1) : 1;
+        // each iteration of the loop launches all its kernels
+        e->launches += !loop ? 1 : sweep_of(e) ? 2 * (e->h_ctrl->sweeps + 1) : (ull)e->graph_launches * (e->h_ctrl->pass + 1);
     } else {
         // snapshot and plan, read the plan back (one sync per pass), then the pushes it chose
         for (int p = 0; p <= max_passes; p++) {
-            cudaEvent_t* ev = e->prof && !use_graph ? e->ev : nullptr;
+            cudaEvent_t* ev = e->prof ? e->ev : nullptr;
             enqueue_plan(e, list_frac, max_passes, e->s_main, ev);
             EX_CUDA(cudaMemcpyAsync(e->h_ctrl, e->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, e->s_main));
             EX_CUDA(cudaStreamSynchronize(e->s_main));

@@ -179,9 +179,9 @@ int excent_engine_sync(excent_engine* e);
  * init, then passes of snapshot -> on-device fetch plan -> push until no
  * vertex is pending or max_passes. With use_graph there is no host round trip
  * per pass: all passes are one cooperative launch, or, where passes are swept
- * chunk by chunk, one CUDA graph with a conditional while node; without it, and
- * on a graph of 2^25 entries or more that is not swept, the host reads each
- * pass's plan back and launches its pushes.
+ * chunk by chunk or the graph is large, one CUDA graph with a conditional while
+ * node; without it the host reads each pass's plan back and
+ * launches its pushes.
  * Per-pass log and totals are kept for excent_engine_stats. */
 int excent_engine_solve(excent_engine* e, double list_frac, int max_passes, int use_graph);
 

@@ -253,3 +253,37 @@ def test_slots_and_one_launch_pushes_do_not_run_side_by_side():
         now = r.sum() + (np.where(deg == 0, 1.0, 0.15) * x).sum()
         assert abs(now - before) <= 1e-5 * before, (cap, sweep, now / before)
         eng.close()
+
+
+@pytest.mark.parametrize("measure,scale,ef", [("pr", 21, 17), ("pr", 22, 2), ("all", 20, 8)])
+def test_unswept_solves_of_large_graphs_ask_the_host_nothing(measure, scale, ef):
+    """Where the passes of a solve are launches of their own they still run in one submission, and a
+    pass limit ends them all: no high-degree list is pushed past it, and nothing is lost (what is taken
+    is delivered: sum r + (1 - 0.85) sum x of PageRank stays as it was)."""
+    from torch.profiler import ProfilerActivity, profile
+    g = X.DeviceGraph(scale, ef, 5)
+    di, da, _ = g.device_ptrs()
+    idx = np.empty(g.n + 1, dtype=np.uint64)
+    adj = np.empty(g.m, dtype=np.int32)
+    g.download(idx, adj)
+    deg = np.diff(idx.astype(np.int64))
+    assert (deg > 256).any()
+    meas = X.measures(measure, eps_pr=0.01, eps_katz=0.01, eps_ev=0.01, alpha=1e-4, lam=1e3)
+    eng = X.Engine(g.n, g.m, meas, *X.plan_chunks(idx, g.m))
+    eng.upload_device(di, da)
+    eng.solve(max_passes=1)
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        st = eng.solve(max_passes=40)
+    waits = sum(ev.name == "cudaStreamSynchronize" for ev in prof.events())
+    assert st.passes > 10 and waits <= 2, (st.passes, waits)
+    for passes in (1, 2, 5, 100000):
+        st, log = (eng.solve(max_passes=passes), eng.stats(with_log=True)[1])
+        assert st.passes == passes or passes == 100000
+        assert sum(int(p.pushed) for p in log) == st.pushed
+        res = [eng.read(i, residual=True) for i in range(meas.nm)]
+        pending = np.any([np.abs(r) > np.float32(0.01) for r in res], axis=0)
+        assert np.array_equal(np.sort(eng.chunk_list(0)), np.nonzero(pending)[0])
+        total = res[0].astype(np.float64).sum() + (np.where(deg == 0, 1.0, 0.15) * eng.read(0)).sum()
+        assert abs(total - 0.15 * g.n) <= 1e-5 * 0.15 * g.n
+    eng.close()
+    g.close()
