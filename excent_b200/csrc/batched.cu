@@ -168,12 +168,14 @@ __device__ __forceinline__ int compact_groups(const float4 (&p)[NV], const bool 
 //
 // What bounds it: in the dense passes the warps whose word holds 32 vertices
 // with long lists, one row after the other; in the others the latency of the
-// two phases. Neighbouring words go to different SMs, the next row's offsets
-// are loaded while a row is pushed, the values are added by reductions, which
-// nothing waits for, and rows with many active groups scatter over their
-// groups. 64 queries on 131k vertices to 1e-6: 9.8 ms as three kernels a pass
-// in a graph, 7.4 ms; 256 on 50k: 36 and 19 ms. Sharing a word's rows between
-// a block's warps as well gave 5.7 and 12 ms, but it moves the takes of those
+// two phases. Neighbouring words go to different SMs, the values are added by
+// reductions, which nothing waits for, and rows with many active groups scatter
+// over their groups. 64 queries on 131k vertices to 1e-6: 10.4 ms as three
+// kernels a pass in a graph, 8.2 ms; 256 on 65k: 36.7 and 17.5 ms; 256 on 16.8M
+// vertices to 1e-4 of their mass, where 18M rows are checked and 0.25M pushed:
+// 28.9 and 27.5 ms (31.0 with the offsets of every checked row loaded, and its
+// groups gone through, before it was known to push). Sharing a word's rows between
+// a block's warps as well took 5.7 ms where this took 7.4, but it moves the takes of those
 // vertices ahead of the others', and what a solve leaves below eps with them
 // (3e-4 of its norm, against 7e-5 between two runs).
 template <int LPR, int NV>
@@ -219,17 +221,12 @@ __global__ void __launch_bounds__(BB, 1) k_bsolve(BArgs a) {
             return (int)(wbase + b);
         };
         float4 rv[NV];
-        ull b0 = 0, b1 = 0;
-        auto load_offsets = [&](int v) {
-            if (v >= 0) { b0 = a.idx[v]; b1 = a.idx[v + 1]; }
-        };
         int v = next_row();
-        load_offsets(v);
         while (v >= 0) {
             float4* rrow = a.R + (size_t)v * a.V;
 #pragma unroll
             for (int k = 0; k < NV; k++)
-                rv[k] = v >= 0 && lane < LPR ? a.R[(size_t)v * a.V + j0 + LPR * k] : make_float4(0.f, 0.f, 0.f, 0.f);
+                rv[k] = lane < LPR ? rrow[j0 + LPR * k] : make_float4(0.f, 0.f, 0.f, 0.f);
             float4 d[NV];
             // a row with any pending lane is pushed whole (greedy): every lane with a nonzero
             // residual is taken, since the one read of the list serves them all
@@ -238,11 +235,14 @@ __global__ void __launch_bounds__(BB, 1) k_bsolve(BArgs a) {
             for (int k = 0; k < NV; k++)
                 pend |= lane < LPR && (fabsf(rv[k].x) > eps[k].x || fabsf(rv[k].y) > eps[k].y ||
                                        fabsf(rv[k].z) > eps[k].z || fabsf(rv[k].w) > eps[k].w);
-            const bool row_pend = __any_sync(FULL, pend);
+            if (!__any_sync(FULL, pend)) {   // most of the rows that are checked, on a large graph
+                v = next_row();
+                continue;
+            }
 #pragma unroll
             for (int k = 0; k < NV; k++) {
                 d[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (lane < LPR && row_pend) {
+                if (lane < LPR) {
                     if (a.greedy) {
                         // the whole 16-byte group in one exchange when any of its lanes is nonzero
                         if (nonzero(rv[k])) d[k] = atomicExch(rrow + j0 + LPR * k, make_float4(0.f, 0.f, 0.f, 0.f));
@@ -256,10 +256,9 @@ __global__ void __launch_bounds__(BB, 1) k_bsolve(BArgs a) {
                     }
                 }
             }
-            const ull l0 = b0;
-            const unsigned deg = (unsigned)(b1 - b0);
+            const ull l0 = a.idx[v];
+            const unsigned deg = (unsigned)(a.idx[v + 1] - l0);
             const int vn = next_row();
-            load_offsets(vn);   // in flight while this row is pushed
 #pragma unroll
             for (int k = 0; k < NV; k++)
                 if (nonzero(d[k])) {   // one writer per value: a reduction, for its load is not waited for
