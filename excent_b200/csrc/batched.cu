@@ -71,6 +71,7 @@ struct BArgs {
     BCtrl* ctrl;
     int greedy;               // take every nonzero lane of a pushed row, not only the pending ones
     int dense;                // hub segments of rows with more active groups scatter over the groups
+    int dense_row;            // rows of shorter lists likewise
 };
 
 __device__ __forceinline__ float take_lane(float* rp, float rv, float eps) {
@@ -107,35 +108,47 @@ __device__ __forceinline__ ull scatter_lanes(float4* R, int V, uint32_t* nxt, co
 // Scatter for rows with many active groups: the lanes over the row's groups
 // (lane j0 + LPR * k of each LPR-lane sub-warp), 32 / LPR target rows per
 // step, so each reduction instruction covers one contiguous stretch of a
-// target row instead of 32 unrelated rows.
+// target row instead of 32 unrelated rows. 128 entries' indices and marks in
+// flight and four steps unrolled: 64 lanes on 131k vertices 7.6 -> 7.1 ms, on
+// 50k 12.2 -> 9.7.
 template <int LPR, int NV>
 __device__ __forceinline__ ull scatter_rowpar(float4* R, int V, uint32_t* nxt, const int* nb, unsigned deg,
                                               const float4 (&p)[NV], const bool (&act)[NV], int lane) {
     constexpr int RPW = 32 / LPR;
     const int sub = lane / LPR, j0 = lane % LPR;
     ull upd = 0;
-    for (unsigned e0 = 0; e0 < deg; e0 += 32) {
-        const int ul = e0 + lane < deg ? ld_edge(nb + e0 + lane) : -1;
-        if (ul >= 0) {   // each lane marks its own entry's target, all 32 at once
-            const uint32_t bit = 1u << (ul & 31);
-            if (!(nxt[ul >> 5] & bit)) atomicOr(&nxt[ul >> 5], bit);
-        }
-        const unsigned cnt = min(32u, deg - e0);
-        for (unsigned g = 0; g < cnt; g += RPW) {
-            const int u = __shfl_sync(FULL, ul, (int)g + sub);
-            if (g + sub < cnt) {
-                float4* row = R + (size_t)u * V;
+    for (unsigned e0 = 0; e0 < deg; e0 += 128) {
+        int ul[4];
 #pragma unroll
-                for (int k = 0; k < NV; k++)
-                    if (act[k]) { red_add(row, j0 + LPR * k, p[k]); upd++; }
+        for (int q = 0; q < 4; q++) {   // four index loads, then four marks, in flight
+            const unsigned e = e0 + 32 * q + lane;
+            ul[q] = e < deg ? ld_edge(nb + e) : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {   // each lane marks its own entry's target, all 32 at once
+            if (ul[q] < 0) continue;
+            const uint32_t bit = 1u << (ul[q] & 31);
+            if (!(nxt[ul[q] >> 5] & bit)) atomicOr(&nxt[ul[q] >> 5], bit);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (e0 + 32 * q >= deg) break;
+            const unsigned cnt = min(32u, deg - e0 - 32 * q);
+#pragma unroll 4
+            for (unsigned g = 0; g < cnt; g += RPW) {
+                const int u = __shfl_sync(FULL, ul[q], (int)g + sub);
+                if (g + sub < cnt) {
+                    float4* row = R + (size_t)u * V;
+#pragma unroll
+                    for (int k = 0; k < NV; k++)
+                        if (act[k]) { red_add(row, j0 + LPR * k, p[k]); upd++; }
+                }
             }
         }
     }
     return upd;
 }
 
-// Rows of short lists with more active 16-byte groups than this scatter over their groups.
-static constexpr int DENSE_ROW = 4;
 // Default: segments of rows with more active 16-byte groups than this scatter over their groups.
 static constexpr int DENSE_GROUPS = 4;
 
@@ -169,12 +182,13 @@ __device__ __forceinline__ int compact_groups(const float4 (&p)[NV], const bool 
 // What bounds it: in the dense passes the warps whose word holds 32 vertices
 // with long lists, one row after the other; in the others the latency of the
 // two phases. Neighbouring words go to different SMs, the values are added by
-// reductions, which nothing waits for, and rows with many active groups scatter
-// over their groups. 64 queries on 131k vertices to 1e-6: 10.4 ms as three
-// kernels a pass in a graph, 8.2 ms; 256 on 65k: 36.7 and 17.5 ms; 256 on 16.8M
-// vertices to 1e-4 of their mass, where 18M rows are checked and 0.25M pushed:
-// 28.9 and 27.5 ms (31.0 with the offsets of every checked row loaded, and its
-// groups gone through, before it was known to push). Sharing a word's rows between
+// reductions, which nothing waits for, a row that does not push is left at
+// once, and rows with many active groups scatter over their groups. As three
+// kernels a pass in a graph and so: 64 queries on 131k vertices to 1e-6 10.4 and
+// 7.5 ms, on 8k 6.1 and 5.0; 256 on 65k 36.9 and 17.8; 256 on 16.8M vertices to
+// 1e-4 of their mass, where 18M rows are checked and 0.25M pushed, 28.9 and 27.7
+// (31.0 with the offsets of every checked row loaded, and its groups gone
+// through, before it was known to push). Sharing a word's rows between
 // a block's warps as well took 5.7 ms where this took 7.4, but it moves the takes of those
 // vertices ahead of the others', and what a solve leaves below eps with them
 // (3e-4 of its norm, against 7e-5 between two runs).
@@ -312,7 +326,7 @@ __global__ void __launch_bounds__(BB, 1) k_bsolve(BArgs a) {
                 continue;
             }
             const int nact = compact_groups<LPR, NV>(p, act, s_gp[wib], s_gi[wib], lane);
-            if (nact > DENSE_ROW) upd += scatter_rowpar<LPR, NV>(a.R, a.V, nxt, nb, deg, p, act, lane);
+            if (nact > a.dense_row) upd += scatter_rowpar<LPR, NV>(a.R, a.V, nxt, nb, deg, p, act, lane);
             else upd += scatter_lanes(a.R, a.V, nxt, nb, deg, s_gp[wib], s_gi[wib], nact, lane);
             __syncwarp();
         }
@@ -444,6 +458,13 @@ static BArgs bargs(excent_batch* b) {
     a.ctrl = b->d_ctrl;
     a.greedy = b->greedy;
     a.dense = b->dense;
+    // With words for fewer than half of the warps (an eighth, with 256 lanes) a solve lasts as long as the warp with the longest
+    // lists, which is faster with its lanes over entries; with more of them what counts is the reductions'
+    // throughput, better over groups when most are active. 64 lanes, greedy, lanes over entries and over
+    // groups: 8k vertices 5.0 and 7.0 ms, 50k 6.4 and 9.7, 90k of 32 entries each 11.0 and 8.5, 131k 9.6 and
+    // 7.0; 256 lanes: 8k 10.2 and 12.5, 20k 15.5 and 15.6, 70k 18.7 and 16.6; 128 lanes on 131k, not greedy
+    // (fewer groups active) 2.6 and 3.5, 3.0 by this rule.
+    a.dense_row = (a.V > 32 ? 8 : 2) * (ull)a.words >= (ull)b->sms * (BB / 32) ? a.V / 2 : a.V;
     return a;
 }
 
