@@ -1106,10 +1106,10 @@ static int free_engine(excent_engine* e) {
 #define EX_HALLOC(ptr, bytes) do { if (cudaMallocHost((void**)&(ptr), (bytes)) != cudaSuccess) { cudaGetLastError(); \
     ::excent::set_error("pinned allocation of %llu bytes failed (%s)", (ull)(bytes), #ptr); return EXCENT_ERR_NOMEM; } } while (0)
 
-// Segments of a wave's longer lists: short ones spread a small graph's lists over more warps (host-driven
-// passes over 1M entries, one measure 4.1 ms a solve, 4.5-4.9 with HUB_SEG, three 5.6 and 5.9-6.6). From 3M
-// to 263M entries they make no difference (1 %), and from 2^26 on the longer ones save three quarters of the
-// queue, 0.125 bytes an entry.
+// Segments of a wave's longer lists: short ones spread a small graph's lists over more warps. PageRank
+// with 256 and with 1024 entries to a segment: 1M entries 0.89 and 1.01 ms (three measures 2.65 and 3.12),
+// 3M 2.24 and 2.18, 16M and 32M the same to 1 %, 65M 18.1 and 17.6, 131M 26.2 and 25.6, 263M the same.
+// The line lies where the short ones' queue, 0.125 bytes an entry, starts to count.
 static constexpr ull wave_seg(ull m) { return m < (1ull << 26) ? 256 : HUB_SEG; }
 // Most items of a wave, whatever the occupancy (148 SMs x 2048 threads).
 static constexpr int WAVE_MAX = 1 << 18;
