@@ -461,7 +461,7 @@ def run_ours(a, world, rank, local, dist):
         "e2e": {"value": round(e_pushed / te / 1e9, 4), "unit": "GTEPS", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": round(te / a.steps * 1e3, 3),
                 "wall_ms_per_step": round(te_wall / a.steps * 1e3, 3)},
-        "roofline": {"bound": "hbm", "kernel": "k_push + k_segments of a profiled solve by the host-driven loop (one logical push: the takes, the short lists, then the queued long-list segments); the timed solves run k_passes and k_sweep_gather, inside a graph whose kernels cannot be timed one by one",
+        "roofline": {"bound": "hbm", "kernel": "k_push + k_segments of a profiled solve by the host-driven loop (one logical push: the takes, the short lists, then the queued long-list segments); the timed solves run k_passes and k_sweep_gather (without a chunk sweep these same two), inside a graph whose kernels cannot be timed one by one",
                      "achieved": round(achieved, 1), "peak": peak, "peak_source": peak_kind, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": traffic,
                      "traffic_note": traffic_note,

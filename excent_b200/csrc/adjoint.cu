@@ -98,8 +98,8 @@ struct WGather {
 // latency of the phases (75 us for a dense pass of 16.8M entries). On an R-MAT
 // of 1M vertices and 16.8M entries, forward and gradient together took 305 ms
 // with whole lists on one warp, 58.7 ms scattering them split (38 G entries/s:
-// reductions to the same vertices serialise) and take 14.5 ms gathering
-// (181-196 G entries/s).
+// reductions to the same vertices serialise) and take 14.8 ms gathering, to
+// eps / 2 (14.5 ms to eps; 181-196 G entries/s).
 __global__ void __launch_bounds__(WP, 1) k_wsolve(WArgs a) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const long long gw = (long long)wib * gridDim.x + blockIdx.x;   // neighbouring tiles on different SMs

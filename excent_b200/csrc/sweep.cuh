@@ -3,8 +3,8 @@
 // A swept pass pushes most of the graph, where a gather is faster than the
 // scatter (pull.cuh): on an R-MAT of 16.8M vertices and 263M entries a swept
 // pass takes 1.3 ms for one measure (scatter: 2.5) and 2.0 ms for three (3.4).
-// What bounds it is one L1 lookup per entry (284 G/s for the GPU: 0.93 ms a
-// pass; the long late parts reach 85-100 % of that) and, for the many lists of
+// What bounds it is one L1 lookup per entry (284 G/s for the GPU, less where
+// lanes share one: 0.93 ms a pass; the long late parts reach 85-100 % of that) and, for the many lists of
 // a few entries, chains of dependent loads in each of the phases. (Filling the
 // ends of the phases with late segments, and keys loaded a batch ahead, gained
 // nothing.) On a symmetric graph the push of vertex u is the same as every
@@ -110,7 +110,8 @@ __global__ void k_sweep_phase(int n, const ull* idx, const int* cv0, int nc, con
     }
 }
 
-// A bijective mix of the ordered pair (a, b).
+// A bijective mix of the ordered pair (a, b): variant 1 of David Stafford's finalizers of 64 bits
+// ("Better Bit Mixing", 2011).
 __device__ __forceinline__ ull mix_pair(int a, int b) {
     ull z = ((ull)(unsigned)a << 32) | (unsigned)b;
     z = (z ^ (z >> 31)) * 0x7FB5D329728EA185ull;

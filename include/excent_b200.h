@@ -128,7 +128,9 @@ int excent_engine_chunk_list(excent_engine* e, int c, int32_t* ids, unsigned int
  * each as its pending list when cnt < list_frac * chunk vertices, else as
  * its whole vertex range with the push-time re-check. Replaces the resident
  * loop and launch_chunk (src/excent.cu:629-652, 684-688). mode and cnt are
- * host arrays (cnt as returned by the last snapshot). */
+ * host arrays (cnt as returned by the last snapshot). When every chunk with
+ * cnt > 0 is among them, the push takes residuals without exchanges, and it
+ * and pushes of the slots wait for one another on the device. */
 int excent_engine_push_cached(excent_engine* e, const unsigned char* mode, const unsigned long long* cnt,
                               double list_frac);
 
@@ -182,7 +184,11 @@ int excent_engine_sync(excent_engine* e);
  * chunk by chunk or the graph is large, one CUDA graph with a conditional while
  * node; without it the host reads each pass's plan back and
  * launches its pushes.
- * Per-pass log and totals are kept for excent_engine_stats. */
+ * Per-pass log and totals are kept for excent_engine_stats. The first solve
+ * (or cached push) that sweeps newly loaded lists of a symmetric graph splits a
+ * copy of them for gathers, in at most an eighth of the free device memory,
+ * which the engine keeps until its cache is reserved again; a high-degree order
+ * other than 3 (excent_engine_set_hub_order) goes without. */
 int excent_engine_solve(excent_engine* e, double list_frac, int max_passes, int use_graph);
 
 /* Same as excent_engine_solve but from the current values and residuals
@@ -236,7 +242,9 @@ int excent_engine_read_trace(excent_engine* e, uint16_t* out);
  * it off and restores plain ids. Call after the cache is reserved: chunks
  * loaded so far are rewritten now, later loads (load_cache, upload_device,
  * cache-filling streamed pushes) as they land; reserving the cache again
- * turns it off. No reference counterpart. */
+ * turns it off. Only targets of at least 64 entries get a slot, so there may be
+ * fewer than k, or none; k itself sets how many items a pass takes together,
+ * and is what the autotuner reports. No reference counterpart. */
 int excent_engine_set_hub_targets(excent_engine* e, int k);
 
 /* Order of the high-degree lists (more than 256 entries) in each pass of the
@@ -500,8 +508,9 @@ int excent_batch_launches(excent_batch* b, unsigned long long* launches);
  * weighted delta-push to an absolute eps. The VJP of a scalar loss with
  * dL/dx = c solves lambda = c + s W lambda by the same push on the transposed
  * lists and returns dL/dt (or dL/dbeta) and dL/dw for the raw weights through
- * the normalisation. All vectors are device pointers. No reference
- * counterpart: the reference has neither weights nor gradients. */
+ * the normalisation. A row whose weights sum to 0 has no normalised weights:
+ * what it pushes is no number and stays with its targets. All vectors are
+ * device pointers. No reference counterpart: the reference has neither weights nor gradients. */
 typedef struct excent_wgraph excent_wgraph;
 int excent_wgraph_create(int device, int n, unsigned long long m, const unsigned long long* d_idx, const int32_t* d_adj,
                          const float* d_w, excent_wgraph** out);
