@@ -272,7 +272,7 @@ def test_unswept_solves_of_large_graphs_ask_the_host_nothing(measure, scale, ef)
     eng = X.Engine(g.n, g.m, meas, *X.plan_chunks(idx, g.m))
     eng.upload_device(di, da)
     eng.solve(max_passes=1)
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as prof:
         st = eng.solve(max_passes=40)
     waits = sum(ev.name == "cudaStreamSynchronize" for ev in prof.events())
     assert st.passes > 10 and waits <= 2, (st.passes, waits)
