@@ -1898,6 +1898,7 @@ static cudaError_t launch_small(excent_engine* e, SolveArgs& a, cudaStream_t st)
     const size_t smem = (hub_smem(e) + 15) / 16 * 16 + recs;
     const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SLOT_BYTES_MAX + (int)recs);
     if (rc != cudaSuccess) return rc;
+    if (e->d_hcache && e->cache_edges == 0) a.list_frac = 0;   // lists in host memory go as a range in every pass (see k_plan)
     return launch_grid(kernel, solve_grid(e), PT, smem, a, &e->d_ctrl->bar, st);
 }
 static cudaError_t launch_passes(excent_engine* e, SolveArgs& a, cudaStream_t st) {

@@ -71,7 +71,6 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     // the pass log is written off the critical path, by the last warp of the last block
     const bool scribe = blockIdx.x == gridDim.x - 1 && threadIdx.x == PT - 32;
-    const bool host_lists = a.cmode[0] == 2;   // the chunk goes as a range in every pass (see k_plan)
     T* r = P.r;
     if (lane < 4) s_took[lane][wib] = 0;
     int v[V];
@@ -171,7 +170,7 @@ __global__ void __launch_bounds__(PT, 1) k_small(const __grid_constant__ SolveAr
         if (!P.sync()) return;
         const ull np = acc->pending;
         const bool stop = pass >= a.max_passes || np == 0;
-        const bool range = host_lists || !((double)np < a.list_frac * n);   // (src/excent.cu:639)
+        const bool range = !((double)np < a.list_frac * n);   // (src/excent.cu:639)
         const unsigned nhub = (unsigned)min((ull)wave->big, a.push.hub_cap);
         if (scribe && !stop && pass < a.log_cap) {
             PassRec& R = a.log[pass];
