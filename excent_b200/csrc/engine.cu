@@ -1912,7 +1912,9 @@ static cudaError_t launch_sweep(excent_engine* e, SolveArgs& a, cudaStream_t st)
     GridBar* bar = a.use_cond ? nullptr : &e->d_ctrl->sweep_bar;
     if (e->sweep_ok && a.order == 3) {
         SweepArgs s{a, e->sweep};
-        return launch_grid(e->L == 1 ? k_sweep_gather<1> : k_sweep_gather<4>, e->sms * G_PER_SM, GT, 0, s, bar, st);
+        auto kernel = a.standalone ? (e->L == 1 ? k_sweep_gather<1, true> : k_sweep_gather<4, true>)
+                                   : (e->L == 1 ? k_sweep_gather<1, false> : k_sweep_gather<4, false>);
+        return launch_grid(kernel, e->sms * G_PER_SM, GT, 0, s, bar, st);
     }
     return launch_grid(e->L == 1 ? k_sweep<1> : k_sweep<4>, solve_grid(e), PT, hub_smem(e), a, bar, st);
 }

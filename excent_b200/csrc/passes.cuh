@@ -418,12 +418,14 @@ template <int L> struct Passes {
     }
 
     // The long lists of hub vertices [h0, h1), all taken before any is scattered. A host-driven push
-    // leaves the vertices of other chunks than it was asked for alone: their lists may not be loaded.
+    // (HOST: it may be one) leaves the vertices of other chunks than it was asked for alone: their lists
+    // may not be loaded.
+    template <bool HOST>
     __device__ __forceinline__ bool push_hubs(long long h0, long long h1, bool listed) {
         if (h1 <= h0) return true;
         return push_wave(h1 - h0, LISTS_LONG, [&](long long i) {
             const int v = a.push.hubv[h0 + i];
-            if (a.standalone && type[chunk_of(v, a.push.cv0, a.push.nc)] == WT_NONE) return -1;
+            if (HOST && a.standalone && type[chunk_of(v, a.push.cv0, a.push.nc)] == WT_NONE) return -1;
             return listed && !bit_of(a.snap.bitmap, v) ? -1 : v;
         });
     }
@@ -597,10 +599,10 @@ __global__ void __launch_bounds__(PT, 1) k_passes(const __grid_constant__ SolveA
         if (take_hubs) {
             if (!P.push_taken_hubs()) return;
         } else if (a.order == 1 || a.order == 3) {
-            if (!P.push_hubs(0, (long long)*a.push.hubv_cnt, false)) return;
+            if (!P.template push_hubs<false>(0, (long long)*a.push.hubv_cnt, false)) return;
         }
         if (!P.push_table(0, items, -1, a.order ? LISTS_SHORT : LISTS_ALL)) return;
-        if (a.order == 2) { if (!P.push_hubs(0, (long long)*a.push.hubv_cnt, false)) return; }
+        if (a.order == 2) { if (!P.template push_hubs<false>(0, (long long)*a.push.hubv_cnt, false)) return; }
         // the counters are read after the next snapshot's barrier
         P.report();
     }
@@ -616,9 +618,9 @@ __global__ void __launch_bounds__(PT, 1) k_table(const __grid_constant__ SolveAr
         for (WaveCount& w : a.push.ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }
     if (!P.sync()) return;
     const long long nh = a.order ? (long long)*a.push.hubv_cnt : 0;
-    if ((a.order == 1 || a.order == 3) && !P.push_hubs(0, nh, false)) return;
+    if ((a.order == 1 || a.order == 3) && !P.template push_hubs<true>(0, nh, false)) return;
     if (!P.push_table(0, P.prefix[a.push.nc], -1, a.order ? LISTS_SHORT : LISTS_ALL)) return;
-    if (a.order == 2 && !P.push_hubs(0, nh, false)) return;
+    if (a.order == 2 && !P.template push_hubs<true>(0, nh, false)) return;
     P.report();
 }
 
@@ -644,17 +646,17 @@ __global__ void __launch_bounds__(PT, 1) k_sweep(const __grid_constant__ SolveAr
         for (WaveCount& w : ctrl->wave) { w.small = 0; w.big = 0; w.claim = 0; }
     if (!P.sync()) return;
     const int order = a.order;
-    if (order == 1 && !P.push_hubs(0, (long long)*a.push.hubv_cnt, false)) return;
+    if (order == 1 && !P.template push_hubs<true>(0, (long long)*a.push.hubv_cnt, false)) return;
     for (int c = 0; c < nc; c++) {
         const long long first = P.prefix[c], total = P.prefix[c + 1];
         if (total == first) continue;
         if (order == 3) {
             const int v0 = a.push.cv0[c], v1 = c + 1 < nc ? a.push.cv0[c + 1] : a.snap.n;
-            if (!P.push_hubs(P.hub_bound(v0), P.hub_bound(v1), P.type[c] == WT_LIST)) return;
+            if (!P.template push_hubs<true>(P.hub_bound(v0), P.hub_bound(v1), P.type[c] == WT_LIST)) return;
         }
         if (!P.push_table(first, total, c, order ? LISTS_SHORT : LISTS_ALL)) return;
     }
-    if (order == 2 && !P.push_hubs(0, (long long)*a.push.hubv_cnt, false)) return;
+    if (order == 2 && !P.template push_hubs<true>(0, (long long)*a.push.hubv_cnt, false)) return;
     P.report();
 }
 

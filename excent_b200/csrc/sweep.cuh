@@ -476,13 +476,13 @@ __device__ __forceinline__ void take_here(typename Lane<L>::T* x, typename Lane<
     }
 }
 
-// One swept pass as gathers, per the table k_passes left.
+// One swept pass as gathers, per the table k_passes left (HOST: per that of a host-driven push).
 static constexpr int GT = 1024, GW = GT / 32, G_PER_SM = 1;   // threads and warps per block, blocks per SM
 struct SweepArgs {
     SolveArgs a;
     SweepLists g;
 };
-template <int L>
+template <int L, bool HOST>
 __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_constant__ SweepArgs args) {
     const SolveArgs& a = args.a;
     const SweepLists& g = args.g;
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
     __shared__ ull s_tot[3][GW];
     __shared__ unsigned s_next;
     Ctrl* ctrl = a.push.ctrl;
-    if (!a.standalone && (ctrl->done || !ctrl->sweep_pass)) return;
+    if (!HOST && (ctrl->done || !ctrl->sweep_pass)) return;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nc = a.push.nc;
     unsigned epoch = 0;
     clear_tables(a, GT);
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(GT, G_PER_SM) k_sweep_gather(const __grid_cons
         while (bits) {
             const int v = (int)w * 32 + __ffs(bits) - 1;
             bits &= bits - 1;
-            if (a.standalone && a.push.wt_type[chunk_of(v, a.push.cv0, nc)] == WT_NONE) continue;   // not asked for
+            if (HOST && a.push.wt_type[chunk_of(v, a.push.cv0, nc)] == WT_NONE) continue;   // not asked for
             take_here<L>(x, r, P, v, r[v], 0, true, false, a.push.M, pushed, lanes, taken);
         }
     }
